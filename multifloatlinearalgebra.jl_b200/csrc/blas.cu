@@ -12,9 +12,14 @@
 // broadcasts.  k-slabs of BK columns of every limb plane are staged in shared
 // memory with cp.async into a double buffer while the previous slab is
 // consumed.  The kernel is FP64-issue bound: per k step a thread reads
-// (TM + TN)*N doubles and executes TM*TN*ops(N) FP64 instructions.
+// (TM + TN)*N doubles and executes TM*TN*ops(N) FP64 instructions.  Tile
+// shapes trade that ratio against the number of CTAs (mm_tile below); a
+// matrix-vector product is a chain per row and has a kernel of its own
+// (mv_kernel).
 #include "mf_device.cuh"
 #include "mflab_internal.h"
+
+#include <algorithm>
 
 MFLAB_DEBUG_RECORD(blas)
 
@@ -48,8 +53,10 @@ struct MMShape {
 // C(i,j) runs over k <= idx (or k >= idx with MM_KGE), idx = i (or j with
 // MM_RIGHT), and with MM_UNIT its diagonal term k == idx adds the other
 // operand's entry instead of a product (trmm.jl:1-80).
-template <int N, int BM, int BN, int BK, int TM, int TN, int TA, bool TB, bool TRI, bool FUSED,
-          bool TRMM>
+// UNR: k steps unrolled together (threads with one output need several steps
+// in flight to hide the shared-memory reads behind the accumulation chain).
+template <int N, int BM, int BN, int BK, int TM, int TN, int UNR, int TA, bool TB, bool TRI,
+          bool FUSED, bool TRMM>
 __global__ void __launch_bounds__(MMShape<N, BM, BN, BK, TM, TN>::NT)
     mm_kernel(int64_t m, int64_t n, int64_t K, Mat A, Mat B, Mat C, scal<N> alpha, scal<N> beta,
               int overwrite, const int *info, int mode) {
@@ -166,7 +173,7 @@ __global__ void __launch_bounds__(MMShape<N, BM, BN, BK, TM, TN>::NT)
         __syncthreads();
         const int64_t rem = kend - k0;
         if (rem >= BK) {
-#pragma unroll 2
+#pragma unroll UNR
             for (int kk = 0; kk < BK; ++kk) step(buf, kk, k0 + kk);
         } else {
             for (int kk = 0; kk < (int)rem; ++kk) step(buf, kk, k0 + kk);
@@ -201,12 +208,12 @@ __global__ void __launch_bounds__(MMShape<N, BM, BN, BK, TM, TN>::NT)
     }
 }
 
-template <int N, int BM, int BN, int BK, int TM, int TN, int TA, bool TB, bool TRI, bool FUSED,
-          bool TRMM>
+template <int N, int BM, int BN, int BK, int TM, int TN, int UNR, int TA, bool TB, bool TRI,
+          bool FUSED, bool TRMM>
 static int run_mm(int64_t m, int64_t n, int64_t k, Mat A, Mat B, Mat C, const double *alpha,
                   const double *beta, cudaStream_t s, const int *info, int mode) {
     using S = MMShape<N, BM, BN, BK, TM, TN>;
-    auto kern = mm_kernel<N, BM, BN, BK, TM, TN, TA, TB, TRI, FUSED, TRMM>;
+    auto kern = mm_kernel<N, BM, BN, BK, TM, TN, UNR, TA, TB, TRI, FUSED, TRMM>;
     static std::atomic<unsigned long long> configured{0};
     if (int rc = set_smem_once((const void *)kern, (int)S::smem_bytes, configured,
                                "mm_kernel attribute"))
@@ -225,34 +232,216 @@ static int run_mm(int64_t m, int64_t n, int64_t k, Mat A, Mat B, Mat C, const do
     return record_cuda_error(cudaGetLastError(), "mm_kernel launch");
 }
 
-// tile shapes per limb count (FP64-issue bound; registers: TM*TN*N accumulators).
-// Products at most 16 columns wide (a blocked factorization's next block
-// columns, a few right-hand sides) take 32 x 16 tiles of two outputs per
-// thread: a 64 x 64 tile would leave three quarters of its threads idle and
-// put the whole product on a few CTAs.  Every output is the same chain in
-// either shape.
+// Tile shapes.  Every output is the same chain in every shape, so the choice
+// is free.  One CTA of at least two outputs per thread keeps an SM's FP64 pipe
+// busy by itself, so a launch takes about
+//     ceil(tiles / SMs) * BM * BN / rate
+// with the tile's measured rate (10^12 FP64 instructions/s on a full chip).
+// Measured, us (x2: 64x64 of 4x4 outputs per thread / 32x16 of 2x1 / 16x8 of 1):
+//     48 x 56 x 40       49.2 / 13.2 / 9.2
+//     256 x 256 x 256     276 / 50.2 / 50.1
+//     515 x 777, k 389    416 /  336 / 330
+//     1000 cubed         2063 / 1911 / 1993
+//     2048 x 2048, k 512 3642 / 3825 / 4147
+// x3 (64x64 / 32x32 / 16x16): 515 x 777, k 389: 1371 / 1018 / 964;
+// 2048 x 2048, k 512: 12494 / 12172 / 12478.  x4 (64x32 / 16x16 / 16x8):
+// 48 x 56 x 40: 197 / 27.6 / 20.5; 515 x 777, k 389: 3075 / 2101 / 2125;
+// 2048 x 2048, k 512: 27455 / 27549 / 27719.
+constexpr int MM_SMS = 148;
+enum { MM_TINY = 0, MM_MID = 1, MM_WIDE = 2 };
+
+static double mm_cost(int64_t m, int64_t n, bool tri, int bm, int bn, double rate, int least) {
+    const int64_t tr = (m + bm - 1) / bm, tc = (n + bn - 1) / bn;
+    int64_t tiles = tr * tc;
+    if (tri) tiles = tiles / 2 + (tr + tc) / 4 + 1;  // tiles above the diagonal return at once
+    const int64_t rounds = std::max<int64_t>((tiles + MM_SMS - 1) / MM_SMS, least);
+    return (double)(rounds * bm * bn) / rate;
+}
+
+// the shape with the smallest estimate; a lone 16 x 8 CTA (one chain per
+// scheduler) leaves the pipe half idle, hence at least two rounds for it
+template <int N>
+static int mm_tile(int64_t m, int64_t n, bool tri) {
+    const double tiny = mm_cost(m, n, tri, 16, 8, N == 2 ? 14.6 : 16.8, 2);
+    const double mid = N == 2 ? mm_cost(m, n, tri, 32, 16, 15.6, 1)
+                              : mm_cost(m, n, tri, 16, 16, N == 3 ? 17.0 : 17.7, 1);
+    const double wide = N == 2   ? mm_cost(m, n, tri, 64, 64, 16.5, 1)
+                        : N == 3 ? mm_cost(m, n, tri, 32, 32, 17.4, 1)
+                                 : 1e300;
+    if (wide <= mid && wide <= tiny) return MM_WIDE;
+    return mid <= tiny ? MM_MID : MM_TINY;
+}
+
 template <int N, int TA, bool TB, bool TRI, bool FUSED, bool TRMM = false>
 static int run_mm_n(int64_t m, int64_t n, int64_t k, Mat A, Mat B, Mat C, const double *alpha,
                     const double *beta, cudaStream_t s, const int *info, int mode) {
-    if constexpr (N >= 2 && !FUSED && !TRMM) {
-        if (n <= 16)
-            return run_mm<N, 32, 16, (N == 2 ? 16 : 8), 2, 1, TA, TB, TRI, FUSED, TRMM>(
+    if constexpr (N == 1) {
+        return run_mm<1, 64, 64, 16, 4, 4, 2, TA, TB, TRI, FUSED, TRMM>(m, n, k, A, B, C, alpha, beta, s, info, mode);
+    } else {
+        const int tile = mm_tile<N>(m, n, TRI);
+        if (tile == MM_TINY)
+            return run_mm<N, 16, 8, 16, 1, 1, (N == 2 ? 8 : N == 3 ? 4 : 2), TA, TB, TRI, FUSED, TRMM>(
                 m, n, k, A, B, C, alpha, beta, s, info, mode);
+        if constexpr (N == 2) {
+            if (tile == MM_MID)
+                return run_mm<2, 32, 16, 16, 2, 1, 4, TA, TB, TRI, FUSED, TRMM>(m, n, k, A, B, C, alpha, beta, s, info, mode);
+            return run_mm<2, 64, 64, 16, 4, 4, 2, TA, TB, TRI, FUSED, TRMM>(m, n, k, A, B, C, alpha, beta, s, info, mode);
+        } else if constexpr (N == 3) {
+            if (tile == MM_MID)
+                return run_mm<3, 16, 16, 16, 1, 1, 4, TA, TB, TRI, FUSED, TRMM>(m, n, k, A, B, C, alpha, beta, s, info, mode);
+            return run_mm<3, 32, 32, 8, 2, 2, 2, TA, TB, TRI, FUSED, TRMM>(m, n, k, A, B, C, alpha, beta, s, info, mode);
+        } else {
+            return run_mm<4, 16, 16, 8, 1, 1, 4, TA, TB, TRI, FUSED, TRMM>(m, n, k, A, B, C, alpha, beta, s, info, mode);
+        }
     }
-    if constexpr (N == 1)
-        return run_mm<1, 64, 64, 16, 4, 4, TA, TB, TRI, FUSED, TRMM>(m, n, k, A, B, C, alpha, beta, s, info, mode);
-    else if constexpr (N == 2)
-        return run_mm<2, 64, 64, 16, 4, 4, TA, TB, TRI, FUSED, TRMM>(m, n, k, A, B, C, alpha, beta, s, info, mode);
-    else if constexpr (N == 3)
-        return run_mm<3, 64, 64, 8, 4, 4, TA, TB, TRI, FUSED, TRMM>(m, n, k, A, B, C, alpha, beta, s, info, mode);
-    else
-        return run_mm<4, 64, 32, 8, 4, 2, TA, TB, TRI, FUSED, TRMM>(m, n, k, A, B, C, alpha, beta, s, info, mode);
+}
+
+// Matrix-vector product y = alpha op(A) x + beta y: row i is one ascending
+// chain acc = acc + a(i,k) x(k), so a launch cannot end before K dependent
+// additions have (about 90 cycles each in x2, 220 in x3, 350 in x4).  A CTA
+// owns 32 rows: one warp runs their chains and does nothing else, six warps on
+// the other three schedulers load A and form the products of the next 32
+// columns into shared memory (two slabs, one CTA barrier per slab).  The
+// second warp on the chain's own scheduler stays idle, and the chain warp's
+// place rotates over the schedulers with the CTA so that CTAs that share an
+// SM do not share a scheduler.  TA as in mm_kernel; a 32 x 32 block of a
+// symmetric matrix lies on one side of the diagonal or on it.  2500 x 3100 in
+// x2: 168 us, 103 cycles a term (590 us on mm_kernel's 32 x 16 tile, of whose
+// sixteen columns one was used; 298 us on 32 x 1 tiles that load and multiply
+// in the chain's own warp).
+constexpr int MV_ROWS = 32, MV_KB = 32, MV_NT = 256, MV_HELPERS = 6;
+
+template <int N>
+struct MVStride {  // odd: the columns of one row fall on all banks
+    static constexpr int value = N * MV_ROWS + 1;
+};
+
+template <int N, int TA>
+__global__ void __launch_bounds__(MV_NT)
+    mv_kernel(int64_t m, int64_t K, Mat A, Mat X, Mat Y, scal<N> alpha, scal<N> beta, int overwrite,
+              const int *info) {
+    if (info && *info) return;
+    extern __shared__ double prod[];  // [2][MV_KB][ST]
+    constexpr int ST = MVStride<N>::value;
+    const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+    const int chain = (int)((blockIdx.x + blockIdx.x / MM_SMS) % 4);
+    const int side = (warp - chain) & 3;                        // scheduler beside the chain's
+    const int helper = side == 0 ? -1 : 2 * (side - 1) + warp / 4;  // 0 .. 5
+    const int64_t row0 = (int64_t)blockIdx.x * MV_ROWS;
+    const int64_t slabs = (K + MV_KB - 1) / MV_KB;
+    constexpr int PER = (MV_KB + MV_HELPERS - 1) / MV_HELPERS;
+
+    auto produce = [&](int64_t s) {
+        double *out = prod + (s & 1) * MV_KB * ST;
+        const int64_t k0 = s * MV_KB;
+        // is the block read down its rows (A[i,k]) or across (A[k,i])?  On the
+        // diagonal block of a symmetric matrix every entry decides for itself.
+        const bool across = TA == 1 || (TA == 2 && k0 > row0) || (TA == 3 && k0 < row0);
+        mf<N> a[PER];
+        if (!across) {
+            const int64_t row = row0 + lane;
+#pragma unroll
+            for (int q = 0; q < PER; ++q) {
+                const int kk = helper + MV_HELPERS * q;
+                const int64_t k = k0 + kk;
+                const bool ok = kk < MV_KB && k < K && row < m;
+                const bool tr = (TA == 2 && k > row) || (TA == 3 && k < row);
+                a[q] = !ok  ? from_double<N>(0.0)
+                       : tr ? load_mf<N>(A.p, A.ld, A.ls, k, row)
+                            : load_mf<N>(A.p, A.ld, A.ls, row, k);
+            }
+#pragma unroll
+            for (int q = 0; q < PER; ++q) {
+                const int kk = helper + MV_HELPERS * q;
+                if (kk >= MV_KB || k0 + kk >= K) break;
+                const mf<N> p = mul(a[q], load_mf<N>(X.p, 0, X.ls, k0 + kk, 0));
+#pragma unroll
+                for (int l = 0; l < N; ++l) out[kk * ST + l * MV_ROWS + lane] = p.v[l];
+            }
+        } else {
+            const int64_t k = k0 + lane;
+            const bool kin = k < K;
+#pragma unroll
+            for (int q = 0; q < PER; ++q) {
+                const int64_t row = row0 + helper + MV_HELPERS * q;
+                const bool ok = kin && helper + MV_HELPERS * q < MV_ROWS && row < m;
+                a[q] = ok ? load_mf<N>(A.p, A.ld, A.ls, k, row) : from_double<N>(0.0);
+            }
+            const mf<N> x = kin ? load_mf<N>(X.p, 0, X.ls, k, 0) : from_double<N>(0.0);
+#pragma unroll
+            for (int q = 0; q < PER; ++q) {
+                const int i = helper + MV_HELPERS * q;
+                if (i >= MV_ROWS) break;
+                const mf<N> p = mul(a[q], x);
+#pragma unroll
+                for (int l = 0; l < N; ++l) out[lane * ST + l * MV_ROWS + i] = p.v[l];
+            }
+        }
+    };
+
+    mf<N> acc = from_double<N>(0.0);
+    if (slabs > 0 && helper >= 0) produce(0);
+    for (int64_t s = 0; s < slabs; ++s) {
+        __syncthreads();
+        if (warp == chain) {
+            const double *in = prod + (s & 1) * MV_KB * ST + lane;
+            auto term = [&](int kk) {
+                mf<N> p;
+#pragma unroll
+                for (int l = 0; l < N; ++l) p.v[l] = in[kk * ST + l * MV_ROWS];
+                acc = add(acc, p);
+            };
+            const int64_t left = K - s * MV_KB;
+            if (left >= MV_KB) {
+#pragma unroll 8
+                for (int kk = 0; kk < MV_KB; ++kk) term(kk);
+            } else {
+                for (int kk = 0; kk < (int)left; ++kk) term(kk);
+            }
+        } else if (helper >= 0 && s + 1 < slabs) {
+            produce(s + 1);
+        }
+    }
+    const int64_t row = row0 + lane;
+    if (warp != chain || row >= m) return;
+    mf<N> r = mul(alpha.get(), acc);
+    if (!overwrite) r = add(r, mul(beta.get(), load_mf<N>(Y.p, 0, Y.ls, row, 0)));
+    store_mf<N>(Y.p, 0, Y.ls, row, 0, r);
+}
+
+template <int N, int TA>
+static int run_mv(int64_t m, int64_t k, Mat A, Mat X, Mat Y, const double *alpha,
+                  const double *beta, cudaStream_t s, const int *info) {
+    constexpr size_t smem = sizeof(double) * 2 * MV_KB * MVStride<N>::value;
+    auto kern = mv_kernel<N, TA>;
+    static std::atomic<unsigned long long> configured{0};
+    if (int rc = set_smem_once((const void *)kern, (int)smem, configured, "mv_kernel attribute"))
+        return rc;
+    scal<N> al{}, be{};
+    int overwrite = 1;
+    for (int l = 0; l < N; ++l) {
+        al.v[l] = alpha[l];
+        be.v[l] = beta[l];
+        if (beta[l] != 0.0) overwrite = 0;
+    }
+    const int64_t grid = (m + MV_ROWS - 1) / MV_ROWS;
+    if (grid > 2147483647LL) return MFLAB_ERR_UNSUPPORTED;
+    kern<<<(unsigned)grid, MV_NT, smem, s>>>(m, k, A, X, Y, al, be, overwrite, info);
+    return record_cuda_error(cudaGetLastError(), "mv_kernel launch");
 }
 
 template <int N>
 static int dispatch_mm(int ta, bool tb, int tri, bool fused3, int64_t m, int64_t n, int64_t k,
                        Mat A, Mat B, Mat C, const double *alpha, const double *beta,
                        cudaStream_t s, const int *info, int mode) {
+    if (n == 1 && m > 0 && !tb && !tri && !mode && !(N == 3 && fused3)) {
+        // one column: every output is a chain over a row (the fused x3 step
+        // has no separate product and stays with the tiles)
+        if (ta == 0) return run_mv<N, 0>(m, k, A, B, C, alpha, beta, s, info);
+        if (ta == 1) return run_mv<N, 1>(m, k, A, B, C, alpha, beta, s, info);
+        if (ta == 2) return run_mv<N, 2>(m, k, A, B, C, alpha, beta, s, info);
+        if (ta == 3) return run_mv<N, 3>(m, k, A, B, C, alpha, beta, s, info);
+    }
     if (ta == 0 && !tb && !tri) {
         if (N == 3 && fused3)
             return run_mm_n<N, 0, false, false, true>(m, n, k, A, B, C, alpha, beta, s, info, mode);
