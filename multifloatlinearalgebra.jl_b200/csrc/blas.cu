@@ -316,11 +316,17 @@ struct MVStride {  // odd: the columns of one row fall on all banks
     static constexpr int value = N * MV_ROWS + 1;
 };
 
-template <int N, int TA>
+// RAW stores the chains themselves (no alpha, no beta).  The kernel returns at
+// once when an earlier step of its factorization stopped: *info != 0 and
+// *info <= last.
+template <int N, int TA, bool RAW>
 __global__ void __launch_bounds__(MV_NT)
     mv_kernel(int64_t m, int64_t K, Mat A, Mat X, Mat Y, scal<N> alpha, scal<N> beta, int overwrite,
-              const int *info) {
-    if (info && *info) return;
+              const int *info, int last) {
+    // may be launched as a programmatic dependent (no effect otherwise)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (info && *info != 0 && *info <= last) return;
     extern __shared__ double prod[];  // [2][MV_KB][ST]
     constexpr int ST = MVStride<N>::value;
     const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
@@ -404,6 +410,10 @@ __global__ void __launch_bounds__(MV_NT)
     }
     const int64_t row = row0 + lane;
     if (warp != chain || row >= m) return;
+    if constexpr (RAW) {
+        store_mf<N>(Y.p, 0, Y.ls, row, 0, acc);
+        return;
+    }
     mf<N> r = mul(alpha.get(), acc);
     if (!overwrite) r = add(r, mul(beta.get(), load_mf<N>(Y.p, 0, Y.ls, row, 0)));
     store_mf<N>(Y.p, 0, Y.ls, row, 0, r);
@@ -413,7 +423,7 @@ template <int N, int TA>
 static int run_mv(int64_t m, int64_t k, Mat A, Mat X, Mat Y, const double *alpha,
                   const double *beta, cudaStream_t s, const int *info) {
     constexpr size_t smem = sizeof(double) * 2 * MV_KB * MVStride<N>::value;
-    auto kern = mv_kernel<N, TA>;
+    auto kern = mv_kernel<N, TA, false>;
     static std::atomic<unsigned long long> configured{0};
     if (int rc = set_smem_once((const void *)kern, (int)smem, configured, "mv_kernel attribute"))
         return rc;
@@ -426,8 +436,33 @@ static int run_mv(int64_t m, int64_t k, Mat A, Mat X, Mat Y, const double *alpha
     }
     const int64_t grid = (m + MV_ROWS - 1) / MV_ROWS;
     if (grid > 2147483647LL) return MFLAB_ERR_UNSUPPORTED;
-    kern<<<(unsigned)grid, MV_NT, smem, s>>>(m, k, A, X, Y, al, be, overwrite, info);
+    kern<<<(unsigned)grid, MV_NT, smem, s>>>(m, k, A, X, Y, al, be, overwrite, info, 0x7fffffff);
     return record_cuda_error(cudaGetLastError(), "mv_kernel launch");
+}
+
+template <int N>
+static int run_column_chains(int64_t cols, int64_t k, Mat A, Mat X, Mat Y, cudaStream_t s,
+                             const int *stop, int last) {
+    constexpr size_t smem = sizeof(double) * 2 * MV_KB * MVStride<N>::value;
+    auto kern = mv_kernel<N, 1, true>;
+    static std::atomic<unsigned long long> configured{0};
+    if (int rc = set_smem_once((const void *)kern, (int)smem, configured, "column chains attribute"))
+        return rc;
+    if (cols <= 0) return MFLAB_OK;
+    const int64_t grid = (cols + MV_ROWS - 1) / MV_ROWS;
+    if (grid > 2147483647LL) return MFLAB_ERR_UNSUPPORTED;
+    return launch_programmatic(kern, dim3((unsigned)grid), dim3(MV_NT), smem, s, "column chains",
+                               cols, k, A, X, Y, scal<N>{}, scal<N>{}, 1, stop, last);
+}
+
+int launch_column_chains(int N, int64_t cols, int64_t k, Mat A, Mat X, Mat Y, cudaStream_t s,
+                         const int *stop, int last) {
+    switch (N) {
+    case 2: return run_column_chains<2>(cols, k, A, X, Y, s, stop, last);
+    case 3: return run_column_chains<3>(cols, k, A, X, Y, s, stop, last);
+    case 4: return run_column_chains<4>(cols, k, A, X, Y, s, stop, last);
+    default: return MFLAB_ERR_UNSUPPORTED;
+    }
 }
 
 template <int N>

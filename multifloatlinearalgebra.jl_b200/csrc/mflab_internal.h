@@ -32,6 +32,12 @@ int launch_mm(int N, int ta, bool tb, int tri, bool fused3, int64_t m, int64_t n
 int launch_trmm_mm(int N, int ta, bool tb, int mode, int64_t m, int64_t n, int64_t k, Mat A, Mat B,
                    Mat C, const double *alpha, cudaStream_t s);
 
+// y[j] = the ascending chain sum_r A[r, j] * x[r], r < k, for every column j:
+// one programmatic dependent launch that does nothing when *stop is nonzero
+// and at most `last`.
+int launch_column_chains(int N, int64_t cols, int64_t k, Mat A, Mat X, Mat Y, cudaStream_t s,
+                         const int *stop, int last);
+
 // Triangular solve (trsm.jl semantics); returns an MFLAB_* code.
 int launch_trsm(int N, int side, int uplo, int trans, int diag, int64_t m, int64_t n, Mat A, Mat B,
                 const double *alpha, cudaStream_t s);

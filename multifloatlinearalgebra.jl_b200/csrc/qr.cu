@@ -9,16 +9,13 @@
 // DLAQPS-style panel with delayed updates, norm downdates and panel breaks
 // (qr.jl:450-604), whose end-of-panel update is the matched GEMM kernel.
 //
-// Parallel structure: the work that is independent across columns (trailing
-// reflector applications, the F recurrence, the R row, norm downdates and
-// rebuilds) runs one column per thread; the sequential pieces (a column
-// norm, the pivot decision) run on one CTA.  Norm state lives in device
-// planes so no step needs the host, except the panel-break test of the
-// blocked route, which the host reads once per step.
+// Parallel structure: what the reference's order makes sequential is the
+// additions of a column norm and of each projection chain; one lane adds while
+// the other warps form the quotients, squares and products it adds next.
+// Norm state lives in device planes and a panel break is a device word that
+// the panel's later steps read first, so the host waits once per panel.
 #include "mf_device.cuh"
 #include "mflab_internal.h"
-
-#include <vector>
 
 namespace mfl {
 
@@ -211,30 +208,141 @@ __global__ void qr_finite_kernel(int64_t m, int64_t n, Mat A, int *flag) {
 }
 
 // _qr_make_reflector! (qr.jl:606-622) for column s; tau at tau[l * lt + s].
-// blocked != 0 (the DLAQPS panel, qr.jl:513-515, 530-541): afterwards save
-// A[s,s] to diag, set A[s,s] = 1 and form aux[p] = -tau * sum_rows
-// A[row, bs+p] v[row] for the ls earlier panel columns.
+// blocked != 0 (the DLAQPS panel, qr.jl:513-515): afterwards save A[s,s] to
+// diag and set A[s,s] = 1.
+//
+// The bound is the norm's chain of m - s additions (90 cycles each in x2), so
+// nothing else is left on it.  The reference's running scale is the running
+// maximum of the magnitudes, which eight warps find with a scan: each of 256
+// rows then has its ratio and square at once, and what its row does to the sum
+// is a flag.  The ninth warp's first lane folds tile t in row order while the
+// eight form tile t + 1.  x2, m = 500: 37 us a column, 23 of them the chain;
+// 127 us with one warp for both and the projections on the earlier panel
+// columns behind it (these are now column chains beside the trailing ones).
+constexpr int QRR_TILE = 256, QRR_NT = QRR_TILE + 32;
+enum : unsigned char { QRR_SKIP = 0, QRR_ADD = 1, QRR_RAISE = 2, QRR_FIRST = 3 };
+
 template <int N>
-__global__ void __launch_bounds__(QR_CTA)
+__global__ void __launch_bounds__(QRR_NT)
     qr_reflector_kernel(int64_t m, int64_t s, Mat A, double *tau, int64_t lt, int blocked,
-                        double *diag, int64_t bs, int64_t ls, double *aux) {
-    // the steps of the unblocked loops are programmatic dependents of one
-    // another: wait for the previous grid, let the next one be placed
+                        double *diag, const int *stop) {
+    // every step's kernels are programmatic dependents of one another: wait
+    // for the previous grid, let the next one be placed
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    __shared__ double slead[N];
+    if (stop && *stop != 0 && *stop <= (int)s) return;
+    __shared__ double val[2][N][QRR_TILE];  // squares (QRR_ADD) or ratios (QRR_RAISE)
+    __shared__ unsigned char flag[2][QRR_TILE];
+    __shared__ unsigned plain[2][QRR_TILE / 32];  // rows of a group that only add
+    __shared__ double wmax[QRR_TILE / 32][N], carry[2][N], slead[N];
     __shared__ int go;
-    __shared__ double nbuf[QR_NORM_BUF(N)];
-    const int tid = threadIdx.x;
-    mf<N> scale, sum;
-    if (tid < 32) norm_state_warp<N>(A, m, s, s, nbuf, scale, sum);
-    if (tid == 0) {
+    const unsigned FULL = 0xffffffffu;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const mf<N> one = from_double<N>(1.0), zero = from_double<N>(0.0);
+    const int64_t tiles = (m - s + QRR_TILE - 1) / QRR_TILE;
+    if (tid < N) carry[0][tid] = 0.0;
+    __syncthreads();
+
+    auto produce = [&](int64_t t) {  // warps 0 .. 7
+        const int b = (int)(t & 1);
+        const int64_t r = s + t * QRR_TILE + tid;
+        const mf<N> mag = r < m ? abs_mf(load_mf<N>(A.p, A.ld, A.ls, r, s)) : zero;
+        const bool nz = !iszero(mag);
+        mf<N> pm = mag;  // running maximum within the warp
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            mf<N> o;
+#pragma unroll
+            for (int l = 0; l < N; ++l) o.v[l] = __shfl_up_sync(FULL, pm.v[l], off);
+            if (lane >= off && gt(o, pm)) pm = o;
+        }
+        if (lane == 31)
+#pragma unroll
+            for (int l = 0; l < N; ++l) wmax[warp][l] = pm.v[l];
+        asm volatile("bar.sync 1, %0;" ::"n"(QRR_TILE) : "memory");
+        mf<N> base;  // the maximum before this warp's rows
+#pragma unroll
+        for (int l = 0; l < N; ++l) base.v[l] = carry[b][l];
+        for (int w = 0; w < warp; ++w) {
+            mf<N> o;
+#pragma unroll
+            for (int l = 0; l < N; ++l) o.v[l] = wmax[w][l];
+            if (gt(o, base)) base = o;
+        }
+        mf<N> before;
+#pragma unroll
+        for (int l = 0; l < N; ++l) before.v[l] = __shfl_up_sync(FULL, pm.v[l], 1);
+        if (lane == 0 || gt(base, before)) before = base;
+        unsigned char f = QRR_SKIP;
+        mf<N> x = zero;
+        if (nz) {
+            if (iszero(before)) {
+                f = QRR_FIRST;
+            } else if (gt(mag, before)) {
+                f = QRR_RAISE;
+                x = div(before, mag);
+            } else {
+                f = QRR_ADD;
+                x = div(mag, before);
+                x = mul(x, x);
+            }
+        }
+#pragma unroll
+        for (int l = 0; l < N; ++l) val[b][l][tid] = x.v[l];
+        flag[b][tid] = f;
+        const unsigned p = __ballot_sync(FULL, f == QRR_ADD);
+        if (lane == 0) plain[b][warp] = p;
+        if (tid == QRR_TILE - 1) {
+            if (gt(base, pm)) pm = base;
+#pragma unroll
+            for (int l = 0; l < N; ++l) carry[b ^ 1][l] = pm.v[l];
+        }
+    };
+
+    mf<N> sum = one;
+    if (warp < QRR_TILE / 32) produce(0);
+    for (int64_t t = 0; t < tiles; ++t) {
+        __syncthreads();
+        if (warp == QRR_TILE / 32) {
+            if (lane == 0) {
+                const int b = (int)(t & 1);
+                for (int g = 0; g < QRR_TILE / 32; ++g) {
+                    auto get = [&](int i) {
+                        mf<N> x;
+#pragma unroll
+                        for (int l = 0; l < N; ++l) x.v[l] = val[b][l][g * 32 + i];
+                        return x;
+                    };
+                    if (plain[b][g] == FULL) {
+#pragma unroll 8
+                        for (int i = 0; i < 32; ++i) sum = add(sum, get(i));
+                    } else {
+                        for (int i = 0; i < 32; ++i) {
+                            const unsigned char f = flag[b][g * 32 + i];
+                            if (f == QRR_SKIP) continue;
+                            const mf<N> x = get(i);
+                            if (f == QRR_FIRST) sum = one;
+                            else if (f == QRR_RAISE) sum = add(one, mul(mul(sum, x), x));
+                            else sum = add(sum, x);
+                        }
+                    }
+                }
+            }
+        } else if (t + 1 < tiles) {
+            produce(t + 1);
+        }
+    }
+    __syncthreads();
+    if (tid == QRR_TILE) {
+        mf<N> scale;
+#pragma unroll
+        for (int l = 0; l < N; ++l) scale.v[l] = carry[tiles & 1][l];
         const mf<N> nrm = norm_value(scale, sum);
-        mf<N> t = from_double<N>(0.0);
+        mf<N> t = zero;
         go = 0;
         if (!iszero(nrm)) {
             const mf<N> alpha = load_mf<N>(A.p, A.ld, A.ls, s, s);
-            const mf<N> beta = ge(alpha, from_double<N>(0.0)) ? neg(nrm) : nrm;
+            const mf<N> beta = ge(alpha, zero) ? neg(nrm) : nrm;
             const mf<N> lead = sub(alpha, beta);
             t = div(sub(beta, alpha), beta);
 #pragma unroll
@@ -250,56 +358,55 @@ __global__ void __launch_bounds__(QR_CTA)
         mf<N> lead;
 #pragma unroll
         for (int l = 0; l < N; ++l) lead.v[l] = slead[l];
-        for (int64_t r = s + 1 + tid; r < m; r += QR_CTA)
+        for (int64_t r = s + 1 + tid; r < m; r += QRR_NT)
             store_mf<N>(A.p, A.ld, A.ls, r, s, div(load_mf<N>(A.p, A.ld, A.ls, r, s), lead));
     }
-    if (!blocked) return;
-    __syncthreads();
-    if (tid == 0) {
+    if (blocked && tid == 0) {
         const mf<N> d = load_mf<N>(A.p, A.ld, A.ls, s, s);
 #pragma unroll
         for (int l = 0; l < N; ++l) diag[l] = d.v[l];
-        store_mf<N>(A.p, A.ld, A.ls, s, s, from_double<N>(1.0));
-    }
-    __syncthreads();
-    if (tid < ls) {
-        mf<N> t;
-#pragma unroll
-        for (int l = 0; l < N; ++l) t.v[l] = tau[l * lt + s];
-        mf<N> acc = from_double<N>(0.0);
-        for (int64_t r = s; r < m; ++r)
-            acc = mac<N, false>(acc, load_mf<N>(A.p, A.ld, A.ls, r, bs + tid),
-                                load_mf<N>(A.p, A.ld, A.ls, r, s));
-        const mf<N> a = mul(neg(t), acc);
-#pragma unroll
-        for (int l = 0; l < N; ++l) aux[tid * N + l] = a.v[l];
+        store_mf<N>(A.p, A.ld, A.ls, s, s, one);
     }
 }
 
 // acc folded over rows r0..m-1 in ascending order, acc = acc + X[r,cx] *
 // Y[r,cy], by one warp: the lanes form 32 products at a time, lane 0 adds
 // them in row order (the reference's chain; only the additions are
-// sequential).  All 32 lanes call it; buf holds 32 N doubles of this warp;
-// the result is returned in every lane.
+// sequential) while the next 32 rows' operands are on their way.  All 32
+// lanes call it; buf holds 32 N doubles of this warp; the result is returned
+// in every lane.
 template <int N>
 __device__ mf<N> chain_warp(mf<N> acc, int64_t r0, int64_t m, const Mat &X, int64_t cx,
                             const Mat &Y, int64_t cy, double *buf) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
+    mf<N> x = from_double<N>(0.0), y = x;
+    auto fetch = [&](int64_t r) {
+        if (r < m) {
+            x = load_mf<N>(X.p, X.ld, X.ls, r, cx);
+            y = load_mf<N>(Y.p, Y.ld, Y.ls, r, cy);
+        }
+    };
+    fetch(r0 + lane);
     for (int64_t base = r0; base < m; base += 32) {
-        const int64_t r = base + lane;
-        mf<N> pr = from_double<N>(0.0);
-        if (r < m) pr = mul(load_mf<N>(X.p, X.ld, X.ls, r, cx), load_mf<N>(Y.p, Y.ld, Y.ls, r, cy));
+        const mf<N> pr = mul(x, y);  // of a row past the end: never added
 #pragma unroll
         for (int l = 0; l < N; ++l) buf[l * 32 + lane] = pr.v[l];
         __syncwarp();
+        fetch(base + 32 + lane);
         if (lane == 0) {
-            const int cnt = m - base < 32 ? (int)(m - base) : 32;
-            for (int i = 0; i < cnt; ++i) {
-                mf<N> x;
+            auto term = [&](int i) {
+                mf<N> p;
 #pragma unroll
-                for (int l = 0; l < N; ++l) x.v[l] = buf[l * 32 + i];
-                acc = add(acc, x);
+                for (int l = 0; l < N; ++l) p.v[l] = buf[l * 32 + i];
+                acc = add(acc, p);
+            };
+            const int cnt = m - base < 32 ? (int)(m - base) : 32;
+            if (cnt == 32) {
+#pragma unroll 8
+                for (int i = 0; i < 32; ++i) term(i);
+            } else {
+                for (int i = 0; i < cnt; ++i) term(i);
             }
         }
         __syncwarp();
@@ -352,8 +459,8 @@ __global__ void __launch_bounds__(32 * QR_COL_WARPS)
 // apply_q! (qr.jl:890-956): every reflector in order on one column of D
 template <int N>
 __global__ void __launch_bounds__(32 * QR_COL_WARPS)
-    qr_apply_all_kernel(int64_t m, int64_t r, Mat V, const double *tau, int64_t lt, Mat D,
-                        int64_t nd, int trans) {
+    qr_apply_all_warp_kernel(int64_t m, int64_t r, Mat V, const double *tau, int64_t lt, Mat D,
+                             int64_t nd, int trans) {
     __shared__ double buf[QR_COL_WARPS][32 * N];
     const int w = threadIdx.x >> 5;
     const int64_t c = (int64_t)blockIdx.x * QR_COL_WARPS + w;
@@ -365,6 +472,79 @@ __global__ void __launch_bounds__(32 * QR_COL_WARPS)
         for (int l = 0; l < N; ++l) t.v[l] = tau[l * lt + s];
         if (iszero(t)) continue;
         apply_reflector_col_warp<N>(m, s, V, t, D, c, buf[w]);
+    }
+}
+
+// The same, one CTA per column.  r reflectors are r chains of m - s additions
+// one after another; the ninth warp's first lane runs them while eight warps
+// form the next 256 products, and all nine apply the update.  Taken for up to
+// QR_APPLY_CTAS columns: the chains of CTAs that share an SM share one of its
+// four schedulers (40 of a chain's 90 cycles an addition are issue in x2), so
+// beyond two of them the warp kernel above is the faster one.  x2, m = 500,
+// 40 reflectors, 3 columns: 977 us (1257 us with a warp per column).
+constexpr int64_t QR_APPLY_CTAS = 2 * 148;
+
+template <int N>
+__global__ void __launch_bounds__(QRR_NT)
+    qr_apply_all_kernel(int64_t m, int64_t r, Mat V, const double *tau, int64_t lt, Mat D,
+                        int trans) {
+    __shared__ double buf[2][N][QRR_TILE];
+    __shared__ double sproj[N];
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int64_t c = blockIdx.x;
+    for (int64_t i = 0; i < r; ++i) {
+        const int64_t s = trans ? i : r - 1 - i;
+        mf<N> t;
+#pragma unroll
+        for (int l = 0; l < N; ++l) t.v[l] = tau[l * lt + s];
+        if (iszero(t)) continue;  // the same in every thread
+        const int64_t r0 = s + 1, tiles = (m - r0 + QRR_TILE - 1) / QRR_TILE;
+        auto produce = [&](int64_t b) {
+            const int64_t row = r0 + b * QRR_TILE + tid;
+            if (row >= m) return;
+            const mf<N> p = mul(load_mf<N>(V.p, V.ld, V.ls, row, s),
+                                load_mf<N>(D.p, D.ld, D.ls, row, c));
+#pragma unroll
+            for (int l = 0; l < N; ++l) buf[b & 1][l][tid] = p.v[l];
+        };
+        mf<N> acc;
+        if (tid == QRR_TILE) acc = load_mf<N>(D.p, D.ld, D.ls, s, c);
+        if (warp < QRR_TILE / 32 && tiles > 0) produce(0);
+        for (int64_t b = 0; b < tiles; ++b) {
+            __syncthreads();
+            if (tid == QRR_TILE) {
+                auto term = [&](int k) {
+                    mf<N> p;
+#pragma unroll
+                    for (int l = 0; l < N; ++l) p.v[l] = buf[b & 1][l][k];
+                    acc = add(acc, p);
+                };
+                const int64_t left = m - r0 - b * QRR_TILE;
+                const int cnt = left < QRR_TILE ? (int)left : QRR_TILE;
+                int k = 0;
+                for (; k + 8 <= cnt; k += 8)
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) term(k + q);
+                for (; k < cnt; ++k) term(k);
+            } else if (warp < QRR_TILE / 32 && b + 1 < tiles) {
+                produce(b + 1);
+            }
+        }
+        if (tid == QRR_TILE) {
+            const mf<N> proj = mul(acc, t);
+#pragma unroll
+            for (int l = 0; l < N; ++l) sproj[l] = proj.v[l];
+            store_mf<N>(D.p, D.ld, D.ls, s, c, sub(load_mf<N>(D.p, D.ld, D.ls, s, c), proj));
+        }
+        __syncthreads();
+        mf<N> proj;
+#pragma unroll
+        for (int l = 0; l < N; ++l) proj.v[l] = sproj[l];
+        for (int64_t row = r0 + tid; row < m; row += QRR_NT)
+            store_mf<N>(D.p, D.ld, D.ls, row, c,
+                        submul(load_mf<N>(D.p, D.ld, D.ls, row, c),
+                               load_mf<N>(V.p, V.ld, V.ls, row, s), proj));
+        __syncthreads();  // the column and sproj before the next reflector
     }
 }
 
@@ -510,7 +690,10 @@ constexpr int QR_PIVOT_CTA = 1024;
 template <int N>
 __global__ void __launch_bounds__(QR_PIVOT_CTA)
     qr_dlaqps_pivot_kernel(int64_t m, int64_t step, int64_t bs, int64_t ls, Mat A, int64_t *perm,
-                           QRNorms<N> S, Mat F) {
+                           QRNorms<N> S, Mat F, const int *stop) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (*stop != 0 && *stop <= (int)step) return;
     __shared__ double sval[N][QR_PIVOT_CTA];
     __shared__ int64_t sidx[QR_PIVOT_CTA];
     const int tid = threadIdx.x;
@@ -530,7 +713,9 @@ __global__ void __launch_bounds__(QR_PIVOT_CTA)
     for (int l = 0; l < N; ++l) sval[l][tid] = bv.v[l];
     sidx[tid] = bi;
     __syncthreads();
-    for (int s = QR_PIVOT_CTA / 2; s > 0; s >>= 1) {
+    int width = 32;  // threads that hold a column
+    while (width < QR_PIVOT_CTA && width < S.n - step) width <<= 1;
+    for (int s = width / 2; s > 0; s >>= 1) {
         if (tid < s && sidx[tid + s] >= 0) {
             const int64_t ia = sidx[tid], ib = sidx[tid + s];
             mf<N> va, vb;
@@ -572,6 +757,7 @@ __global__ void __launch_bounds__(QR_PIVOT_CTA)
     if (ls > 0)
         for (int64_t r = step + tid; r < m; r += QR_PIVOT_CTA) {
             mf<N> corr = from_double<N>(0.0);
+#pragma unroll 4
             for (int64_t p = 0; p < ls; ++p)
                 corr = mac<N, false>(corr, load_mf<N>(A.p, A.ld, A.ls, r, bs + p),
                                      load_mf<N>(F.p, F.ld, F.ls, p, step));
@@ -579,47 +765,90 @@ __global__ void __launch_bounds__(QR_PIVOT_CTA)
         }
 }
 
-// DLAQPS step body, one trailing column per thread (qr.jl:517-576): the new
-// F row (gemv! trans = :T, then the correction through aux), the R row, and
-// the norm downdate; any column left unreliable raises *unreliable
+// DLAQPS step body after the column chains acc[j] = sum_r A[r, bs+j] v[r]
+// (gemv! trans = :T), one trailing column per thread (qr.jl:517-576): aux[p]
+// = -tau acc[p] of the earlier panel columns, the new F row, the R row and
+// the norm downdate.  A column left unreliable ends the panel after this
+// step: *stop = step + 1, read by every later step of the panel.
 template <int N>
-__global__ void __launch_bounds__(32 * QR_COL_WARPS)
+__global__ void __launch_bounds__(QR_COLS_PER_CTA)
     qr_dlaqps_columns_kernel(int64_t m, int64_t step, int64_t bs, int64_t ls, Mat A,
-                             const double *tau, int64_t lt, const double *aux, Mat F, QRNorms<N> S,
-                             scal<N> floor_, int *unreliable) {
-    __shared__ double buf[QR_COL_WARPS][32 * N];
-    const int w = threadIdx.x >> 5;
-    const int64_t c = step + 1 + (int64_t)blockIdx.x * QR_COL_WARPS + w;
-    if (c >= S.n) return;  // whole warps leave together
+                             const double *tau, int64_t lt, const double *chains, Mat F,
+                             QRNorms<N> S, scal<N> floor_, int *stop) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (*stop != 0 && *stop <= (int)step) return;
+    // the panel's entries the correction loops read, staged so that no load
+    // waits inside a chain
+    __shared__ double aux[QR_BLOCK][N], row[QR_BLOCK][N];
+    __shared__ double Fs[QR_BLOCK][N][QR_COLS_PER_CTA];
+    const int tid = threadIdx.x;
+    const int64_t c = step + 1 + (int64_t)blockIdx.x * QR_COLS_PER_CTA + tid;
     mf<N> t;
 #pragma unroll
     for (int l = 0; l < N; ++l) t.v[l] = tau[l * lt + step];
-    // gemv! trans = :T chain of column c with the reflector (rows step..m-1)
-    const mf<N> acc = chain_warp<N>(from_double<N>(0.0), step, m, A, c, A, step, buf[w]);
-    if ((threadIdx.x & 31) != 0) return;
-    mf<N> f = mul(t, acc);
+    if (tid <= ls) {
+        const mf<N> x = load_mf<N>(A.p, A.ld, A.ls, step, bs + tid);
+#pragma unroll
+        for (int l = 0; l < N; ++l) row[tid][l] = x.v[l];
+    }
+    if (tid < ls) {
+        const mf<N> a = mul(neg(t), load_mf<N>(chains, 0, S.n, tid, 0));
+#pragma unroll
+        for (int l = 0; l < N; ++l) aux[tid][l] = a.v[l];
+    }
+    mf<N> chain = from_double<N>(0.0), old = chain;
+    if (c < S.n) {
+        chain = load_mf<N>(chains, 0, S.n, c - bs, 0);
+        old = load_mf<N>(A.p, A.ld, A.ls, step, c);
+#pragma unroll 4
+        for (int64_t p = 0; p < ls; ++p) {
+            const mf<N> f = load_mf<N>(F.p, F.ld, F.ls, p, c);
+#pragma unroll
+            for (int l = 0; l < N; ++l) Fs[p][l][tid] = f.v[l];
+        }
+    }
+    __syncthreads();
+    if (c >= S.n) return;
+    auto Fat = [&](int64_t p) {
+        mf<N> f;
+#pragma unroll
+        for (int l = 0; l < N; ++l) f.v[l] = Fs[p][l][tid];
+        return f;
+    };
+    auto get = [&](const double *v) {
+        mf<N> x;
+#pragma unroll
+        for (int l = 0; l < N; ++l) x.v[l] = v[l];
+        return x;
+    };
+    mf<N> f = mul(t, chain);
     if (ls > 0) {
         mf<N> corr = from_double<N>(0.0);
-        for (int64_t p = 0; p < ls; ++p) {
-            mf<N> a;
-#pragma unroll
-            for (int l = 0; l < N; ++l) a.v[l] = aux[p * N + l];
-            corr = mac<N, false>(corr, load_mf<N>(F.p, F.ld, F.ls, p, c), a);
-        }
+        for (int64_t p = 0; p < ls; ++p) corr = mac<N, false>(corr, Fat(p), get(aux[p]));
         f = add(f, corr);
     }
     store_mf<N>(F.p, F.ld, F.ls, ls, c, f);
     mf<N> corr = from_double<N>(0.0);
-    for (int64_t p = 0; p <= ls; ++p)
-        corr = mac<N, false>(corr, load_mf<N>(A.p, A.ld, A.ls, step, bs + p),
-                             load_mf<N>(F.p, F.ld, F.ls, p, c));
-    store_mf<N>(A.p, A.ld, A.ls, step, c, sub(load_mf<N>(A.p, A.ld, A.ls, step, c), corr));
+    for (int64_t p = 0; p < ls; ++p) corr = mac<N, false>(corr, get(row[p]), Fat(p));
+    corr = mac<N, false>(corr, get(row[ls]), f);
+    store_mf<N>(A.p, A.ld, A.ls, step, c, sub(old, corr));
     if (!iszero(t)) update_norm_col<N>(m, step, c, A, S, floor_.get(), F, bs, ls + 1);
-    if (S.dirty[c]) atomicExch(unreliable, 1);
+    if (S.dirty[c]) atomicExch(stop, (int)step + 1);
 }
 
-__global__ void qr_restore_diag_kernel(int N, Mat A, int64_t s, const double *diag) {
-    for (int l = 0; l < N; ++l) A.p[l * A.ls + s * A.ld + s] = diag[l];
+// the panel's diagonal entries back in place of the ones, for the steps that ran
+__global__ void qr_restore_diag_kernel(int N, Mat A, int64_t bs, int64_t req, const double *diag,
+                                       const int *stop) {
+    const int64_t actual = *stop ? *stop - bs : req;
+    const int64_t i = threadIdx.x;
+    if (i >= actual) return;
+    for (int l = 0; l < N; ++l) A.p[l * A.ls + (bs + i) * A.ld + bs + i] = diag[i * N + l];
+}
+
+__global__ void qr_identity_kernel(int64_t n, int64_t *perm) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) perm[i] = i + 1;
 }
 
 // numerical_rank (qr.jl:863-888)
@@ -643,9 +872,9 @@ template <int N>
 static int qr_n(mflab_handle *h, cudaStream_t s, int pivoted, int64_t m, int64_t n, Mat A,
                 double *tau, int64_t lt, int64_t *perm, int *info) {
     const int64_t r = m < n ? m : n;
-    // scratch: norm planes, F (QR_BLOCK x n), aux, diag, flags
+    // scratch: norm planes, F (QR_BLOCK x n), column chains, panel diagonal, flags
     const size_t nn = (size_t)(n > 0 ? n : 1);
-    const size_t doubles = 2 * N * nn + (size_t)N * QR_BLOCK * nn + QR_BLOCK * N + N;
+    const size_t doubles = 2 * N * nn + (size_t)N * QR_BLOCK * nn + N * nn + QR_BLOCK * N;
     const size_t bytes = doubles * sizeof(double) + (nn + 4) * sizeof(int);
     int rc = mflab_reserve_scratch(h, bytes);
     if (rc) return rc;
@@ -653,11 +882,10 @@ static int qr_n(mflab_handle *h, cudaStream_t s, int pivoted, int64_t m, int64_t
     QRNorms<N> S{base, base + N * nn, nullptr, n};
     double *Fp = base + 2 * N * nn;
     const Mat F{Fp, QR_BLOCK, (int64_t)(QR_BLOCK * nn)};
-    double *aux = Fp + (size_t)N * QR_BLOCK * nn;
-    double *diag = aux + QR_BLOCK * N;
-    S.dirty = (int *)(diag + N);
+    double *chains = Fp + (size_t)N * QR_BLOCK * nn;
+    double *diag = chains + N * nn;
+    S.dirty = (int *)(diag + QR_BLOCK * N);
     int *flag = S.dirty + nn;
-    int *hflag = nullptr;
 
     cudaError_t e = cudaSuccess;
     for (int l = 0; l < N; ++l) {
@@ -666,12 +894,7 @@ static int qr_n(mflab_handle *h, cudaStream_t s, int pivoted, int64_t m, int64_t
     }
     // identity permutation, finiteness
     {
-        std::vector<int64_t> id(n);
-        for (int64_t i = 0; i < n; ++i) id[i] = i + 1;
-        if (n > 0) {
-            e = cudaMemcpyAsync(perm, id.data(), n * sizeof(int64_t), cudaMemcpyHostToDevice, s);
-            if (e != cudaSuccess) return record_cuda_error(e, "qr perm");
-        }
+        if (n > 0) qr_identity_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, perm);
         qr_finite_kernel_init<<<1, 1, 0, s>>>(flag);
         const int64_t g = (m * n + 255) / 256;
         qr_finite_kernel<N><<<(unsigned)(g < 1184 ? (g > 0 ? g : 1) : 1184), 256, 0, s>>>(m, n, A, flag);
@@ -686,13 +909,11 @@ static int qr_n(mflab_handle *h, cudaStream_t s, int pivoted, int64_t m, int64_t
             return record_cuda_error(e, "qr info");
         }
     }
-    (void)hflag;
     if (!pivoted) {
         // each step's kernels are programmatic dependent launches
         for (int64_t st = 0; st < r; ++st) {
-            int rc = launch_programmatic(qr_reflector_kernel<N>, dim3(1), dim3(QR_CTA), 0, s,
-                                         "qr reflector", m, st, A, tau, lt, 0, nullptr, 0, 0,
-                                         nullptr);
+            int rc = launch_programmatic(qr_reflector_kernel<N>, dim3(1), dim3(QRR_NT), 0, s,
+                                         "qr reflector", m, st, A, tau, lt, 0, nullptr, nullptr);
             if (rc) return rc;
             if (st + 1 < n) {
                 rc = launch_programmatic(qr_apply_kernel<N>, dim3(warp_col_grid(n - st - 1)),
@@ -720,8 +941,8 @@ static int qr_n(mflab_handle *h, cudaStream_t s, int pivoted, int64_t m, int64_t
                 int rc = launch_programmatic(qr_hybrid_pivot_kernel<N>, dim3(1), dim3(QR_CTA), 0,
                                              s, "qr pivot", m, st, A, perm, S, om);
                 if (rc == MFLAB_OK)
-                    rc = launch_programmatic(qr_reflector_kernel<N>, dim3(1), dim3(QR_CTA), 0, s,
-                                             "qr reflector", m, st, A, tau, lt, 0, nullptr, 0, 0,
+                    rc = launch_programmatic(qr_reflector_kernel<N>, dim3(1), dim3(QRR_NT), 0, s,
+                                             "qr reflector", m, st, A, tau, lt, 0, nullptr,
                                              nullptr);
                 if (rc == MFLAB_OK && st + 1 < n) {
                     rc = launch_programmatic(qr_apply_kernel<N>, dim3(warp_col_grid(n - st - 1)),
@@ -736,38 +957,49 @@ static int qr_n(mflab_handle *h, cudaStream_t s, int pivoted, int64_t m, int64_t
                 if (rc) return rc;
             }
         } else {
-            e = cudaMallocHost(&hflag, sizeof(int));
-            if (e != cudaSuccess) return record_cuda_error(e, "qr host flag");
             int64_t bs = 0;
             rc = MFLAB_OK;
             while (bs < r && rc == MFLAB_OK) {
                 const int64_t req = (r - bs) < QR_BLOCK ? (r - bs) : QR_BLOCK;
                 for (int l = 0; l < N && e == cudaSuccess; ++l)
                     e = cudaMemsetAsync(Fp + l * F.ls, 0, QR_BLOCK * nn * sizeof(double), s);
+                if (e == cudaSuccess) e = cudaMemsetAsync(flag, 0, sizeof(int), s);
                 if (e != cudaSuccess) {
                     rc = record_cuda_error(e, "qr F");
                     break;
                 }
-                int64_t actual = 0;
-                for (int64_t ls = 0; ls < req; ++ls) {
+                // the whole panel is issued; after a break its later steps
+                // return at once, and the host reads how far it came
+                for (int64_t ls = 0; ls < req && rc == MFLAB_OK; ++ls) {
                     const int64_t st = bs + ls;
-                    qr_dlaqps_pivot_kernel<N><<<1, QR_PIVOT_CTA, 0, s>>>(m, st, bs, ls, A, perm, S, F);
-                    qr_reflector_kernel<N><<<1, QR_CTA, 0, s>>>(m, st, A, tau, lt, 1, diag, bs, ls, aux);
-                    qr_finite_kernel_init<<<1, 1, 0, s>>>(flag);
-                    if (st + 1 < n)
-                        qr_dlaqps_columns_kernel<N><<<warp_col_grid(n - st - 1), 32 * QR_COL_WARPS, 0, s>>>(
-                            m, st, bs, ls, A, tau, lt, aux, F, S, fl, flag);
-                    qr_restore_diag_kernel<<<1, 1, 0, s>>>(N, A, st, diag);
-                    actual = ls + 1;
-                    e = cudaMemcpyAsync(hflag, flag, sizeof(int), cudaMemcpyDeviceToHost, s);
-                    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-                    if (e != cudaSuccess) {
-                        rc = record_cuda_error(e, "qr panel flag");
-                        break;
+                    rc = launch_programmatic(qr_dlaqps_pivot_kernel<N>, dim3(1), dim3(QR_PIVOT_CTA),
+                                             0, s, "qr panel pivot", m, st, bs, ls, A, perm, S, F,
+                                             (const int *)flag);
+                    if (rc == MFLAB_OK)
+                        rc = launch_programmatic(qr_reflector_kernel<N>, dim3(1), dim3(QRR_NT), 0,
+                                                 s, "qr panel reflector", m, st, A, tau, lt, 1,
+                                                 diag + ls * N, (const int *)flag);
+                    if (rc == MFLAB_OK && st + 1 < n) {
+                        // every panel and trailing column (the step's own is unused)
+                        rc = launch_column_chains(N, n - bs, m - st, A.at(st, bs), A.at(st, st),
+                                                  Mat{chains, n, n}, s, flag, (int)st);
+                        if (rc == MFLAB_OK)
+                            rc = launch_programmatic(
+                                qr_dlaqps_columns_kernel<N>, dim3(col_grid(n - st - 1)),
+                                dim3(QR_COLS_PER_CTA), 0, s, "qr panel columns", m, st, bs, ls, A,
+                                (const double *)tau, lt, (const double *)chains, F, S, fl, flag);
                     }
-                    if (*hflag) break;
                 }
                 if (rc) break;
+                qr_restore_diag_kernel<<<1, QR_BLOCK, 0, s>>>(N, A, bs, req, diag, flag);
+                int stopped = 0;
+                e = cudaMemcpyAsync(&stopped, flag, sizeof(int), cudaMemcpyDeviceToHost, s);
+                if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+                if (e != cudaSuccess) {
+                    rc = record_cuda_error(e, "qr panel flag");
+                    break;
+                }
+                const int64_t actual = stopped ? stopped - bs : req;
                 const int64_t be = bs + actual;
                 if (be < m && be < n) {
                     const double mone[4] = {-1.0, 0.0, 0.0, 0.0}, one[4] = {1.0, 0.0, 0.0, 0.0};
@@ -779,15 +1011,23 @@ static int qr_n(mflab_handle *h, cudaStream_t s, int pivoted, int64_t m, int64_t
                     qr_norm_init_kernel<N><<<norm_grid(n - be), 32 * QR_NORM_WARPS, 0, s>>>(m, be, be, A, S);
                 bs = be;
             }
-            cudaFreeHost(hflag);
             if (rc) return rc;
         }
     }
-    const int zero = 0;
-    e = cudaMemcpyAsync(info, &zero, sizeof(int), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    e = cudaMemsetAsync(info, 0, sizeof(int), s);
     if (e != cudaSuccess) return record_cuda_error(e, "qr info");
     return record_cuda_error(cudaGetLastError(), "qr launch");
+}
+
+template <int N>
+static int apply_q_n(int64_t m, int64_t r, Mat F, const double *tau, int64_t lst, Mat D, int64_t nd,
+                     int trans, cudaStream_t s) {
+    if (nd <= QR_APPLY_CTAS)
+        qr_apply_all_kernel<N><<<(unsigned)nd, QRR_NT, 0, s>>>(m, r, F, tau, lst, D, trans);
+    else
+        qr_apply_all_warp_kernel<N><<<warp_col_grid(nd), 32 * QR_COL_WARPS, 0, s>>>(
+            m, r, F, tau, lst, D, nd, trans);
+    return record_cuda_error(cudaGetLastError(), "apply_q launch");
 }
 
 }  // namespace mfl
@@ -825,14 +1065,11 @@ extern "C" int mflab_apply_q(mflab_handle *h, void *stream, int limbs, int trans
     if (mfl::views_overlap(D, ldd, lsd, m, nd, limbs, F, ldf, lsf, m, r)) return MFLAB_ERR_ALIAS;
     const Mat Fm{(double *)F, ldf, lsf}, Dm{D, ldd, lsd};
     cudaStream_t s = (cudaStream_t)stream;
-    const unsigned g = mfl::warp_col_grid(nd);
-    const unsigned bt = 32 * mfl::QR_COL_WARPS;
     switch (limbs) {
-    case 2: mfl::qr_apply_all_kernel<2><<<g, bt, 0, s>>>(m, r, Fm, tau, lst, Dm, nd, trans); break;
-    case 3: mfl::qr_apply_all_kernel<3><<<g, bt, 0, s>>>(m, r, Fm, tau, lst, Dm, nd, trans); break;
-    default: mfl::qr_apply_all_kernel<4><<<g, bt, 0, s>>>(m, r, Fm, tau, lst, Dm, nd, trans); break;
+    case 2: return mfl::apply_q_n<2>(m, r, Fm, tau, lst, Dm, nd, trans, s);
+    case 3: return mfl::apply_q_n<3>(m, r, Fm, tau, lst, Dm, nd, trans, s);
+    default: return mfl::apply_q_n<4>(m, r, Fm, tau, lst, Dm, nd, trans, s);
     }
-    return mfl::record_cuda_error(cudaGetLastError(), "apply_q launch");
 }
 
 extern "C" int mflab_qr_numerical_rank(mflab_handle *h, void *stream, int limbs, int64_t m,
