@@ -11,8 +11,11 @@
 //     the diagonal), broadcasts it through shared memory, and every later row
 //     applies its term k.  Each row thus receives its terms in the reference's
 //     ascending order while the rows progress in parallel.
+//   * trsm_left_warp: the same with the rows over the lanes of a warp, for
+//     triangles of at most 64 rows (LU's U12 block).
+//   * trsm_left_backward_cta: backward substitution, one CTA per column.
 //   * trsm_left_thread: one thread per right-hand-side column, the plain
-//     serial loop (used when the triangle is short, e.g. LU's U12 block).
+//     serial loop (many columns of a backward substitution).
 //   * trsm_right_thread: one thread per row of B, the plain serial loop (the
 //     Cholesky panel solve A21 <- A21 / L11^T).
 #include "mf_device.cuh"
@@ -34,7 +37,11 @@ __global__ void scale_kernel(int64_t m, int64_t n, Mat B, scal<N> alpha) {
     store_mf<N>(B.p, B.ld, B.ls, r, c, mul(v, alpha.get()));
 }
 
-// one CTA per column; NT threads; each thread owns up to MAXR rows
+// one CTA per column; NT threads; each thread owns up to MAXR rows.  A step is
+// a division, a CTA barrier and the rows' multiply-subtracts; the coefficients
+// of the next step (the diagonal among them, for the row it finalises) are
+// loaded behind the ones just used.  x2, n = 2048, 64 columns: 4200 us
+// (4711 us with the loads inside the step).
 template <int N, int NT, int MAXR>
 __global__ void __launch_bounds__(NT) trsm_left_cta(int64_t m, int64_t n, Mat A, Mat B,
                                                     bool eff_lower, bool transposed, bool unit,
@@ -44,25 +51,34 @@ __global__ void __launch_bounds__(NT) trsm_left_cta(int64_t m, int64_t n, Mat A,
     const int64_t col = blockIdx.x;
     if (col >= n) return;
     const int t = threadIdx.x;
-    mf<N> v[MAXR];
+    mf<N> v[MAXR], coef[MAXR];
+    auto fetch = [&](int q, int64_t k) {
+        const int64_t r = t + (int64_t)q * NT;
+        if (r < m && (eff_lower ? r >= k && k < m : r <= k && k >= 0) && !(unit && r == k))
+            coef[q] = tri_coef<N>(A, r, k, transposed);
+    };
+    const int64_t k0 = eff_lower ? 0 : m - 1;
 #pragma unroll
     for (int q = 0; q < MAXR; ++q) {
         int64_t r = t + (int64_t)q * NT;
         v[q] = r < m ? load_mf<N>(B.p, B.ld, B.ls, r, col) : from_double<N>(0.0);
+        coef[q] = from_double<N>(1.0);
+        fetch(q, k0);
     }
     for (int64_t s = 0; s < m; ++s) {
         const int64_t k = eff_lower ? s : m - 1 - s;  // row finalised at this step
+        const int64_t kn = eff_lower ? k + 1 : k - 1;
         const int slot = (int)(s & 1);
         if ((k % NT) == t) {
             const int qk = (int)(k / NT);
-            mf<N> x;
+            mf<N> x, d;
 #pragma unroll
             for (int q = 0; q < MAXR; ++q)
-                if (q == qk) x = v[q];
-            if (!unit) x = div(x, load_mf<N>(A.p, A.ld, A.ls, k, k));
-#pragma unroll
-            for (int q = 0; q < MAXR; ++q)
-                if (q == qk) v[q] = x;
+                if (q == qk) {
+                    x = v[q];
+                    d = coef[q];
+                }
+            if (!unit) x = div(x, d);
             store_mf<N>(B.p, B.ld, B.ls, k, col, x);
 #pragma unroll
             for (int l = 0; l < N; ++l) xs[slot][l] = x.v[l];
@@ -75,52 +91,181 @@ __global__ void __launch_bounds__(NT) trsm_left_cta(int64_t m, int64_t n, Mat A,
         for (int q = 0; q < MAXR; ++q) {
             const int64_t r = t + (int64_t)q * NT;
             const bool later = eff_lower ? (r > k) : (r < k);
-            if (r < m && later) v[q] = submul(v[q], tri_coef<N>(A, r, k, transposed), xk);
+            if (r < m && later) {
+                v[q] = submul(v[q], coef[q], xk);
+                fetch(q, kn);
+            }
         }
     }
 }
 
+// Forward substitution of a triangle of at most 64 rows: W lanes per column, RPL
+// rows per lane, the triangle staged in shared memory row-contiguous.  Row k's
+// lane finalises X[k] and broadcasts it; the rows below apply their term k.
+// A column of 16 rows is 16 steps of a broadcast and a multiply-subtract.
+// x4, 16 unit rows, 685 columns: about 7 us (77 us with a thread per column
+// whose 120 terms wait for their loads one by one).
+constexpr int TRSW_NT = 128;
+
+template <int N, int W, int RPL>
+__global__ void __launch_bounds__(TRSW_NT)
+    trsm_left_warp(int m, int64_t n, Mat A, Mat B, bool transposed, bool unit, const int *info) {
+    if (info && *info) return;
+    extern __shared__ double tri[];  // [N][m][m]: tri[(l*m + k)*m + row], row >= k
+    for (int e = threadIdx.x; e < m * m; e += TRSW_NT) {
+        const int i = e % m, j = e / m;
+        const int row = transposed ? j : i, k = transposed ? i : j;  // op(A)[row, k]
+        if (row < k || (unit && row == k)) continue;
+        const mf<N> a = tri_coef<N>(A, row, k, transposed);
+#pragma unroll
+        for (int l = 0; l < N; ++l) tri[(l * m + k) * m + row] = a.v[l];
+    }
+    __syncthreads();
+    const int sub = threadIdx.x % W;
+    const int64_t col = (int64_t)blockIdx.x * (TRSW_NT / W) + threadIdx.x / W;
+    const bool in = col < n;  // the lanes of a warp stay together
+    auto coef = [&](int row, int k) {
+        mf<N> a;
+#pragma unroll
+        for (int l = 0; l < N; ++l) a.v[l] = tri[(l * m + k) * m + row];
+        return a;
+    };
+    mf<N> v[RPL];
+#pragma unroll
+    for (int q = 0; q < RPL; ++q) {
+        const int row = sub + q * W;
+        v[q] = in && row < m ? load_mf<N>(B.p, B.ld, B.ls, row, col) : from_double<N>(0.0);
+    }
+#pragma unroll
+    for (int qk = 0; qk < RPL; ++qk) {
+        for (int kl = 0; kl < W; ++kl) {
+            const int k = qk * W + kl;
+            if (k >= m) break;
+            if (!unit && sub == kl) v[qk] = div(v[qk], coef(k, k));
+            mf<N> x;
+#pragma unroll
+            for (int l = 0; l < N; ++l) x.v[l] = __shfl_sync(0xffffffffu, v[qk].v[l], kl, W);
+#pragma unroll
+            for (int q = 0; q < RPL; ++q) {
+                const int row = sub + q * W;
+                if (q >= qk && row > k && row < m) v[q] = submul(v[q], coef(row, k), x);
+            }
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < RPL; ++q) {
+        const int row = sub + q * W;
+        if (in && row < m) store_mf<N>(B.p, B.ld, B.ls, row, col, v[q]);
+    }
+}
+
+template <int N>
+static int run_trsm_left_warp(int64_t m, int64_t n, Mat A, Mat B, bool transposed, bool unit,
+                              cudaStream_t s, const int *info) {
+    const size_t smem = (size_t)N * m * m * sizeof(double);
+    const int w = m <= 16 ? 16 : 32;
+    const int64_t grid = (n + TRSW_NT / w - 1) / (TRSW_NT / w);
+    if (grid > 2147483647LL) return MFLAB_ERR_UNSUPPORTED;
+    auto launch = [&](auto kern, std::atomic<unsigned long long> &configured) -> int {
+        if (int rc = set_smem_once((const void *)kern, N * 64 * 64 * (int)sizeof(double),
+                                   configured, "trsm left warp attribute"))
+            return rc;
+        kern<<<(unsigned)grid, TRSW_NT, smem, s>>>((int)m, n, A, B, transposed, unit, info);
+        return record_cuda_error(cudaGetLastError(), "trsm left warp");
+    };
+    static std::atomic<unsigned long long> done[3];
+    if (m <= 16) return launch(trsm_left_warp<N, 16, 1>, done[0]);
+    if (m <= 32) return launch(trsm_left_warp<N, 32, 1>, done[1]);
+    return launch(trsm_left_warp<N, 32, 2>, done[2]);
+}
+
 // Backward substitution (effective upper, left side) in the reference order:
 // row r's chain v = B[r]; v -= coef(r,k) * X[k] for k = r+1..m-1 ascending.
-// One CTA per right-hand-side column: the products of row r are formed by all
-// threads into shared memory, thread 0 runs the subtraction chain and the
-// division.  The column is read from and written to global memory.
-template <int N, int NT>
-__global__ void __launch_bounds__(NT) trsm_left_backward_cta(int64_t m, int64_t n, Mat A, Mat B,
-                                                             bool transposed, bool unit,
-                                                             const int *info) {
+// X[r+1] enters row r's chain first, so a column is one chain of m(m-1)/2
+// subtractions (about 92 / 220 / 340 cycles each in x2 / x3 / x4): nothing but
+// that chain is left on the critical path.  One CTA per column; one warp's
+// first lane runs the chain and the divisions, eight warps form the products
+// of the next 256 terms, across the row's end too: only the product with the
+// unknown just found is the chain's own (its slot holds the coefficient).  The
+// chain warp's place rotates over the schedulers with the CTA.  x2, n = 2048,
+// 64 columns: 101 ms (105.2 ms with the products of a row formed between
+// two barriers before its chain).
+constexpr int TRSB_TILE = 256, TRSB_NT = TRSB_TILE + 32, TRSB_SMS = 148;
+
+template <int N>
+__global__ void __launch_bounds__(TRSB_NT)
+    trsm_left_backward_cta(int64_t m, int64_t n, Mat A, Mat B, bool transposed, bool unit,
+                           const int *info) {
     if (info && *info) return;
-    extern __shared__ double prod[];  // [m][N]
+    __shared__ double prod[2][TRSB_TILE][N];
+    __shared__ double head[2][2][N];  // right-hand side and diagonal of a row
     const int64_t col = blockIdx.x;
     if (col >= n) return;
-    const int t = threadIdx.x;
-    for (int64_t r = m - 1; r >= 0; --r) {
-        for (int64_t k = r + 1 + t; k < m; k += NT) {
-            const mf<N> p = mul(tri_coef<N>(A, r, k, transposed), load_mf<N>(B.p, B.ld, B.ls, k, col));
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int chain = (int)((blockIdx.x + blockIdx.x / TRSB_SMS) % 4);
+    const int slot = (warp - (warp > chain ? 1 : 0)) * 32 + lane;  // of a producing thread
+    auto slabs = [&](int64_t r) { return (m - 1 - r + TRSB_TILE - 1) / TRSB_TILE; };
+    auto produce = [&](int64_t r, int64_t j, int b) {
+        const int64_t k = r + 1 + j * TRSB_TILE + slot;
+        if (k < m) {
+            mf<N> p = tri_coef<N>(A, r, k, transposed);
+            if (k > r + 1) p = mul(p, load_mf<N>(B.p, B.ld, B.ls, k, col));
 #pragma unroll
-            for (int l = 0; l < N; ++l) prod[k * N + l] = p.v[l];
+            for (int l = 0; l < N; ++l) prod[b][slot][l] = p.v[l];
         }
-        __syncthreads();
-        if (t == 0) {
-            // the chain of subtractions is the row's latency; the product of
-            // the next term is read from shared memory while the current one
-            // is subtracted
-            mf<N> v = load_mf<N>(B.p, B.ld, B.ls, r, col);
-            mf<N> pn;
+        if (j == 0 && slot >= TRSB_TILE - 2) {
+            const int which = slot - (TRSB_TILE - 2);
+            if (which == 0 || !unit) {
+                const mf<N> x = which == 0 ? load_mf<N>(B.p, B.ld, B.ls, r, col)
+                                           : load_mf<N>(A.p, A.ld, A.ls, r, r);
 #pragma unroll
-            for (int l = 0; l < N; ++l) pn.v[l] = r + 1 < m ? prod[(r + 1) * N + l] : 0.0;
-            for (int64_t k = r + 1; k < m; ++k) {
-                const mf<N> p = pn;
-                if (k + 1 < m) {
-#pragma unroll
-                    for (int l = 0; l < N; ++l) pn.v[l] = prod[(k + 1) * N + l];
-                }
-                v = sub(v, p);
+                for (int l = 0; l < N; ++l) head[b][which][l] = x.v[l];
             }
-            if (!unit) v = div(v, load_mf<N>(A.p, A.ld, A.ls, r, r));
-            store_mf<N>(B.p, B.ld, B.ls, r, col, v);
         }
+    };
+    mf<N> v = from_double<N>(0.0), x = v, d = v;
+    int64_t r = m - 1, j = 0;
+    if (warp != chain) produce(r, 0, 0);
+    for (int b = 0;; b ^= 1) {
         __syncthreads();
+        const bool last = j + 1 >= slabs(r);
+        const int64_t rn = last ? r - 1 : r, jn = last ? 0 : j + 1;
+        if (warp != chain) {
+            if (rn >= 0) produce(rn, jn, b ^ 1);
+        } else if (lane == 0) {
+            const int64_t left = m - 1 - r - j * TRSB_TILE;
+            const int cnt = left < TRSB_TILE ? (int)left : TRSB_TILE;
+            auto get = [&](const double *q) {
+                mf<N> p;
+#pragma unroll
+                for (int l = 0; l < N; ++l) p.v[l] = q[l];
+                return p;
+            };
+            int i = 0;
+            if (j == 0) {
+                v = get(head[b][0]);
+                if (!unit) d = get(head[b][1]);
+                if (cnt > 0) {
+                    v = sub(v, mul(get(prod[b][0]), x));
+                    i = 1;
+                }
+            }
+            // terms unrolled together: a loop end costs about 13 cycles, the
+            // longer networks fill the instruction cache sooner
+            constexpr int U = N == 2 ? 32 : N == 3 ? 16 : 8;
+            for (; i + U <= cnt; i += U)
+#pragma unroll
+                for (int q = 0; q < U; ++q) v = sub(v, get(prod[b][i + q]));
+            for (; i < cnt; ++i) v = sub(v, get(prod[b][i]));
+            if (last) {
+                if (!unit) v = div(v, d);
+                store_mf<N>(B.p, B.ld, B.ls, r, col, v);
+                x = v;
+            }
+        }
+        if (last && r == 0) break;
+        r = rn;
+        j = jn;
     }
 }
 
@@ -264,15 +409,15 @@ static int run_trsm(int side, int uplo, int trans, int diag, int64_t m, int64_t 
     const bool wavefront_ok = eff_lower || N == 1 || order == MFLAB_ORDER_FAST;
     if (N == 1 && !transposed && m > 2 * TRSM64_NB && n <= 65535 && !info)
         return trsm64_blocked(m, n, A, B, eff_lower, unit, s, info);
-    if (!eff_lower && !wavefront_ok && m > 64 && n < 4096 && (size_t)m * N * 8 <= 200 * 1024) {
-        const size_t smem = (size_t)m * N * sizeof(double);
-        static std::atomic<unsigned long long> configured{0};
-        if (int rc = set_smem_once((const void *)trsm_left_backward_cta<N, 256>, 200 * 1024,
-                                   configured, "trsm backward attribute"))
-            return rc;
-        trsm_left_backward_cta<N, 256><<<(unsigned)n, 256, smem, s>>>(m, n, A, B, transposed,
-                                                                       unit, info);
-        return record_cuda_error(cudaGetLastError(), "trsm left backward");
+    if constexpr (N >= 2) {
+        if (eff_lower && m <= 64) return run_trsm_left_warp<N>(m, n, A, B, transposed, unit, s, info);
+        // one CTA per column; short triangles of many columns go to the
+        // thread kernel, whose 32 chains share a warp
+        if (!wavefront_ok && n < (m <= 64 ? (N == 4 ? 2 : 4) * TRSB_SMS : 4096)) {
+            trsm_left_backward_cta<N><<<(unsigned)n, TRSB_NT, 0, s>>>(m, n, A, B, transposed, unit,
+                                                                     info);
+            return record_cuda_error(cudaGetLastError(), "trsm left backward");
+        }
     }
     if (m <= 64 || n >= 4096 || !wavefront_ok) {
         trsm_left_thread<N><<<(unsigned)((n + 127) / 128), 128, 0, s>>>(m, n, A, B, eff_lower,
