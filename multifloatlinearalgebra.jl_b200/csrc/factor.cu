@@ -1639,17 +1639,26 @@ __global__ void __launch_bounds__(NT) maxabs_partial_kernel(int64_t m, int64_t n
     }
 }
 
+// one warp over the partial maxima
 template <int N>
 __global__ void maxabs_final_kernel(int nparts, const double *part, double *out) {
     mf<N> best = from_double<N>(0.0);
-    int fin = 1;
-    for (int i = 0; i < nparts; ++i) {
+    bool fin = true;
+    for (int i = threadIdx.x; i < nparts; i += 32) {
         mf<N> v;
 #pragma unroll
         for (int l = 0; l < N; ++l) v.v[l] = part[i * (N + 1) + l];
         best = max_mf(best, v);
-        if (part[i * (N + 1) + N] == 0.0) fin = 0;
+        fin = fin && part[i * (N + 1) + N] != 0.0;
     }
+    for (int off = 16; off > 0; off >>= 1) {
+        mf<N> o;
+#pragma unroll
+        for (int l = 0; l < N; ++l) o.v[l] = __shfl_xor_sync(0xffffffffu, best.v[l], off);
+        best = max_mf(best, o);
+    }
+    fin = __all_sync(0xffffffffu, fin);
+    if (threadIdx.x) return;
 #pragma unroll
     for (int l = 0; l < N; ++l) out[l] = best.v[l];
     out[N] = fin ? 1.0 : 0.0;
@@ -1703,7 +1712,7 @@ static int maxabs_n(int64_t m, int64_t n, Mat A, int region, double *part, int n
     maxabs_partial_kernel<N, 256><<<nparts, 256, 0, s>>>(m, n, A, region, part);
     int rc = record_cuda_error(cudaGetLastError(), "maxabs partial");
     if (rc) return rc;
-    maxabs_final_kernel<N><<<1, 1, 0, s>>>(nparts, part, out);
+    maxabs_final_kernel<N><<<1, 32, 0, s>>>(nparts, part, out);
     return record_cuda_error(cudaGetLastError(), "maxabs final");
 }
 

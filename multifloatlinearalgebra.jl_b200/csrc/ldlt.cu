@@ -1,15 +1,16 @@
 // Bunch-Kaufman LDL^T (1x1 and 2x2 pivots) with its solve and inertia.
 //
 // Follows src/factorizations/ldlt.jl of MultiFloatLinearAlgebra.jl:
-//   * unblocked route (ldlt.jl:352-412): one cooperative CTA runs the pivot
+//   * unblocked route (ldlt.jl:352-412): one cluster of CTAs runs the pivot
 //     steps; each step's column scan, row scan, symmetric swap, column scaling
-//     and rank-1 / rank-2 update are spread over the CTA's threads, the pivot
-//     decisions are taken by thread 0 exactly as ldlt.jl:183-219 orders them;
-//   * blocked route (ldlt_gemmt.jl:36-73): per panel one cooperative CTA runs
-//     the lazy panel (every entry evaluated against the earlier pivots of the
-//     panel, ldlt.jl:414-593), then W = L21 * D (ldlt.jl:595-632), the lower
-//     trailing update A22 = -1 * L21 W^T + 1 * A22 through the shared mainloop
-//     (gemmt) and the upper mirror.
+//     and rank-1 / rank-2 update are spread over the cluster's threads, the
+//     pivot decisions are taken by every thread from the same values exactly
+//     as ldlt.jl:183-219 orders them;
+//   * blocked route (ldlt_gemmt.jl:36-73): per panel the same cluster kernel
+//     runs the lazy panel (every entry evaluated against the earlier pivots of
+//     the panel, ldlt.jl:414-593), then W = L21 * D (ldlt.jl:595-632), the
+//     lower trailing update A22 = -1 * L21 W^T + 1 * A22 through the shared
+//     mainloop (gemmt) and the upper mirror.
 // Every per-element expression and its association is the reference's, so the
 // result is bitwise the oracle's; the parallel loops only distribute
 // independent elements.  When a step fails (info > 0) the factor content after
@@ -41,434 +42,620 @@ struct Ldlt {
 #pragma unroll
         for (int l = 0; l < N; ++l) dsub[l * lsd + k] = v.v[l];
     }
-    // lazily updated Schur-complement entry (ldlt.jl:414-449)
-    __device__ mf<N> panel_entry(int64_t i1, int64_t i2, int64_t pf, int64_t pivot_first) const {
-        const int64_t row = i1 > i2 ? i1 : i2, col = i1 > i2 ? i2 : i1;
-        mf<N> v = at(row, col);
-        int64_t q = pf;
-        while (q < pivot_first) {
-            if (blocks[q] == 1) {
-                v = sub(v, mul(at(row, q), mul(at(q, q), at(col, q))));
-                q += 1;
-            } else {
-                const mf<N> rf = at(row, q), rs = at(row, q + 1);
-                const mf<N> cf = at(col, q), cs = at(col, q + 1);
-                const mf<N> c1 = add(mul(at(q, q), cf), mul(ds(q), cs));
-                const mf<N> c2 = add(mul(ds(q), cf), mul(at(q + 1, q + 1), cs));
-                v = sub(v, add(mul(rf, c1), mul(rs, c2)));
-                q += 2;
-            }
-        }
-        return v;
-    }
-    __device__ mf<N> entry(int64_t i, int64_t j, bool lazy, int64_t pf, int64_t k) const {
-        return lazy ? panel_entry(i, j, pf, k) : at(i, j);
-    }
 };
+
+// The pivot kernels run each of their long expressions once per column on few
+// warps: kept as calls, their code stays in the instruction cache.
+template <int N>
+__device__ __noinline__ mf<N> div_call(mf<N> x, mf<N> y) {
+    return div(x, y);
+}
 
 // ldlt.jl:65-101; returns nonsingular
 template <int N>
-__device__ bool solve_2x2(const mf<N> &d11, const mf<N> &d21, const mf<N> &d22, const mf<N> &first,
+__device__ __noinline__ bool solve_2x2(const mf<N> &d11, const mf<N> &d21, const mf<N> &d22, const mf<N> &first,
                           const mf<N> &second, mf<N> &x1, mf<N> &x2) {
     const mf<N> scale = max_mf(max_mf(abs_mf(d11), abs_mf(d21)), abs_mf(d22));
     x1 = from_double<N>(0.0);
     x2 = from_double<N>(0.0);
     if (iszero(scale) || !isfinite_mf(scale)) return false;
-    const mf<N> a = div(d11, scale), b = div(d21, scale), c = div(d22, scale);
-    const mf<N> r1 = div(first, scale), r2 = div(second, scale);
+    const mf<N> a = div_call(d11, scale), b = div_call(d21, scale), c = div_call(d22, scale);
+    const mf<N> r1 = div_call(first, scale), r2 = div_call(second, scale);
     if (ge(abs_mf(a), abs_mf(b))) {
         if (iszero(a)) return false;
-        const mf<N> t = div(b, a);
+        const mf<N> t = div_call(b, a);
         const mf<N> u = submul(c, t, b);
         if (iszero(u) || !isfinite_mf(u)) return false;
-        const mf<N> y2 = div(submul(r2, t, r1), u);
-        x1 = div(submul(r1, b, y2), a);
+        const mf<N> y2 = div_call(submul(r2, t, r1), u);
+        x1 = div_call(submul(r1, b, y2), a);
         x2 = y2;
         return true;
     }
     if (iszero(b)) return false;
-    const mf<N> t = div(a, b);
+    const mf<N> t = div_call(a, b);
     const mf<N> u = submul(b, t, c);
     if (iszero(u) || !isfinite_mf(u)) return false;
-    const mf<N> y2 = div(submul(r1, t, r2), u);
-    x1 = div(submul(r2, c, y2), b);
+    const mf<N> y2 = div_call(submul(r1, t, r2), u);
+    x1 = div_call(submul(r2, c, y2), b);
     x2 = y2;
     return true;
 }
 
-// shared scratch of the cooperative kernels
-template <int N, int NT>
-struct CoopShared {
-    double val[NT][N];
-    int64_t idx[NT];
-    double bcast[8][N];
-    int64_t ibcast[4];
+// ---------------------------------------------------- cluster kernel ------
+// One launch runs a lazy panel (LAZY) or the whole unblocked factorization on
+// one cluster.  A pivot step is a few dependent scans of a column with a
+// decision after each, so its time is latency: the scans' chains and the
+// cluster barriers.  What keeps both short:
+//   * rows are dealt to the cluster's warps in groups of 32, so a scan is one
+//     chain per thread and the rank updates use every CTA's FP64 pipe;
+//   * in a lazy entry row r, column c (ldlt.jl:414-449),
+//         v = A[r,c]; v -= A[r,q] * (D[q] * A[c,q]) over the panel's pivots q,
+//     the inner product depends on the column alone: it is formed once per
+//     column and CTA in shared memory, where it was formed anew in every
+//     entry, and the pivots' D stay there too;
+//   * candidates are written into every CTA of the cluster before the barrier
+//     and read locally after it; a step takes two to four barriers;
+//   * the symmetric swap is one pass over disjoint pairs.
+// x3, n = 600: 215 us a 12-column panel (495 us on one CTA).
+constexpr int LD_NT = 256, LD_WARPS = LD_NT / 32, LD_MAXC = 16, LD_PANEL = 66;
+
+__device__ __forceinline__ void ld_cluster_sync() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t ld_remote(const void *p, uint32_t rank) {
+    uint32_t a = (uint32_t)__cvta_generic_to_shared(p), r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void ld_remote_f64(uint32_t a, double v) {
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+__device__ __forceinline__ void ld_remote_s32(uint32_t a, int v) {
+    asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+
+template <int N>
+struct LdShared {
+    double coef[2][LD_PANEL][N];  // D * A[col, panel] of the columns k and imax / k+1
+    double rowi[LD_PANEL][N];     // A[imax, panel]
+    double d[LD_PANEL][N], ds[LD_PANEL][N];
+    double cand[2][LD_MAXC][N];   // every CTA's column / row maximum
+    int candi[2][LD_MAXC];
+    double red[LD_WARPS][N];
+    int redi[LD_WARPS];
+    double val[3][N];             // diagonal entries formed by single lanes
+    double blk[6][N];             // the 2x2 block's scale, a, b, c, t, u (ld_block)
+    int regular;                  // 0 singular, 1 |a| >= |b|, 2 |a| < |b|
+    unsigned char type[LD_PANEL];
     int flag;
 };
 
-// first strictly larger |entry(r, k)| over r in [r0, n) (smallest index among the maxima)
-template <int N, int NT>
-__device__ void coop_colmax(const Ldlt<N> &F, CoopShared<N, NT> &sh, int64_t r0, int64_t k,
-                            bool lazy, int64_t pf, mf<N> &best, int64_t &bidx) {
-    const int t = threadIdx.x;
-    mf<N> b = from_double<N>(0.0);
-    int64_t bi = -1;
-    for (int64_t r = r0 + t; r < F.n; r += NT) {
-        const mf<N> c = abs_mf(F.entry(r, k, lazy, pf, k));
-        if (bi < 0 || gt(c, b)) {
-            b = c;
-            bi = r;
-        }
-    }
-#pragma unroll
-    for (int l = 0; l < N; ++l) sh.val[t][l] = b.v[l];
-    sh.idx[t] = bi;
-    __syncthreads();
-    for (int off = NT / 2; off > 0; off >>= 1) {
-        if (t < off) {
-            mf<N> a, c;
-#pragma unroll
-            for (int l = 0; l < N; ++l) {
-                a.v[l] = sh.val[t][l];
-                c.v[l] = sh.val[t + off][l];
-            }
-            const int64_t ia = sh.idx[t], ic = sh.idx[t + off];
-            bool take;
-            if (ic < 0) take = false;
-            else if (ia < 0) take = true;
-            else if (gt(c, a)) take = true;
-            else if (gt(a, c)) take = false;
-            else take = ic < ia;
-            if (take) {
-#pragma unroll
-                for (int l = 0; l < N; ++l) sh.val[t][l] = c.v[l];
-                sh.idx[t] = ic;
-            }
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int l = 0; l < N; ++l) best.v[l] = sh.val[0][l];
-    bidx = sh.idx[0];
-    __syncthreads();
-}
-
-// max |entry| along row imax of the active matrix (ldlt.jl:203-209)
-template <int N, int NT>
-__device__ mf<N> coop_rowmax(const Ldlt<N> &F, CoopShared<N, NT> &sh, int64_t k, int64_t imax,
-                             bool lazy, int64_t pf) {
-    const int t = threadIdx.x;
-    mf<N> b = from_double<N>(0.0);
-    for (int64_t c = k + t; c < imax; c += NT) b = max_mf(b, abs_mf(F.entry(imax, c, lazy, pf, k)));
-    for (int64_t r = imax + 1 + t; r < F.n; r += NT) b = max_mf(b, abs_mf(F.entry(r, imax, lazy, pf, k)));
-#pragma unroll
-    for (int l = 0; l < N; ++l) sh.val[t][l] = b.v[l];
-    __syncthreads();
-    for (int off = NT / 2; off > 0; off >>= 1) {
-        if (t < off) {
-            mf<N> a, c;
-#pragma unroll
-            for (int l = 0; l < N; ++l) {
-                a.v[l] = sh.val[t][l];
-                c.v[l] = sh.val[t + off][l];
-            }
-            const mf<N> r = max_mf(a, c);
-#pragma unroll
-            for (int l = 0; l < N; ++l) sh.val[t][l] = r.v[l];
-        }
-        __syncthreads();
-    }
-    mf<N> out;
-#pragma unroll
-    for (int l = 0; l < N; ++l) out.v[l] = sh.val[0][l];
-    __syncthreads();
-    return out;
-}
-
-template <int N, int NT>
-__device__ void put_bcast(CoopShared<N, NT> &sh, int slot, const mf<N> &v) {
-#pragma unroll
-    for (int l = 0; l < N; ++l) sh.bcast[slot][l] = v.v[l];
-}
-template <int N, int NT>
-__device__ mf<N> get_bcast(CoopShared<N, NT> &sh, int slot) {
+template <int N>
+__device__ __forceinline__ mf<N> ld_get(const double *p) {
     mf<N> v;
 #pragma unroll
-    for (int l = 0; l < N; ++l) v.v[l] = sh.bcast[slot][l];
+    for (int l = 0; l < N; ++l) v.v[l] = p[l];
     return v;
 }
-
-// Bunch-Kaufman pivot choice (ldlt.jl:183-219 / 451-508); returns block size,
-// pivot row in *piv.  All threads call it and get the same answer.
-template <int N, int NT>
-__device__ int select_bk(const Ldlt<N> &F, CoopShared<N, NT> &sh, int64_t k, const mf<N> &alpha,
-                         bool lazy, int64_t pf, int64_t *piv) {
-    const int t = threadIdx.x;
-    const int64_t n = F.n;
-    if (t == 0) put_bcast(sh, 0, abs_mf(F.entry(k, k, lazy, pf, k)));
-    __syncthreads();
-    const mf<N> absakk = get_bcast(sh, 0);
-    __syncthreads();
-    if (k == n - 1) {
-        *piv = k;
-        return iszero(absakk) ? 0 : 1;
-    }
-    mf<N> colmax;
-    int64_t imax;
-    coop_colmax(F, sh, k + 1, k, lazy, pf, colmax, imax);
-    if (iszero(max_mf(absakk, colmax))) {
-        *piv = k;
-        return 0;
-    }
-    if (ge(absakk, mul(alpha, colmax))) {
-        *piv = k;
-        return 1;
-    }
-    const mf<N> rowmax = coop_rowmax(F, sh, k, imax, lazy, pf);
-    if (ge(absakk, mul(mul(alpha, colmax), div(colmax, rowmax)))) {
-        *piv = k;
-        return 1;
-    }
-    if (t == 0) put_bcast(sh, 1, abs_mf(F.entry(imax, imax, lazy, pf, k)));
-    __syncthreads();
-    const mf<N> cand = get_bcast(sh, 1);
-    __syncthreads();
-    *piv = imax;
-    return ge(cand, mul(alpha, rowmax)) ? 1 : 2;
+template <int N>
+__device__ __forceinline__ void ld_put(double *p, const mf<N> &v) {
+#pragma unroll
+    for (int l = 0; l < N; ++l) p[l] = v.v[l];
 }
 
-// P A P^T on the active part plus the row swap of the earlier L columns
-// (ldlt.jl:155-181): all rows first, then the active columns.
-template <int N, int NT>
-__device__ void coop_sym_swap(const Ldlt<N> &F, int64_t a, int64_t b, int64_t active_first) {
-    if (a == b) return;
-    const int t = threadIdx.x;
-    for (int64_t c = t; c < F.n; c += NT) {
-#pragma unroll
-        for (int l = 0; l < N; ++l) {
-            double *col = F.A.p + l * F.A.ls + c * F.A.ld;
-            const double x = col[a];
-            col[a] = col[b];
-            col[b] = x;
+// coefficients D * A[col, pf + i], i < cnt, of one column's lazy entries
+template <int N>
+__device__ void ld_stage_coef(const Ldlt<N> &F, LdShared<N> &sh, double (*dst)[N], int64_t col,
+                              int64_t pf, int cnt) {
+    for (int i = threadIdx.x; i < cnt; i += LD_NT) {
+        const mf<N> d = ld_get<N>(sh.d[i]), c = F.at(col, pf + i);
+        if (sh.type[i] == 1) {
+            ld_put<N>(dst[i], mul(d, c));
+        } else if (sh.type[i] == 2) {
+            const mf<N> cs = F.at(col, pf + i + 1), o = ld_get<N>(sh.ds[i]);
+            ld_put<N>(dst[i], add(mul(d, c), mul(o, cs)));
+            ld_put<N>(dst[i + 1], add(mul(o, c), mul(ld_get<N>(sh.d[i + 1]), cs)));
         }
     }
-    __syncthreads();
-    for (int64_t r = active_first + t; r < F.n; r += NT) {
-#pragma unroll
-        for (int l = 0; l < N; ++l) {
-            double *pa = F.A.p + l * F.A.ls + a * F.A.ld + r;
-            double *pb = F.A.p + l * F.A.ls + b * F.A.ld + r;
-            const double x = *pa;
-            *pa = *pb;
-            *pb = x;
-        }
-    }
-    __syncthreads();
 }
 
-// unblocked route, one CTA (ldlt.jl:352-412)
-template <int N, int NT>
-__global__ void __launch_bounds__(NT) ldlt_unblocked_kernel(Ldlt<N> F, scal<N> alpha_s, int *info) {
-    __shared__ CoopShared<N, NT> sh;
-    if (*info) return;
-    const int t = threadIdx.x;
-    const int64_t n = F.n;
-    const mf<N> alpha = alpha_s.get();
-    int64_t k = 0;
-    while (k < n) {
-        int64_t piv;
-        const int bs = select_bk<N, NT>(F, sh, k, alpha, false, 0, &piv);
-        if (bs == 0) {
-            if (t == 0) *info = (int)(k + 1);
-            return;
+// entry (r, col), r >= col, from the column's staged coefficients; the panel
+// values are fetched two terms ahead
+template <int N>
+__device__ __noinline__ mf<N> ld_entry(const Ldlt<N> &F, const LdShared<N> &sh, const double (*coef)[N],
+                          int64_t r, int64_t col, int64_t pf, int cnt) {
+    mf<N> v = F.at(r, col);
+    if (cnt == 0) return v;
+    auto fetch = [&](int i) { return i < cnt ? F.at(r, pf + i) : from_double<N>(0.0); };
+    mf<N> a = fetch(0), b = fetch(1), c = fetch(2);
+    // the product of term i, whose panel values are a (and b)
+    auto term = [&](int i) {
+        mf<N> p = mul(a, ld_get<N>(coef[i]));
+        if (sh.type[i] != 1) p = add(p, mul(b, ld_get<N>(coef[i + 1])));
+        return p;
+    };
+    mf<N> p = term(0);
+    for (int i = 0;;) {
+        const bool one = sh.type[i] == 1;
+        const mf<N> n0 = fetch(i + 3);
+        if (one) {
+            a = b;
+            b = c;
+            c = n0;
+            i += 1;
+        } else {
+            a = c;
+            b = n0;
+            c = fetch(i + 4);
+            i += 2;
+        }
+        if (i >= cnt) return sub(v, p);
+        const mf<N> q = term(i);  // the next product beside this subtraction
+        v = sub(v, p);
+        p = q;
+    }
+}
+
+// entry (imax, c), c < imax: row imax staged, the coefficients are column c's own
+template <int N>
+__device__ __noinline__ mf<N> ld_row_entry(const Ldlt<N> &F, const LdShared<N> &sh, int64_t imax, int64_t c,
+                              int64_t pf, int cnt) {
+    mf<N> v = F.at(imax, c);
+    if (cnt == 0) return v;
+    auto fetch = [&](int i) { return i < cnt ? F.at(c, pf + i) : from_double<N>(0.0); };
+    mf<N> a = fetch(0), b = fetch(1);
+    auto term = [&](int i) {
+        const mf<N> d = ld_get<N>(sh.d[i]);
+        if (sh.type[i] == 1) return mul(ld_get<N>(sh.rowi[i]), mul(d, a));
+        const mf<N> o = ld_get<N>(sh.ds[i]);
+        const mf<N> c1 = add(mul(d, a), mul(o, b));
+        const mf<N> c2 = add(mul(o, a), mul(ld_get<N>(sh.d[i + 1]), b));
+        return add(mul(ld_get<N>(sh.rowi[i]), c1), mul(ld_get<N>(sh.rowi[i + 1]), c2));
+    };
+    mf<N> p = term(0);
+    for (int i = 0;;) {
+        const bool one = sh.type[i] == 1;
+        const mf<N> n0 = fetch(i + 2);
+        if (one) {
+            a = b;
+            b = n0;
+            i += 1;
+        } else {
+            a = n0;
+            b = fetch(i + 3);
+            i += 2;
+        }
+        if (i >= cnt) return sub(v, p);
+        const mf<N> q = term(i);
+        v = sub(v, p);
+        p = q;
+    }
+}
+
+// larger of two candidates: the first strictly larger value in ascending index
+// order; index -1 holds no candidate
+template <int N>
+__device__ __forceinline__ void ld_better(mf<N> &v, int &i, const mf<N> &o, int oi) {
+    bool take = oi >= 0;
+    if (take && i >= 0) take = gt(o, v) ? true : gt(v, o) ? false : oi < i;
+    if (take) {
+        v = o;
+        i = oi;
+    }
+}
+
+// best candidate of the lanes' groups of `width` lanes, in every lane
+template <int N>
+__device__ __forceinline__ void ld_lanes(mf<N> &v, int &i, int width) {
+    for (int off = width / 2; off > 0; off >>= 1) {
+        mf<N> o;
+#pragma unroll
+        for (int l = 0; l < N; ++l) o.v[l] = __shfl_xor_sync(0xffffffffu, v.v[l], off);
+        const int oi = __shfl_xor_sync(0xffffffffu, i, off);
+        ld_better(v, i, o, oi);
+    }
+}
+
+// cluster-wide best candidate, in every thread: buffer b of the candidates;
+// one CTA barrier and one cluster barrier
+template <int N>
+__device__ void ld_reduce(LdShared<N> &sh, int b, uint32_t rank, int nc, mf<N> &v, int &i) {
+    const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+    ld_lanes(v, i, 32);
+    if (lane == 0) {
+        ld_put<N>(sh.red[warp], v);
+        sh.redi[warp] = i;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        v = ld_get<N>(sh.red[lane % LD_WARPS]);
+        i = sh.redi[lane % LD_WARPS];
+        ld_lanes(v, i, LD_WARPS);
+        if (lane < nc) {
+#pragma unroll
+            for (int l = 0; l < N; ++l)
+                ld_remote_f64(ld_remote(&sh.cand[b][rank][l], (uint32_t)lane), v.v[l]);
+            ld_remote_s32(ld_remote(&sh.candi[b][rank], (uint32_t)lane), i);
+        }
+    }
+    ld_cluster_sync();
+    v = lane < nc ? ld_get<N>(sh.cand[b][lane]) : from_double<N>(0.0);
+    i = lane < nc ? sh.candi[b][lane] : -1;
+    ld_lanes(v, i, 32);
+}
+
+// solve_2x2 in two parts with the same operations: what depends on the block
+// alone, by one warp (the three quotients by the scale on a lane each), and a
+// right-hand side's part given that.
+template <int N>
+__device__ __noinline__ void ld_block(LdShared<N> &sh, const mf<N> &d11, const mf<N> &d21,
+                                      const mf<N> &d22) {
+    const int lane = threadIdx.x % 32;
+    const mf<N> scale = max_mf(max_mf(abs_mf(d11), abs_mf(d21)), abs_mf(d22));
+    if (iszero(scale) || !isfinite_mf(scale)) {
+        if (lane == 0) sh.regular = 0;
+        return;
+    }
+    const mf<N> mine = div_call(lane == 0 ? d11 : lane == 1 ? d21 : d22, scale);
+    mf<N> a, b, c;
+#pragma unroll
+    for (int l = 0; l < N; ++l) {
+        a.v[l] = __shfl_sync(0xffffffffu, mine.v[l], 0);
+        b.v[l] = __shfl_sync(0xffffffffu, mine.v[l], 1);
+        c.v[l] = __shfl_sync(0xffffffffu, mine.v[l], 2);
+    }
+    const bool first = ge(abs_mf(a), abs_mf(b));
+    const mf<N> lead = first ? a : b;
+    int regular = 0;
+    mf<N> t = lead, u = lead;
+    if (!iszero(lead)) {
+        t = div_call(first ? b : a, lead);
+        u = first ? submul(c, t, b) : submul(b, t, c);
+        if (!iszero(u) && isfinite_mf(u)) regular = first ? 1 : 2;
+    }
+    if (lane == 0) {
+        const mf<N> out[6] = {scale, a, b, c, t, u};
+#pragma unroll
+        for (int i = 0; i < 6; ++i) ld_put<N>(sh.blk[i], out[i]);
+        sh.regular = regular;
+    }
+}
+
+template <int N>
+__device__ __noinline__ void ld_block_solve(const LdShared<N> &sh, const mf<N> &r1, const mf<N> &r2,
+                                            mf<N> &x1, mf<N> &x2) {
+    const mf<N> a = ld_get<N>(sh.blk[1]), b = ld_get<N>(sh.blk[2]), c = ld_get<N>(sh.blk[3]);
+    const mf<N> t = ld_get<N>(sh.blk[4]), u = ld_get<N>(sh.blk[5]);
+    const bool first = sh.regular == 1;
+    x2 = div_call(first ? submul(r2, t, r1) : submul(r1, t, r2), u);
+    x1 = div_call(first ? submul(r1, b, x2) : submul(r2, c, x2), first ? a : b);
+}
+
+// P A P^T of rows / columns a < b on the active part plus the row swap of the
+// earlier columns (ldlt.jl:155-181), as disjoint exchanges: rows a and b in
+// every other column, columns a and b in every other row from `first` on, and
+// the four entries where they cross
+template <int N>
+__device__ void ld_sym_swap(const Ldlt<N> &F, int64_t a, int64_t b, int64_t first, int64_t gt_,
+                            int64_t total) {
+    const int64_t ld = F.A.ld;
+    for (int64_t c = gt_; c < F.n; c += total) {
+        // all loads before the stores: x <-> y and, from `first` on, u <-> w
+        const int64_t ix = c * ld + a, iy = c == a ? b * ld + b : c == b ? a * ld + b : c * ld + b;
+        const bool cols = c != a && c != b && c >= first;
+        const int64_t iu = a * ld + c, iw = b * ld + c;
+        const mf<N> x = load_mf<N>(F.A.p, 0, F.A.ls, ix, 0), y = load_mf<N>(F.A.p, 0, F.A.ls, iy, 0);
+        mf<N> u = x, w = y;
+        if (cols) {
+            u = load_mf<N>(F.A.p, 0, F.A.ls, iu, 0);
+            w = load_mf<N>(F.A.p, 0, F.A.ls, iw, 0);
+        }
+        store_mf<N>(F.A.p, 0, F.A.ls, ix, 0, y);
+        store_mf<N>(F.A.p, 0, F.A.ls, iy, 0, x);
+        if (cols) {
+            store_mf<N>(F.A.p, 0, F.A.ls, iu, 0, w);
+            store_mf<N>(F.A.p, 0, F.A.ls, iw, 0, u);
+        }
+    }
+}
+
+template <int N, bool LAZY>
+__global__ void __launch_bounds__(LD_NT)
+    ldlt_cluster_kernel(Ldlt<N> F, scal<N> alpha_s, int64_t pf, int64_t requested_last, int *info,
+                        int64_t *status) {
+    __shared__ LdShared<N> sh;
+    const int t = threadIdx.x, lane = t % 32, warp = t / 32;
+    if (*info) {  // the same in every thread of the cluster
+        if (LAZY && t == 0) status[1] = *info;
+        return;
+    }
+    uint32_t rank, ncu;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(ncu));
+    const int nc = (int)ncu;
+    const bool writer = rank == 0 && t == 0;
+    const int64_t n = F.n, total = (int64_t)nc * LD_NT;
+    // this thread's rows: group g of 32 goes to CTA g mod nc, warp (g / nc) mod 8
+    const int64_t mine = 32 * (rank + (int64_t)nc * warp) + lane;
+    const mf<N> alpha = alpha_s.get(), zero = from_double<N>(0.0);
+    int64_t pl = LAZY ? requested_last : n - 1;
+    int64_t k = LAZY ? pf : 0;
+    if (t == 0) sh.flag = 0;
+    // no CTA writes into another one before that one has started
+    ld_cluster_sync();
+    auto report = [&](int64_t failed) {  // {last column of the panel, failed column or 0}
+        if (LAZY && writer) {
+            status[0] = pl;
+            status[1] = failed;
+        }
+    };
+    auto fail = [&](int64_t kk) {
+        if (writer) *info = (int)(kk + 1);
+        report(kk + 1);
+    };
+    auto entry = [&](int which, int64_t r, int64_t col) {
+        if constexpr (LAZY) return ld_entry<N>(F, sh, sh.coef[which], r, col, pf, (int)(k - pf));
+        else return F.at(r, col);
+    };
+    while (k <= pl) {
+        const int cnt = LAZY ? (int)(k - pf) : 0;
+        if (LAZY) {
+            ld_stage_coef<N>(F, sh, sh.coef[0], k, pf, cnt);
+            __syncthreads();
+        }
+        // ---- pivot choice (ldlt.jl:183-219 / 451-508)
+        int bs = 1;
+        int64_t piv = k;
+        mf<N> held = zero;  // the entry of this thread's first row below k
+        int64_t held_row = -1;
+        {
+            mf<N> best = zero;
+            int bi = -1;
+            if (k < n - 1) {
+                for (int64_t r = mine; r < n; r += total) {
+                    if (r <= k) continue;
+                    const mf<N> e = entry(0, r, k);
+                    if (held_row < 0) {
+                        held = e;
+                        held_row = r;
+                    }
+                    ld_better(best, bi, abs_mf(e), (int)r);
+                }
+            }
+            if (t == LD_NT - 1) ld_put<N>(sh.val[0], entry(0, k, k));
+            __syncwarp();
+            ld_reduce<N>(sh, 0, rank, nc, best, bi);
+            const mf<N> absakk = abs_mf(ld_get<N>(sh.val[0]));
+            if (k == n - 1) {
+                if (iszero(absakk)) bs = 0;
+            } else if (iszero(max_mf(absakk, best))) {
+                bs = 0;
+            } else if (!ge(absakk, mul(alpha, best))) {
+                const int64_t imax = bi;
+                if (LAZY) {
+                    ld_stage_coef<N>(F, sh, sh.coef[1], imax, pf, cnt);
+                    for (int i = t; i < cnt; i += LD_NT) ld_put<N>(sh.rowi[i], F.at(imax, pf + i));
+                    __syncthreads();
+                }
+                // max |entry| along row imax of the active matrix
+                mf<N> rowmax = zero;
+                for (int64_t c = mine; c < n; c += total) {
+                    if (c < k || c == imax) continue;
+                    mf<N> e;
+                    if (c > imax) e = entry(1, c, imax);
+                    else if constexpr (LAZY) e = ld_row_entry<N>(F, sh, imax, c, pf, cnt);
+                    else e = F.at(imax, c);
+                    rowmax = max_mf(rowmax, abs_mf(e));
+                }
+                if (t == LD_NT - 1) ld_put<N>(sh.val[1], entry(1, imax, imax));
+                __syncwarp();
+                int ri = 0;
+                ld_reduce<N>(sh, 1, rank, nc, rowmax, ri);
+                if (!ge(absakk, mul(mul(alpha, best), div_call(best, rowmax)))) {
+                    piv = imax;
+                    bs = ge(abs_mf(ld_get<N>(sh.val[1])), mul(alpha, rowmax)) ? 1 : 2;
+                }
+            }
+        }
+        if (bs == 0) return fail(k);
+        if (LAZY ? (bs == 2 && k == pl) : bs == 2) {
+            if (!(k < n - 1)) return fail(k);
+            if (LAZY) pl += 1;
         }
         if (bs == 1) {
-            if (t == 0) {
+            if (writer) {
                 F.pivots[k] = piv + 1;
                 F.blocks[k] = 1;
             }
-            coop_sym_swap<N, NT>(F, k, piv, k);
-            const mf<N> d = F.at(k, k);
-            if (iszero(d)) {
-                if (t == 0) *info = (int)(k + 1);
-                return;
-            }
-            for (int64_t r = k + 1 + t; r < n; r += NT) F.put(r, k, div(F.at(r, k), d));
-            __syncthreads();
-            if (k < n - 1) {
-                // rank-1 update of the lower active part with its mirror
-                const int64_t m = n - k - 1;
-                const int64_t tot = m * (m + 1) / 2;
-                for (int64_t e = t; e < tot; e += NT) {
-                    // column-major enumeration of the lower triangle of the active part
-                    int64_t c = (int64_t)((2.0 * m + 1.0 - sqrt((2.0 * m + 1.0) * (2.0 * m + 1.0) - 8.0 * e)) / 2.0);
-                    while (c > 0 && c * m - c * (c - 1) / 2 > e) --c;
-                    while ((c + 1) * m - (c + 1) * c / 2 <= e) ++c;
-                    const int64_t r = c + (e - (c * m - c * (c - 1) / 2));
-                    const int64_t col = k + 1 + c, row = k + 1 + r;
-                    const mf<N> coef = mul(d, F.at(col, k));
-                    const mf<N> v = submul(F.at(row, col), F.at(row, k), coef);
-                    F.put(row, col, v);
-                    F.put(col, row, v);
+            if (piv != k) {
+                ld_sym_swap<N>(F, k, piv, k, rank * LD_NT + t, total);
+                ld_cluster_sync();
+                if (LAZY) {
+                    ld_stage_coef<N>(F, sh, sh.coef[0], k, pf, cnt);
+                    __syncthreads();
                 }
+                held_row = -1;
+                for (int64_t r = mine; r < n && held_row < 0; r += total)
+                    if (r > k) {
+                        held = entry(0, r, k);
+                        held_row = r;
+                    }
+                if (t == LD_NT - 1) ld_put<N>(sh.val[0], entry(0, k, k));
                 __syncthreads();
+            }
+            const mf<N> d = ld_get<N>(sh.val[0]);
+            if (iszero(d)) return fail(k);
+            for (int64_t r = mine; r < n; r += total)
+                if (r > k) F.put(r, k, div_call(r == held_row ? held : entry(0, r, k), d));
+            if (LAZY && t == 0) {
+                sh.type[cnt] = 1;
+                ld_put<N>(sh.d[cnt], d);
+            }
+            ld_cluster_sync();
+            if (LAZY) {
+                if (writer) F.put(k, k, d);
+            } else if (k < n - 1) {
+                // rank-1 update of the lower active part with its mirror, one
+                // column per warp
+                for (int64_t col = k + 1 + rank + (int64_t)nc * warp; col < n; col += nc * LD_WARPS) {
+                    const mf<N> coef = mul(d, F.at(col, k));
+                    for (int64_t row = col + lane; row < n; row += 32) {
+                        const mf<N> v = submul(F.at(row, col), F.at(row, k), coef);
+                        F.put(row, col, v);
+                        F.put(col, row, v);
+                    }
+                }
+                ld_cluster_sync();
             }
             k += 1;
         } else {
-            if (!(k < n - 1)) {
-                if (t == 0) *info = (int)(k + 1);
-                return;
-            }
-            if (t == 0) {
+            if (writer) {
                 F.pivots[k] = piv + 1;
                 F.blocks[k] = 2;
                 F.blocks[k + 1] = 0;
             }
-            coop_sym_swap<N, NT>(F, k + 1, piv, k);
-            const mf<N> d11 = F.at(k, k), d21 = F.at(k + 1, k), d22 = F.at(k + 1, k + 1);
-            if (t == 0) F.set_ds(k, d21);
-            mf<N> x1, x2;
-            if (!solve_2x2(d11, d21, d22, from_double<N>(0.0), from_double<N>(0.0), x1, x2)) {
-                if (t == 0) *info = (int)(k + 1);
-                return;
+            if (piv != k + 1) {
+                ld_sym_swap<N>(F, k + 1, piv, k, rank * LD_NT + t, total);
+                ld_cluster_sync();
             }
-            if (t == 0) sh.flag = 0;
-            __syncthreads();
-            for (int64_t r = k + 2 + t; r < n; r += NT) {
-                const bool ok = solve_2x2(d11, d21, d22, F.at(r, k), F.at(r, k + 1), x1, x2);
-                if (!(ok && isfinite_mf(x1) && isfinite_mf(x2))) {
-                    sh.flag = 1;
-                } else {
-                    F.put(r, k, x1);
-                    F.put(r, k + 1, x2);
+            __syncthreads();  // the readers of val and coef[1] are done
+            if (LAZY) {
+                ld_stage_coef<N>(F, sh, sh.coef[1], k + 1, pf, cnt);
+                __syncthreads();
+            }
+            // the block's three entries on a lane each, beside the rows' pairs
+            if (lane == 31 && warp >= LD_WARPS - 3) {
+                const int w = warp - (LD_WARPS - 3);
+                ld_put<N>(sh.val[w], w == 0 ? entry(0, k, k)
+                                            : w == 1 ? entry(0, k + 1, k) : entry(1, k + 1, k + 1));
+            }
+            __syncwarp();
+            mf<N> e1 = zero, e2 = zero;
+            held_row = -1;
+            for (int64_t r = mine; r < n && held_row < 0; r += total)
+                if (r > k + 1) {
+                    e1 = entry(0, r, k);
+                    e2 = entry(1, r, k + 1);
+                    held_row = r;
                 }
+            __syncthreads();
+            const mf<N> d11 = ld_get<N>(sh.val[0]), d21 = ld_get<N>(sh.val[1]),
+                        d22 = ld_get<N>(sh.val[2]);
+            // the block's quotients on the last warp, the first row's scaled
+            // pair beside them
+            const mf<N> scale = max_mf(max_mf(abs_mf(d11), abs_mf(d21)), abs_mf(d22));
+            mf<N> r1 = zero, r2 = zero;
+            if (warp == LD_WARPS - 1) ld_block<N>(sh, d11, d21, d22);
+            __syncwarp();
+            if (held_row >= 0) {
+                r1 = div_call(e1, scale);
+                r2 = div_call(e2, scale);
             }
             __syncthreads();
-            if (sh.flag) {
-                if (t == 0) *info = (int)(k + 1);
-                return;
+            const bool regular = sh.regular != 0;
+            if (regular)
+                for (int64_t r = mine; r < n; r += total) {
+                    if (r <= k + 1) continue;
+                    if (r != held_row) {
+                        r1 = div_call(entry(0, r, k), scale);
+                        r2 = div_call(entry(1, r, k + 1), scale);
+                    }
+                    mf<N> x1, x2;
+                    ld_block_solve<N>(sh, r1, r2, x1, x2);
+                    if (!(isfinite_mf(x1) && isfinite_mf(x2))) {
+                        for (int q = 0; q < nc; ++q)
+                            ld_remote_s32(ld_remote(&sh.flag, (uint32_t)q), 1);
+                    } else {
+                        F.put(r, k, x1);
+                        F.put(r, k + 1, x2);
+                    }
+                }
+            if (LAZY && t == 0) {
+                sh.type[cnt] = 2;
+                sh.type[cnt + 1] = 0;
+                ld_put<N>(sh.d[cnt], d11);
+                ld_put<N>(sh.d[cnt + 1], d22);
+                ld_put<N>(sh.ds[cnt], d21);
             }
-            if (k + 1 < n - 1) {
+            ld_cluster_sync();
+            if (writer) {
+                if (LAZY) {
+                    F.put(k, k, d11);
+                    F.put(k + 1, k + 1, d22);
+                }
+                F.set_ds(k, d21);
+            }
+            if (!regular || sh.flag) return fail(k);
+            if (!LAZY && k + 1 < n - 1) {
                 // rank-2 update (ldlt.jl:261-326): rows in full groups of four
                 // from the column use v - (f1 c1 + f2 c2), the remainder rows
                 // (v - f1 c1) - f2 c2
-                const int64_t m = n - k - 2;
-                const int64_t tot = m * (m + 1) / 2;
-                for (int64_t e = t; e < tot; e += NT) {
-                    int64_t c = (int64_t)((2.0 * m + 1.0 - sqrt((2.0 * m + 1.0) * (2.0 * m + 1.0) - 8.0 * e)) / 2.0);
-                    while (c > 0 && c * m - c * (c - 1) / 2 > e) --c;
-                    while ((c + 1) * m - (c + 1) * c / 2 <= e) ++c;
-                    const int64_t r = c + (e - (c * m - c * (c - 1) / 2));
-                    const int64_t col = k + 2 + c, row = k + 2 + r;
+                for (int64_t col = k + 2 + rank + (int64_t)nc * warp; col < n; col += nc * LD_WARPS) {
                     const mf<N> l1 = F.at(col, k), l2 = F.at(col, k + 1);
                     const mf<N> c1 = add(mul(d11, l1), mul(d21, l2));
                     const mf<N> c2 = add(mul(d21, l1), mul(d22, l2));
-                    const mf<N> v0 = F.at(row, col), f1 = F.at(row, k), f2 = F.at(row, k + 1);
-                    const int64_t span = n - col;  // rows col..n-1
-                    const bool grouped = (row - col) < 4 * (span / 4);
-                    mf<N> v;
-                    if (grouped)
-                        v = sub(v0, add(mul(f1, c1), mul(f2, c2)));
-                    else
-                        v = submul(submul(v0, f1, c1), f2, c2);
-                    F.put(row, col, v);
-                    F.put(col, row, v);
+                    const int64_t grouped = col + 4 * ((n - col) / 4);
+                    for (int64_t row = col + lane; row < n; row += 32) {
+                        const mf<N> v0 = F.at(row, col), f1 = F.at(row, k), f2 = F.at(row, k + 1);
+                        const mf<N> v = row < grouped
+                                            ? sub(v0, add(mul(f1, c1), mul(f2, c2)))
+                                            : submul(submul(v0, f1, c1), f2, c2);
+                        F.put(row, col, v);
+                        F.put(col, row, v);
+                    }
                 }
-                __syncthreads();
+                ld_cluster_sync();
             }
-            if (t == 0) {
-                F.put(k + 1, k, from_double<N>(0.0));
-                F.put(k, k + 1, from_double<N>(0.0));
+            if (writer) {
+                F.put(k + 1, k, zero);
+                F.put(k, k + 1, zero);
             }
-            __syncthreads();
             k += 2;
         }
     }
+    report(0);
 }
 
-// one lazy panel (ldlt.jl:510-593); status[0] = info, status[1] = panel_last
-template <int N, int NT>
-__global__ void __launch_bounds__(NT) ldlt_panel_kernel(Ldlt<N> F, scal<N> alpha_s, int64_t pf,
-                                                        int64_t requested_last, int *info,
-                                                        int64_t *panel_last_out) {
-    __shared__ CoopShared<N, NT> sh;
-    if (*info) return;
-    const int t = threadIdx.x;
-    const int64_t n = F.n;
-    const mf<N> alpha = alpha_s.get();
-    int64_t pl = requested_last;
-    int64_t k = pf;
-    auto fail = [&](int64_t kk) {
-        if (t == 0) {
-            *info = (int)(kk + 1);
-            *panel_last_out = pl;
-        }
-    };
-    while (k <= pl) {
-        int64_t piv;
-        const int bs = select_bk<N, NT>(F, sh, k, alpha, true, pf, &piv);
-        if (bs == 0) return fail(k);
-        if (bs == 2 && k == pl) {
-            if (!(k < n - 1)) return fail(k);
-            pl += 1;
-        }
-        if (bs == 1) {
-            if (t == 0) {
-                F.pivots[k] = piv + 1;
-                F.blocks[k] = 1;
-            }
-            coop_sym_swap<N, NT>(F, k, piv, k);
-            const mf<N> d = F.panel_entry(k, k, pf, k);
-            if (iszero(d)) return fail(k);
-            // entries first (they read column k's unswapped-then-swapped values
-            // and the earlier pivots), then the writes
-            __syncthreads();
-            if (t == 0) F.put(k, k, d);
-            for (int64_t r = k + 1 + t; r < n; r += NT) F.put(r, k, div(F.panel_entry(r, k, pf, k), d));
-            __syncthreads();
-            k += 1;
-        } else {
-            if (t == 0) {
-                F.pivots[k] = piv + 1;
-                F.blocks[k] = 2;
-                F.blocks[k + 1] = 0;
-            }
-            coop_sym_swap<N, NT>(F, k + 1, piv, k);
-            const mf<N> d11 = F.panel_entry(k, k, pf, k);
-            const mf<N> d21 = F.panel_entry(k + 1, k, pf, k);
-            const mf<N> d22 = F.panel_entry(k + 1, k + 1, pf, k);
-            __syncthreads();
-            if (t == 0) {
-                F.put(k, k, d11);
-                F.put(k + 1, k + 1, d22);
-                F.set_ds(k, d21);
-                sh.flag = 0;
-            }
-            mf<N> x1, x2;
-            if (!solve_2x2(d11, d21, d22, from_double<N>(0.0), from_double<N>(0.0), x1, x2))
-                return fail(k);
-            __syncthreads();
-            for (int64_t r = k + 2 + t; r < n; r += NT) {
-                const mf<N> e1 = F.panel_entry(r, k, pf, k), e2 = F.panel_entry(r, k + 1, pf, k);
-                const bool ok = solve_2x2(d11, d21, d22, e1, e2, x1, x2);
-                if (!(ok && isfinite_mf(x1) && isfinite_mf(x2))) {
-                    sh.flag = 1;
-                } else {
-                    F.put(r, k, x1);
-                    F.put(r, k + 1, x2);
-                }
-            }
-            __syncthreads();
-            if (sh.flag) return fail(k);
-            if (t == 0) {
-                F.put(k + 1, k, from_double<N>(0.0));
-                F.put(k, k + 1, from_double<N>(0.0));
-            }
-            __syncthreads();
-            k += 2;
-        }
+// Cluster size: one CTA per 32 rows up to sixteen (the larger sizes that the
+// device can place; eight where sixteen cannot be).
+template <int N, bool LAZY>
+static int launch_ldlt_cluster(const Ldlt<N> &F, const scal<N> &alpha, int64_t pf, int64_t req,
+                               int *info, int64_t *status, int64_t rows, cudaStream_t s) {
+    auto kern = ldlt_cluster_kernel<N, LAZY>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(LD_NT);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    // per device: asked, and able to place sixteen
+    static std::atomic<unsigned long long> asked{0}, sixteen{0};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return record_cuda_error(e, "sytrf device");
+    const unsigned long long bit = 1ULL << (dev & 63);
+    if (!(asked.load(std::memory_order_acquire) & bit)) {
+        int clusters = 0;
+        cfg.gridDim = dim3(LD_MAXC);
+        attr[0].val.clusterDim.x = LD_MAXC;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+                cudaSuccess &&
+            cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) == cudaSuccess && clusters > 0)
+            sixteen.fetch_or(bit, std::memory_order_release);
+        else
+            cudaGetLastError();
+        asked.fetch_or(bit, std::memory_order_release);
     }
-    if (t == 0) *panel_last_out = pl;
+    const int most = sixteen.load(std::memory_order_acquire) & bit ? LD_MAXC : 8;
+    int nc = 1;
+    while (nc < most && nc * 32 < rows) nc *= 2;
+    cfg.gridDim = dim3((unsigned)nc);
+    attr[0].val.clusterDim.x = (unsigned)nc;
+    return record_cuda_error(cudaLaunchKernelEx(&cfg, kern, F, alpha, pf, req, info, status),
+                             "sytrf cluster");
 }
 
 // W = L21 * D for the panel (ldlt.jl:595-632): one thread per trailing row
@@ -533,8 +720,6 @@ __global__ void ldlt_alpha_kernel(double *out) {
     for (int l = 0; l < N; ++l) out[l] = a.v[l];
 }
 
-constexpr int LDLT_NT = 512;
-
 template <int N>
 static int sytrf_n(mflab_handle *h, int64_t n, Mat A, double *dsub, int64_t lsd, int64_t *pivots,
                    uint8_t *blocks, int blocked, int64_t block, int *info, cudaStream_t s) {
@@ -552,7 +737,7 @@ static int sytrf_n(mflab_handle *h, int64_t n, Mat A, double *dsub, int64_t lsd,
     if (rc) return rc;
     double *W = (double *)h->scratch;
     double *alpha_dev = (double *)((char *)h->scratch + (wbytes + 255) / 256 * 256);
-    int64_t *pl_dev = (int64_t *)(alpha_dev + 4);
+    int64_t *st_dev = (int64_t *)(alpha_dev + 4);
     ldlt_alpha_kernel<N><<<1, 1, 0, s>>>(alpha_dev);
     scal<N> al{};
     double alpha_host[4] = {0, 0, 0, 0};
@@ -561,25 +746,19 @@ static int sytrf_n(mflab_handle *h, int64_t n, Mat A, double *dsub, int64_t lsd,
     if (e != cudaSuccess) return record_cuda_error(e, "sytrf alpha");
     for (int l = 0; l < N; ++l) al.v[l] = alpha_host[l];
     Ldlt<N> F{A, n, dsub, lsd, pivots, blocks};
-    if (!blocked) {
-        ldlt_unblocked_kernel<N, LDLT_NT><<<1, LDLT_NT, 0, s>>>(F, al, info);
-        return record_cuda_error(cudaGetLastError(), "sytrf unblocked");
-    }
+    if (!blocked) return launch_ldlt_cluster<N, false>(F, al, 0, n - 1, info, st_dev, n, s);
     const double mone[4] = {-1.0, 0.0, 0.0, 0.0}, one[4] = {1.0, 0.0, 0.0, 0.0};
     int64_t pf = 0;
     while (pf < n) {
         const int64_t req = pf + block - 1 < n - 1 ? pf + block - 1 : n - 1;
-        ldlt_panel_kernel<N, LDLT_NT><<<1, LDLT_NT, 0, s>>>(F, al, pf, req, info, pl_dev);
-        rc = record_cuda_error(cudaGetLastError(), "sytrf panel");
+        rc = launch_ldlt_cluster<N, true>(F, al, pf, req, info, st_dev, n - pf, s);
         if (rc) return rc;
-        int info_h = 0;
-        int64_t pl = 0;
-        e = cudaMemcpyAsync(&info_h, info, sizeof(int), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(&pl, pl_dev, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+        int64_t status[2] = {0, 0};
+        e = cudaMemcpyAsync(status, st_dev, sizeof(status), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return record_cuda_error(e, "sytrf panel status");
-        if (info_h) return MFLAB_OK;
+        if (status[1]) return MFLAB_OK;
+        const int64_t pl = status[0];
         if (pl < n - 1) {
             const int64_t tc = n - 1 - pl, pw = pl - pf + 1;
             Mat Wm{W, n, n * (block + 1)};
@@ -639,6 +818,62 @@ __global__ void ldlt_pivots_kernel(int64_t n, int64_t nrhs, Mat B, const int64_t
             }
         }
     }
+}
+
+// The same interchanges, one CTA per right-hand-side column: one thread replays
+// them on an index array in shared memory (a swap there is two reads, not two
+// rounds to L2), then the column is gathered.  x3, n = 600, 5 columns: 30 us
+// (286 us with the swaps in the column itself).
+constexpr int64_t LDLT_GATHER_MAXN = 12000;  // 16 bytes a row of shared memory
+
+template <int N>
+__global__ void __launch_bounds__(256)
+    ldlt_gather_kernel(int64_t n, Mat B, const int64_t *pivots, const uint8_t *blocks, int reverse) {
+    extern __shared__ double gather_raw[];
+    double *buf = gather_raw;        // [n] one limb of the column
+    int *idx = (int *)(buf + n);     // [n] source row of every row
+    int *with = idx + n;             // [n] step k exchanges rows k and with[k]
+    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
+        idx[i] = (int)i;
+        // the second row of a 2x2 block is the one exchanged (marker 0)
+        with[i] = (int)(blocks[i] == 1 ? pivots[i] - 1 : blocks[i] == 2 || i == 0 ? i : pivots[i - 1] - 1);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int64_t s = 0; s < n; ++s) {
+            const int64_t k = reverse ? n - 1 - s : s;
+            const int p = with[k];
+            if (p != (int)k) {
+                const int t = idx[k];
+                idx[k] = idx[p];
+                idx[p] = t;
+            }
+        }
+    }
+    for (int l = 0; l < N; ++l) {
+        double *x = B.p + l * B.ls + (int64_t)blockIdx.x * B.ld;
+        for (int64_t i = threadIdx.x; i < n; i += blockDim.x) buf[i] = x[i];
+        __syncthreads();
+        for (int64_t i = threadIdx.x; i < n; i += blockDim.x) x[i] = buf[idx[i]];
+        __syncthreads();
+    }
+}
+
+template <int N>
+static int ldlt_interchange(int64_t n, int64_t nrhs, Mat B, const int64_t *pivots,
+                            const uint8_t *blocks, int reverse, cudaStream_t s) {
+    if (n <= LDLT_GATHER_MAXN) {
+        static std::atomic<unsigned long long> configured{0};
+        if (int rc = set_smem_once((const void *)ldlt_gather_kernel<N>, (int)(16 * LDLT_GATHER_MAXN),
+                                   configured, "sytrs interchange attribute"))
+            return rc;
+        ldlt_gather_kernel<N><<<(unsigned)nrhs, 256, (size_t)(16 * n), s>>>(n, B, pivots, blocks,
+                                                                           reverse);
+    } else {
+        ldlt_pivots_kernel<N><<<(unsigned)((nrhs + 127) / 128), 128, 0, s>>>(n, nrhs, B, pivots,
+                                                                             blocks, reverse);
+    }
+    return record_cuda_error(cudaGetLastError(), "sytrs interchange");
 }
 
 // D solve (solve.jl:251-296): independent per (block, column)
@@ -807,14 +1042,16 @@ extern "C" int mflab_sytrs(mflab_handle *h, void *stream, int limbs, int64_t n, 
     Mat f{(double *)F, ldf, lsf}, b{B, ldb, lsb};
     cudaError_t e = cudaMemsetAsync(fail, 0x7f, sizeof(int), s);  // 0x7f7f7f7f = no failure
     if (e != cudaSuccess) return mfl::record_cuda_error(e, "sytrs flag");
-    const unsigned g = (unsigned)((nrhs + 127) / 128);
     const dim3 gd((unsigned)((n + 127) / 128), (unsigned)nrhs);
-    int rc;
-    switch (limbs) {
-    case 2: mfl::ldlt_pivots_kernel<2><<<g, 128, 0, s>>>(n, nrhs, b, pivots, blocks, 0); break;
-    case 3: mfl::ldlt_pivots_kernel<3><<<g, 128, 0, s>>>(n, nrhs, b, pivots, blocks, 0); break;
-    default: mfl::ldlt_pivots_kernel<4><<<g, 128, 0, s>>>(n, nrhs, b, pivots, blocks, 0); break;
-    }
+    auto interchange = [&](int reverse) {
+        switch (limbs) {
+        case 2: return mfl::ldlt_interchange<2>(n, nrhs, b, pivots, blocks, reverse, s);
+        case 3: return mfl::ldlt_interchange<3>(n, nrhs, b, pivots, blocks, reverse, s);
+        default: return mfl::ldlt_interchange<4>(n, nrhs, b, pivots, blocks, reverse, s);
+        }
+    };
+    int rc = interchange(0);
+    if (rc) return rc;
     rc = mfl::launch_trsm_info(limbs, 0, 0, 0, 1, n, nrhs, f, b, one, s, nullptr, h->solve_order);
     if (rc) return rc;
     switch (limbs) {
@@ -824,12 +1061,8 @@ extern "C" int mflab_sytrs(mflab_handle *h, void *stream, int limbs, int64_t n, 
     }
     rc = mfl::launch_trsm_info(limbs, 0, 0, 1, 1, n, nrhs, f, b, one, s, nullptr, h->solve_order);
     if (rc) return rc;
-    switch (limbs) {
-    case 2: mfl::ldlt_pivots_kernel<2><<<g, 128, 0, s>>>(n, nrhs, b, pivots, blocks, 1); break;
-    case 3: mfl::ldlt_pivots_kernel<3><<<g, 128, 0, s>>>(n, nrhs, b, pivots, blocks, 1); break;
-    default: mfl::ldlt_pivots_kernel<4><<<g, 128, 0, s>>>(n, nrhs, b, pivots, blocks, 1); break;
-    }
-    return mfl::record_cuda_error(cudaGetLastError(), "sytrs");
+    rc = mfl::record_cuda_error(cudaGetLastError(), "sytrs");
+    return rc ? rc : interchange(1);
 }
 
 extern "C" int mflab_ldlt_diagnostics(mflab_handle *h, void *stream, int limbs, int64_t n,
