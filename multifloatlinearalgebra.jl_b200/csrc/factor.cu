@@ -5,9 +5,10 @@
 // factors the diagonal block (rows inside the panel only), the rows below are
 // solved with trsm(side=right, lower, T) and the trailing lower triangle gets
 // -1 * (A21 A21^T) + 1 * A22 from the shared mainloop.  LU follows
-// src/factorizations/lu.jl:34-195: per panel column a pivot kernel (first
-// strictly larger |A[r,k]|, full-row swap, reciprocal scaling) and a rank-1
-// panel update, then trsm(left, lower, unit) on U12 and A22 = -A21 U12 + A22.
+// src/factorizations/lu.jl:34-195: per panel column the pivot (first strictly
+// larger |A[r,k]|, full-row swap, reciprocal scaling) and a rank-1 panel
+// update, then trsm(left, lower, unit) on U12 (the panel and U12: lu.cu) and
+// A22 = -A21 U12 + A22.
 // Every kernel reads the device `info` word first and exits if an earlier step
 // failed, so a whole factorization is enqueued without host synchronisation.
 #include "mf_device.cuh"
@@ -1382,6 +1383,50 @@ static int getrf64_fast(mflab_handle *h, int64_t m, int64_t n, Mat A, int64_t *i
     return rc;
 }
 
+// One panel of the blocked LU, columns first .. last: the cluster kernel, or,
+// for wider panels and more rows than a cluster holds (4096), a pivot search
+// and a rank-1 update per column as programmatic dependents of one another.
+template <int N>
+static int lu_panel_steps(int64_t m, Mat A, int64_t first, int64_t last, int64_t *ipiv, int *info,
+                          cudaStream_t s) {
+    if (last - first < LU_PANEL_W) {
+        const int rc = launch_lu_panel(N, m, A, first, (int)(last - first + 1), ipiv, info, s);
+        if (rc != MFLAB_ERR_UNSUPPORTED) return rc;
+    }
+    for (int64_t k = first; k <= last; ++k) {
+        int rc = launch_programmatic(lu_pivot_kernel<N, 512>, dim3(1), dim3(512), 0, s,
+                                     "getrf pivot", m, first, last + 1, A, k, ipiv, info);
+        if (rc) return rc;
+        if (k < last && k + 1 < m) {
+            const int64_t rows = m - k - 1;
+            rc = launch_programmatic(lu_rank1_kernel<N>, dim3((unsigned)((rows + 127) / 128)),
+                                     dim3(128), 0, s, "getrf rank1", m, A, k, last,
+                                     (const int *)info);
+            if (rc) return rc;
+        }
+    }
+    return MFLAB_OK;
+}
+
+// the panel's interchanges on the other columns, then U12 on columns
+// last + 1 .. solve_hi - 1
+template <int N>
+static int lu_block_row(int64_t n, int64_t solve_hi, Mat A, int64_t first, int64_t last,
+                        const int64_t *ipiv, const int *info, cudaStream_t s) {
+    const int64_t w = last - first + 1;
+    if (n <= w) return MFLAB_OK;
+    if (w <= LU_PANEL_W)
+        return launch_lu_swap_solve(N, n, solve_hi, A, first, (int)w, ipiv, info, s);
+    lu_swap_rest_kernel<N><<<(unsigned)((n - w + 127) / 128), 128, 0, s>>>(n, A, first, last, ipiv,
+                                                                           info);
+    int rc = record_cuda_error(cudaGetLastError(), "getrf swaps");
+    const double one[4] = {1.0, 0.0, 0.0, 0.0};
+    if (!rc && last < solve_hi - 1)
+        rc = launch_trsm_info(N, 0, 0, 0, 1, w, solve_hi - 1 - last, A.at(first, first),
+                              A.at(first, last + 1), one, s, info);
+    return rc;
+}
+
 template <int N>
 static int getrf_n(int64_t m, int64_t n, Mat A, int64_t *ipiv, int64_t block, int *info,
                    cudaStream_t s) {
@@ -1396,33 +1441,11 @@ static int getrf_n(int64_t m, int64_t n, Mat A, int64_t *ipiv, int64_t block, in
     if (rc) return rc;
     for (int64_t first = 0; first < kmax; first += block) {
         const int64_t last = first + block - 1 < kmax - 1 ? first + block - 1 : kmax - 1;
-        for (int64_t k = first; k <= last; ++k) {
-            // the panel's steps are programmatic dependents of one another
-            rc = launch_programmatic(lu_pivot_kernel<N, 512>, dim3(1), dim3(512), 0, s,
-                                     "getrf pivot", m, first, last + 1, A, k, ipiv, info);
-            if (rc) return rc;
-            if (k < last && k + 1 < m) {
-                const int64_t rows = m - k - 1;
-                rc = launch_programmatic(lu_rank1_kernel<N>, dim3((unsigned)((rows + 127) / 128)),
-                                         dim3(128), 0, s, "getrf rank1", m, A, k, last,
-                                         (const int *)info);
-                if (rc) return rc;
-            }
-        }
-        // the panel's interchanges on the other columns (also after a zero
-        // pivot, for the steps before it)
-        if (n > last - first + 1) {
-            const int64_t cols = n - (last - first + 1);
-            lu_swap_rest_kernel<N><<<(unsigned)((cols + 127) / 128), 128, 0, s>>>(n, A, first, last,
-                                                                                  ipiv, info);
-            rc = record_cuda_error(cudaGetLastError(), "getrf swaps");
-            if (rc) return rc;
-        }
+        rc = lu_panel_steps<N>(m, A, first, last, ipiv, info, s);
+        if (!rc) rc = lu_block_row<N>(n, n, A, first, last, ipiv, info, s);
+        if (rc) return rc;
         if (last < n - 1) {
             const int64_t w = last - first + 1, rest = n - 1 - last;
-            rc = launch_trsm_info(N, 0, 0, 0, 1, w, rest, A.at(first, first), A.at(first, last + 1),
-                                  one, s, info);
-            if (rc) return rc;
             if (last < m - 1) {
                 rc = launch_mm(N, false, false, 0, N == 3, m - 1 - last, rest, w, A.at(last + 1, first),
                                A.at(first, last + 1), A.at(last + 1, last + 1), mone, one, s, info);
@@ -1455,30 +1478,11 @@ static int getrf_ozaki_n(mflab_handle *h, int64_t m, int64_t n, Mat A, int64_t *
         const int64_t j1 = j0 + nb < kmax ? j0 + nb : kmax;  // panel columns [j0, j1)
         for (int64_t first = j0; first < j1; first += block) {
             const int64_t last = first + block - 1 < j1 - 1 ? first + block - 1 : j1 - 1;
-            for (int64_t k = first; k <= last; ++k) {
-                lu_pivot_kernel<N, 512><<<1, 512, 0, s>>>(m, first, last + 1, A, k, ipiv, info);
-                rc = record_cuda_error(cudaGetLastError(), "getrf pivot");
-                if (rc) return rc;
-                if (k < last && k + 1 < m) {
-                    const int64_t rows = m - k - 1;
-                    lu_rank1_kernel<N><<<(unsigned)((rows + 127) / 128), 128, 0, s>>>(m, A, k, last,
-                                                                                     info);
-                    rc = record_cuda_error(cudaGetLastError(), "getrf rank1");
-                    if (rc) return rc;
-                }
-            }
-            if (n > last - first + 1) {
-                const int64_t cols = n - (last - first + 1);
-                lu_swap_rest_kernel<N><<<(unsigned)((cols + 127) / 128), 128, 0, s>>>(
-                    n, A, first, last, ipiv, info);
-                rc = record_cuda_error(cudaGetLastError(), "getrf swaps");
-                if (rc) return rc;
-            }
+            rc = lu_panel_steps<N>(m, A, first, last, ipiv, info, s);
+            if (!rc) rc = lu_block_row<N>(n, j1, A, first, last, ipiv, info, s);
+            if (rc) return rc;
             if (last < j1 - 1) {
                 const int64_t w = last - first + 1, cols = j1 - 1 - last;
-                rc = launch_trsm_info(N, 0, 0, 0, 1, w, cols, A.at(first, first),
-                                      A.at(first, last + 1), one, s, info);
-                if (rc) return rc;
                 if (last < m - 1) {
                     rc = launch_mm(N, false, false, 0, N == 3, m - 1 - last, cols, w,
                                    A.at(last + 1, first), A.at(first, last + 1),

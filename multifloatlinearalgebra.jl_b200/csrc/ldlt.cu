@@ -15,6 +15,7 @@
 // result is bitwise the oracle's; the parallel loops only distribute
 // independent elements.  When a step fails (info > 0) the factor content after
 // that step is left as the parallel loop wrote it.
+#include "cluster.cuh"
 #include "mf_device.cuh"
 #include "mflab_internal.h"
 
@@ -43,13 +44,6 @@ struct Ldlt {
         for (int l = 0; l < N; ++l) dsub[l * lsd + k] = v.v[l];
     }
 };
-
-// The pivot kernels run each of their long expressions once per column on few
-// warps: kept as calls, their code stays in the instruction cache.
-template <int N>
-__device__ __noinline__ mf<N> div_call(mf<N> x, mf<N> y) {
-    return div(x, y);
-}
 
 // ldlt.jl:65-101; returns nonsingular
 template <int N>
@@ -97,23 +91,7 @@ __device__ __noinline__ bool solve_2x2(const mf<N> &d11, const mf<N> &d21, const
 //     and read locally after it; a step takes two to four barriers;
 //   * the symmetric swap is one pass over disjoint pairs.
 // x3, n = 600: 215 us a 12-column panel (495 us on one CTA).
-constexpr int LD_NT = 256, LD_WARPS = LD_NT / 32, LD_MAXC = 16, LD_PANEL = 66;
-
-__device__ __forceinline__ void ld_cluster_sync() {
-    __syncwarp();
-    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t ld_remote(const void *p, uint32_t rank) {
-    uint32_t a = (uint32_t)__cvta_generic_to_shared(p), r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void ld_remote_f64(uint32_t a, double v) {
-    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
-}
-__device__ __forceinline__ void ld_remote_s32(uint32_t a, int v) {
-    asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
-}
+constexpr int LD_NT = 256, LD_WARPS = LD_NT / 32, LD_MAXC = MAX_CLUSTER, LD_PANEL = 66;
 
 template <int N>
 struct LdShared {
@@ -130,19 +108,6 @@ struct LdShared {
     unsigned char type[LD_PANEL];
     int flag;
 };
-
-template <int N>
-__device__ __forceinline__ mf<N> ld_get(const double *p) {
-    mf<N> v;
-#pragma unroll
-    for (int l = 0; l < N; ++l) v.v[l] = p[l];
-    return v;
-}
-template <int N>
-__device__ __forceinline__ void ld_put(double *p, const mf<N> &v) {
-#pragma unroll
-    for (int l = 0; l < N; ++l) p[l] = v.v[l];
-}
 
 // coefficients D * A[col, pf + i], i < cnt, of one column's lazy entries
 template <int N>
@@ -230,30 +195,6 @@ __device__ __noinline__ mf<N> ld_row_entry(const Ldlt<N> &F, const LdShared<N> &
         const mf<N> q = term(i);
         v = sub(v, p);
         p = q;
-    }
-}
-
-// larger of two candidates: the first strictly larger value in ascending index
-// order; index -1 holds no candidate
-template <int N>
-__device__ __forceinline__ void ld_better(mf<N> &v, int &i, const mf<N> &o, int oi) {
-    bool take = oi >= 0;
-    if (take && i >= 0) take = gt(o, v) ? true : gt(v, o) ? false : oi < i;
-    if (take) {
-        v = o;
-        i = oi;
-    }
-}
-
-// best candidate of the lanes' groups of `width` lanes, in every lane
-template <int N>
-__device__ __forceinline__ void ld_lanes(mf<N> &v, int &i, int width) {
-    for (int off = width / 2; off > 0; off >>= 1) {
-        mf<N> o;
-#pragma unroll
-        for (int l = 0; l < N; ++l) o.v[l] = __shfl_xor_sync(0xffffffffu, v.v[l], off);
-        const int oi = __shfl_xor_sync(0xffffffffu, i, off);
-        ld_better(v, i, o, oi);
     }
 }
 
@@ -631,25 +572,9 @@ static int launch_ldlt_cluster(const Ldlt<N> &F, const scal<N> &alpha, int64_t p
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    // per device: asked, and able to place sixteen
     static std::atomic<unsigned long long> asked{0}, sixteen{0};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return record_cuda_error(e, "sytrf device");
-    const unsigned long long bit = 1ULL << (dev & 63);
-    if (!(asked.load(std::memory_order_acquire) & bit)) {
-        int clusters = 0;
-        cfg.gridDim = dim3(LD_MAXC);
-        attr[0].val.clusterDim.x = LD_MAXC;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
-                cudaSuccess &&
-            cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) == cudaSuccess && clusters > 0)
-            sixteen.fetch_or(bit, std::memory_order_release);
-        else
-            cudaGetLastError();
-        asked.fetch_or(bit, std::memory_order_release);
-    }
-    const int most = sixteen.load(std::memory_order_acquire) & bit ? LD_MAXC : 8;
+    int most = 0;
+    if (int rc = largest_cluster((const void *)kern, LD_NT, 0, asked, sixteen, &most)) return rc;
     int nc = 1;
     while (nc < most && nc * 32 < rows) nc *= 2;
     cfg.gridDim = dim3((unsigned)nc);

@@ -45,6 +45,16 @@ int launch_trsm_info(int N, int side, int uplo, int trans, int diag, int64_t m, 
                      Mat B, const double *alpha, cudaStream_t s, const int *info,
                      int order = 0);
 
+// LU panel of w <= LU_PANEL_W columns (pivots, interchanges inside the panel,
+// rank-1 terms) in one launch; MFLAB_ERR_UNSUPPORTED when it has more rows than
+// a cluster holds.  Then its interchanges on the other columns with the block
+// row's solve on columns first + w .. solve_hi - 1 (lu.cu).
+constexpr int LU_PANEL_W = 16;
+int launch_lu_panel(int N, int64_t m, Mat A, int64_t first, int w, int64_t *ipiv, int *info,
+                    cudaStream_t s);
+int launch_lu_swap_solve(int N, int64_t n, int64_t solve_hi, Mat A, int64_t first, int w,
+                         const int64_t *ipiv, const int *info, cudaStream_t s);
+
 int record_cuda_error(cudaError_t e, const char *where);
 
 // An NVTX range named after the C entry point for the duration of the call,
