@@ -2,9 +2,9 @@
 
 No reference counterpart: MultiFloatLinearAlgebra.jl factors one matrix per
 call.  Every block here follows cholesky!(S_i) / ldiv!(x_i, F_i) of the
-reference exactly (one persistent CTA per block for the factor and the
-forward substitution, a group of four lanes per block for the backward
-substitution), so per block the results equal the single-matrix routines.
+reference exactly (one persistent CTA per block for the factor, a small CTA
+per block for the forward and a lane per block for the backward substitution),
+so per block the results equal the single-matrix routines.
 
     batch = SPDBatch(N, sizes)              # packed device storage
     batch.set_block(i, S_i); batch.set_rhs(i, b_i)
@@ -12,8 +12,7 @@ substitution), so per block the results equal the single-matrix routines.
     Sbar, bbar = pullback(xbar)             # ChainRulesCore-style pullback
 
 `BatchedSPDGraph` captures the whole solve (counter reset, the persistent
-factor kernel, the backward-substitution kernel) in a CUDA graph and
-replays it.  `autotune` picks the launch shape (CTA size, number of
+factor kernel, the two substitution kernels) in a CUDA graph and replays it.  `autotune` picks the launch shape (CTA size, number of
 persistent CTAs) by timing the batch itself.
 """
 from __future__ import annotations
@@ -229,7 +228,9 @@ def solve_spd_batched_rrule(batch: SPDBatch, block: int = 16, tuning=None):
     def pullback(xbar: torch.Tensor):
         lib = _native.load()
         xb = xbar.clone()
-        sb = torch.zeros_like(batch.S)
+        # every block was factored (a failure raised above), so the kernel
+        # writes every entry
+        sb = torch.empty_like(batch.S) if batch.total_s else torch.zeros_like(batch.S)
         rc = lib.mflab_spd_batched_adjoint_ex(
             _handle(batch.device), torch.cuda.current_stream(batch.device).cuda_stream, batch.N,
             batch.nblocks, int(batch.sizes_host.max()) if batch.nblocks else 0,

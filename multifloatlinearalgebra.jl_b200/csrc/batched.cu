@@ -1,7 +1,7 @@
 // Batched SPD factor + solve of many independent uneven blocks, and its
-// adjoint: a persistent launch factors each block and runs its forward
-// substitution (one CTA per block), a second launch runs the backward
-// substitutions (one group of lanes per block, several blocks per warp).
+// adjoint: a persistent launch factors the blocks (one CTA per block), a second
+// runs the forward substitutions (one small CTA per block), a third the
+// backward substitutions (one lane per block).
 //
 // No reference counterpart (MultiFloatLinearAlgebra.jl factors one matrix per
 // call); every block follows the reference's own single-matrix order, so each
@@ -14,7 +14,8 @@
 // ls_s / ls_x apart.  A CTA takes the next block index from a device counter
 // (atomicAdd: blocks are handed out in the caller's order, normally
 // descending size) until all blocks are done; there is no inter-CTA waiting.
-// Per block, all data stays in global memory (L2-resident at these sizes).
+// Between panels a block's data stays in global memory (L2-resident at these
+// sizes).
 #include <atomic>
 
 #include "mf_device.cuh"
@@ -24,11 +25,10 @@ namespace mfl {
 
 constexpr int BATCH_NT = 256;   // default threads per CTA
 constexpr int BATCH_MAXN = 512;  // largest block size
-// The per-CTA shared row buffer (forward values, then backward products)
-// holds the batch's largest block (dynamic shared memory, 32 bytes per row),
-// so batches of small blocks leave room for many CTAs per SM: each block's
-// factor and solve are chains of dependent steps, and throughput comes from
-// blocks in flight.
+// Dynamic shared memory is sized by the batch's largest block, so batches of
+// small blocks leave room for many CTAs per SM: each block's factor and solve
+// are chains of dependent steps, and throughput comes from blocks in flight.
+constexpr int SPD_W = 16;  // columns of a staged panel
 
 template <int N>
 struct BlockView {
@@ -108,74 +108,101 @@ __device__ int cta_potrf(const BlockView<N> &F, int64_t block, double (*bc)[4], 
     return 0;
 }
 
-// x <- L^{-1} x, the forward half of solve.jl:54-83, one vector, in place, by
-// a CTA of NT threads (thread t owns rows t, t + NT, ... of the wavefront; the
-// running values sit in the shared row buffer)
+// The same with the panel (at most SPD_W columns, all rows below its top) staged
+// in shared memory, P[k][l][row] with `rows` entries per limb row.  The panel
+// and the solve below it run together, right-looking: at step k the owner of
+// row k takes the root, every row below divides, and every row applies its term
+// k to its remaining columns — each entry receives its operations in the order
+// of the two loops above.  A step is a root, a division and a subtraction of
+// latency (2.5 k cycles in x2) for all rows at once, and the trailing update
+// reads both factors of a product from shared memory, where it read four values
+// per product through L1.  10 000 blocks of 8 .. 256 rows in x2: 20.7 ms
+// (29.4 ms with the forward substitution on the loops above, which batches with less than two CTAs of this
+// kind per SM still take).
 template <int N, int NT>
-__device__ void cta_forward(const BlockView<N> &F, double *x, int64_t ls_x, double (*bc)[4],
-                            double (*prod)[4]) {
+__device__ int cta_potrf_staged(const BlockView<N> &F, int block, double *P, int rows, int *flag) {
     const int t = threadIdx.x;
-    const int64_t n = F.n;
-    auto xget = [&](int64_t i) {
+    const int n = (int)F.n;
+    const mf<N> mone = from_double<N>(-1.0), one = from_double<N>(1.0);
+    auto get = [&](int k, int row) {
         mf<N> v;
 #pragma unroll
-        for (int l = 0; l < N; ++l) v.v[l] = x[l * ls_x + i];
+        for (int l = 0; l < N; ++l) v.v[l] = P[(k * N + l) * rows + row];
         return v;
     };
-    auto xput = [&](int64_t i, const mf<N> &v) {
+    auto set = [&](int k, int row, const mf<N> &v) {
 #pragma unroll
-        for (int l = 0; l < N; ++l) x[l * ls_x + i] = v.v[l];
+        for (int l = 0; l < N; ++l) P[(k * N + l) * rows + row] = v.v[l];
     };
-    auto vget = [&](int64_t i) {
-        mf<N> v;
-#pragma unroll
-        for (int l = 0; l < N; ++l) v.v[l] = prod[i][l];
-        return v;
-    };
-    auto vput = [&](int64_t i, const mf<N> &v) {
-#pragma unroll
-        for (int l = 0; l < N; ++l) prod[i][l] = v.v[l];
-    };
-    // forward substitution, wavefront: row r receives its terms k = 0..r-1 in
-    // ascending order as the unknowns are finalised
-    for (int64_t r = t; r < n; r += NT) vput(r, xget(r));
-    // The critical path of a step runs through the owner of row k + 1 (its
-    // update by x_k, then its division): that thread reads L[k+1, k] and
-    // L[k+1, k+1] before the step's barrier, so neither load waits on it.
-    mf<N> dk = F.at(0, 0), ak = dk;
-    for (int64_t k = 0; k < n; ++k) {
-        const bool next = k + 1 < n && ((k + 1) % NT) == t;
-        mf<N> an = ak, dn = dk;
-        if (next) {
-            an = F.at(k + 1, k);
-            dn = F.at(k + 1, k + 1);
-        }
-        if ((k % NT) == t) {
-            const mf<N> vk = div(vget(k), dk);
-            xput(k, vk);
-#pragma unroll
-            for (int l = 0; l < N; ++l) bc[k & 1][l] = vk.v[l];
+    for (int first = 0; first < n; first += block) {
+        const int w = block < n - first ? block : n - first;
+        const int R = n - first;  // rows of the panel
+        for (int k = 0; k < w; ++k)
+            for (int r = k + t; r < R; r += NT) set(k, r, F.at(first + r, first + k));
+        __syncthreads();
+        for (int k = 0; k < w; ++k) {
+            // row k belongs to thread k % NT, which applied its last term itself
+            if (t == k % NT) {
+                const mf<N> d = get(k, k);
+                if (!gt(d, from_double<N>(0.0))) *flag = first + k + 1;
+                else set(k, k, sqrt_mf(d));
+            }
+            __syncthreads();
+            if (*flag) {  // the panel's own columns before the failure
+                for (int c = 0; c < k; ++c)
+                    for (int r = c + t; r < w; r += NT) F.put(first + r, first + c, get(c, r));
+                return *flag;
+            }
+            const mf<N> p = get(k, k);
+            for (int r = t; r < R; r += NT)
+                if (r > k) set(k, r, div(get(k, r), p));
+            __syncthreads();
+            for (int r = t; r < R; r += NT) {
+                if (r <= k) continue;
+                const mf<N> x = get(k, r);
+                const int hi = r < w ? r + 1 : w;
+#pragma unroll 2
+                for (int j = k + 1; j < hi; ++j) set(j, r, submul(get(j, r), x, get(k, j)));
+            }
         }
         __syncthreads();
-        mf<N> xk;
-#pragma unroll
-        for (int l = 0; l < N; ++l) xk.v[l] = bc[k & 1][l];
-        for (int64_t r = k + 1 + ((t - (k + 1)) % NT + NT) % NT; r < n; r += NT)
-            vput(r, submul(vget(r), r == k + 1 ? an : F.at(r, k), xk));
-        if (next) dk = dn;
+        for (int k = 0; k < w; ++k)
+            for (int r = k + t; r < R; r += NT) F.put(first + r, first + k, get(k, r));
+        // lower trailing update: -1 * (A21 A21^T) + 1 * A22 (syrk.jl:1-50), the
+        // packed lower triangle dealt to the threads; entry e is in column c
+        // from c*m - c(c-1)/2 on, and c only moves forward with e
+        const int m = R - w, tot = m * (m + 1) / 2;
+        int c = 0, start = 0;
+        for (int e = t; e < tot; e += NT) {
+            while (start + (m - c) <= e) {
+                start += m - c;
+                ++c;
+            }
+            const int r = c + (e - start);
+            const int64_t row = first + w + r, col = first + w + c;
+            const mf<N> old = F.at(row, col);
+            mf<N> acc = from_double<N>(0.0);
+            if (w == SPD_W) {
+#pragma unroll 4
+                for (int k = 0; k < SPD_W; ++k) acc = add(acc, mul(get(k, w + r), get(k, w + c)));
+            } else {
+                for (int k = 0; k < w; ++k) acc = add(acc, mul(get(k, w + r), get(k, w + c)));
+            }
+            F.put(row, col, add(mul(mone, acc), mul(one, old)));
+        }
+        __syncthreads();
     }
-    __syncthreads();
+    return 0;
 }
 
+// rows > 0: the staged panel of `rows` rows per limb in dynamic shared memory
 template <int N, int NT>
 __global__ void __launch_bounds__(NT)
-    spd_batched_kernel(int64_t nblocks, const int64_t *sizes, const int64_t *offsets,
-                       const int64_t *boffsets, const int64_t *order, double *S, int64_t ls_s,
-                       double *X, int64_t ls_x, int64_t block, int *info, int *counter,
-                       int solve, int64_t maxn) {
+    spd_factor_kernel(int64_t nblocks, const int64_t *sizes, const int64_t *offsets,
+                      const int64_t *order, double *S, int64_t ls_s, int64_t block, int *info,
+                      int *counter, int64_t maxn, int rows) {
+    extern __shared__ double spd_panel[];
     __shared__ double bc[2][4];
-    extern __shared__ double prod_raw[];  // [max block size][4]
-    double(*prod)[4] = reinterpret_cast<double(*)[4]>(prod_raw);
     __shared__ int64_t job;
     __shared__ int flag;
     const int t = threadIdx.x;
@@ -189,154 +216,254 @@ __global__ void __launch_bounds__(NT)
         if (idx >= nblocks) return;
         const int64_t b = order[idx];
         const int64_t n = sizes[b];
-        if (n > maxn) {  // the row buffer holds maxn rows: refuse the block
+        if (n > maxn) {  // shared memory is sized for maxn rows: refuse the block
             if (t == 0) info[b] = -1;
             __syncthreads();
             continue;
         }
         BlockView<N> F{Mat{S + offsets[b], n > 0 ? n : 1, ls_s}, n};
-        const int st = cta_potrf<N, NT>(F, block, bc, &flag);
+        const int st = rows > 0 ? cta_potrf_staged<N, NT>(F, (int)block, spd_panel, rows, &flag)
+                                : cta_potrf<N, NT>(F, block, bc, &flag);
         if (t == 0) info[b] = st;
-        if (st == 0 && solve) cta_forward<N, NT>(F, X + boffsets[b], ls_x, bc, prod);
         __syncthreads();
     }
 }
 
-// Backward substitution x <- L^{-T} y of every factored block, after the
-// factor kernel's forward pass.  The reference's chain for row r is
-// v = y[r]; v -= L[k, r] * x[k] for k = r+1..n-1 ascending; v /= L[r, r]
-// (solve.jl:54-83 through trsm.jl's upper-transposed loop): one dependent
-// subtraction per term, n(n-1)/2 per block, that no reordering may shorten.
-// A group of BW_G lanes serves one block: the group forms the products of a
-// row in parallel (coalesced reads of column r of L) into its shared slice,
-// then its first lane runs the chain.  A warp carries 32 / BW_G blocks, so
-// every instruction of the chains advances that many blocks at once, where a
-// whole CTA per block would leave all but one thread waiting on the chain.
-constexpr int BW_G = 4;                 // lanes per block
-constexpr int BW_PER_WARP = 32 / BW_G;  // blocks per warp (one warp per CTA)
-
-template <int N>
+// Forward substitution x <- L^{-1} x of every factored block (solve.jl:54-83):
+// row r receives its terms k = 0..r-1 in ascending order as the unknowns are
+// finalised.  G lanes per block: every lane forms the unknown itself (a
+// division costs a warp the same issue slots for one lane as for 32), and the
+// lanes share the rows below.  Many blocks are bound by issue, so two share a
+// warp; few are bound by a block's own steps and take a warp each.  us, x2,
+// 10 000 blocks of 8 .. 256 rows: G = 8 985, 16 616, 32 977 (64 threads per
+// block behind a CTA barrier 1158); x4, 600 blocks of 8 .. 200 rows: G = 16
+// 1130, 32 910, 128 1067.
+template <int N, int G>
 __global__ void __launch_bounds__(32)
-    spd_batched_backward_kernel(int64_t nblocks, const int64_t *sizes, const int64_t *offsets,
-                                const int64_t *boffsets, const int64_t *order, const double *L,
-                                int64_t ls_s, double *X, int64_t ls_x, const int *info,
-                                int64_t maxn) {
-    extern __shared__ double bw_prod[];  // BW_PER_WARP slices of maxn * N (+1 pad)
-    const int lane = threadIdx.x;
-    const int g = lane / BW_G, m = lane % BW_G;
-    const int64_t idx = (int64_t)blockIdx.x * BW_PER_WARP + g;
-    int64_t b = 0, n = 0;
+    spd_forward_kernel(int64_t nblocks, const int64_t *sizes, const int64_t *offsets,
+                       const int64_t *boffsets, const int64_t *order, const double *L, int64_t ls_s,
+                       double *X, int64_t ls_x, const int *info, int64_t maxn) {
+    extern __shared__ double fw_v[];  // a slice [N][maxn] of running values per block
+    const int g = threadIdx.x / G, m = threadIdx.x % G, rows = (int)maxn;
+    const int64_t idx = (int64_t)blockIdx.x * (32 / G) + g;
+    int64_t b = 0;
+    int n = 0;
     if (idx < nblocks) {
         b = order[idx];
-        n = sizes[b];
-        if (n > maxn || info[b] != 0) n = 0;  // nothing to solve for this group
+        n = sizes[b] > maxn || info[b] != 0 ? 0 : (int)sizes[b];  // 0: nothing to solve
     }
-    // The groups step together: step i solves row n - 1 - i of every block
-    // (a chain of i terms in each), so the warp's loops have the same trip
-    // counts in all groups and its lanes stay converged; a group whose block
-    // is smaller (blocks come in descending size, so rarely) sits out its
-    // last steps.
-    const int nmax = __reduce_max_sync(0xffffffffu, (unsigned)n);
-    double *P = bw_prod + (size_t)g * (size_t)(maxn * N + 1);
-    const double *Lb = L + (n ? offsets[b] : 0);
+    const int nmax = __reduce_max_sync(0xffffffffu, n);
+    const double *col = L + (n ? offsets[b] : 0);  // column k
     double *x = X + (n ? boffsets[b] : 0);
-    for (int i = 0; i < nmax; ++i) {
-        const bool act = i < n;
-        const int64_t r = n - 1 - i;
-        const double *col = Lb + r * n;
-        if (act) {
-            for (int j = m; j < i; j += BW_G) {
-                const int64_t k = r + 1 + j;
-                mf<N> a, xv;
+    double *v = fw_v + g * N * rows;
+    for (int r = m; r < n; r += G)
 #pragma unroll
-                for (int l = 0; l < N; ++l) {
-                    a.v[l] = __ldg(col + l * ls_s + k);
-                    xv.v[l] = x[l * ls_x + k];
-                }
-                const mf<N> p = mul(a, xv);
+        for (int l = 0; l < N; ++l) v[l * rows + r] = x[l * ls_x + r];
+    __syncwarp();
+    // a column is read in groups of FW_U rows per lane, all loads before the
+    // first use, the first group of the next column a step ahead
+    constexpr int FW_U = N == 2 ? 8 : 4;
+    mf<N> d = from_double<N>(1.0), ahead[FW_U];
+    auto fetch = [&](mf<N> *a, const double *c, int r0) {
 #pragma unroll
-                for (int l = 0; l < N; ++l) P[k * N + l] = p.v[l];
+        for (int u = 0; u < FW_U; ++u)
+            if (r0 + G * u < n) a[u] = load_mf<N>(c, 0, ls_s, r0 + G * u, 0);
+    };
+    if (n > 0) d = load_mf<N>(col, 0, ls_s, 0, 0);
+#pragma unroll
+    for (int u = 0; u < FW_U; ++u) ahead[u] = d;
+    fetch(ahead, col, 1 + m);
+    for (int k = 0; k < nmax; ++k) {
+        if (k < n) {
+            mf<N> dn = d, a[FW_U];
+#pragma unroll
+            for (int u = 0; u < FW_U; ++u) a[u] = ahead[u];
+            if (k + 1 < n) {
+                dn = load_mf<N>(col + n, 0, ls_s, k + 1, 0);
+                fetch(ahead, col + n, k + 2 + m);
             }
+            const mf<N> xk = div(load_mf<N>(v, 0, rows, k, 0), d);
+            for (int r0 = k + 1 + m; r0 < n; r0 += G * FW_U) {
+                if (r0 > k + 1 + m) fetch(a, col, r0);
+#pragma unroll
+                for (int u = 0; u < FW_U; ++u) {
+                    const int r = r0 + G * u;
+                    if (r >= n) break;
+                    const mf<N> w = submul(load_mf<N>(v, 0, rows, r, 0), a[u], xk);
+#pragma unroll
+                    for (int l = 0; l < N; ++l) v[l * rows + r] = w.v[l];
+                }
+            }
+            if (m == 0) store_mf<N>(x, 0, ls_x, k, 0, xk);
+            d = dn;
+            col += n;
         }
         __syncwarp();
-        if (act && m == 0) {
-            mf<N> v, d;
-#pragma unroll
-            for (int l = 0; l < N; ++l) {
-                v.v[l] = x[l * ls_x + r];
-                d.v[l] = __ldg(col + l * ls_s + r);
-            }
-            // the next term is read from shared memory while the current
-            // subtraction runs, keeping the load off the chain
-            mf<N> p = v;
-            if (r + 1 < n) {
-#pragma unroll
-                for (int l = 0; l < N; ++l) p.v[l] = P[(r + 1) * N + l];
-            }
-            for (int64_t k = r + 1; k < n; ++k) {
-                mf<N> pn = p;
-                if (k + 1 < n) {
-#pragma unroll
-                    for (int l = 0; l < N; ++l) pn.v[l] = P[(k + 1) * N + l];
-                }
-                v = sub(v, p);
-                p = pn;
-            }
-            v = div(v, d);
-#pragma unroll
-            for (int l = 0; l < N; ++l) x[l * ls_x + r] = v.v[l];
+    }
+}
+
+// Backward substitution x <- L^{-T} y of every factored block.  The
+// reference's chain for row r is v = y[r]; v -= L[k, r] * x[k] for
+// k = r+1..n-1 ascending; v /= L[r, r] (solve.jl:54-83 through trsm.jl's
+// upper-transposed loop): one dependent subtraction per term, n(n-1)/2 per
+// block, that no reordering may shorten.  A CTA serves 32 blocks: one warp runs
+// their chains, a block per lane, all on the same row counted from the end;
+// seven warps form the next 32 terms of every block (coalesced reads of column
+// r of L), across row ends: only the product with the unknown just found is
+// the chain's own (its slot holds the coefficient).  The chain warp's place
+// rotates over the schedulers with the CTA.  10 000 blocks in x2: 2.1 ms
+// (3.8 ms with four lanes per block that formed a row's products before its
+// chain); the largest block's chain alone is 1.7 ms.
+constexpr int BW_NT = 256, BW_BLOCKS = 32, BW_TERMS = 32, BW_SMS = 148;
+
+template <int N>
+struct BwStride {  // odd: the terms of one block fall on all banks
+    static constexpr int value = N * BW_BLOCKS + 1;
+};
+
+template <int N>
+__global__ void __launch_bounds__(BW_NT)
+    spd_backward_kernel(int64_t nblocks, const int64_t *sizes, const int64_t *offsets,
+                        const int64_t *boffsets, const int64_t *order, const double *L,
+                        int64_t ls_s, double *X, int64_t ls_x, const int *info, int64_t maxn) {
+    extern __shared__ double bw_prod[];  // [2][BW_TERMS][stride]
+    __shared__ int size_s[BW_BLOCKS];
+    __shared__ const double *L_s[BW_BLOCKS];
+    __shared__ double *x_s[BW_BLOCKS];
+    constexpr int ST = BwStride<N>::value, PER = (BW_BLOCKS + 6) / 7;
+    const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+    const int chain = (int)((blockIdx.x + blockIdx.x / BW_SMS) % 4);
+    const int helper = warp - (warp > chain ? 1 : 0);  // 0 .. 6
+    if (warp == 0) {
+        const int64_t idx = (int64_t)blockIdx.x * BW_BLOCKS + lane;
+        int64_t b = 0, n = 0;
+        if (idx < nblocks) {
+            b = order[idx];
+            n = sizes[b];
+            if (n > maxn || info[b] != 0) n = 0;  // nothing to solve
         }
-        __syncwarp();
+        size_s[lane] = (int)n;
+        L_s[lane] = L + (n ? offsets[b] : 0);
+        x_s[lane] = X + (n ? boffsets[b] : 0);
+    }
+    __syncthreads();
+    const int nmax = __reduce_max_sync(0xffffffffu, size_s[lane]);
+    // row i from the end has i terms; slab j holds the terms 32 j ..
+    auto slabs = [](int i) { return i <= BW_TERMS ? 1 : (i + BW_TERMS - 1) / BW_TERMS; };
+    auto produce = [&](int i, int j, int buf) {
+        double *out = bw_prod + buf * BW_TERMS * ST;
+        mf<N> a[PER], y[PER];
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
+            const int q = helper + 7 * u;
+            const int n = q < BW_BLOCKS ? size_s[q] : 0;
+            const int r = n - 1 - i, k = r + 1 + j * BW_TERMS + lane;
+            const bool ok = r >= 0 && k < n;
+            a[u] = from_double<N>(0.0);
+            y[u] = a[u];
+            if (ok) {
+                a[u] = load_mf<N>(L_s[q], n, ls_s, k, r);
+                if (k > r + 1) y[u] = load_mf<N>(x_s[q], 0, ls_x, k, 0);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
+            const int q = helper + 7 * u;
+            if (q >= BW_BLOCKS) break;
+            const mf<N> p = j == 0 && lane == 0 ? a[u] : mul(a[u], y[u]);
+#pragma unroll
+            for (int l = 0; l < N; ++l) out[lane * ST + l * BW_BLOCKS + q] = p.v[l];
+        }
+    };
+    const int n = size_s[lane];
+    const double *Lb = L_s[lane];
+    double *x = x_s[lane];
+    mf<N> v = from_double<N>(0.0), xr = v, d = v, vn = v, dn = v;
+    auto head = [&](int i) {  // right-hand side and diagonal of row i
+        const int r = n - 1 - i;
+        if (warp == chain && r >= 0) {
+            vn = load_mf<N>(x, 0, ls_x, r, 0);
+            dn = load_mf<N>(Lb, n, ls_s, r, r);
+        }
+    };
+    head(0);
+    int i = 0, j = 0;
+    if (warp != chain && nmax > 0) produce(0, 0, 0);
+    for (int buf = 0; i < nmax; buf ^= 1) {
+        __syncthreads();
+        const bool last = j + 1 >= slabs(i);
+        const int in = last ? i + 1 : i, jn = last ? 0 : j + 1;
+        if (warp != chain) {
+            if (in < nmax) produce(in, jn, buf ^ 1);
+        } else {
+            const double *src = bw_prod + buf * BW_TERMS * ST + lane;
+            auto term = [&](int q) {
+                mf<N> p;
+#pragma unroll
+                for (int l = 0; l < N; ++l) p.v[l] = src[q * ST + l * BW_BLOCKS];
+                return p;
+            };
+            const int left = i - j * BW_TERMS;
+            const int cnt = left < BW_TERMS ? left : BW_TERMS;
+            int q = 0;
+            if (j == 0) {
+                v = vn;
+                d = dn;
+                head(i + 1);
+                if (cnt > 0) {
+                    v = sub(v, mul(term(0), xr));
+                    q = 1;
+                }
+            }
+            for (; q + 8 <= cnt; q += 8)
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v = sub(v, term(q + e));
+            for (; q < cnt; ++q) v = sub(v, term(q));
+            if (last) {
+                xr = div(v, d);
+                if (i < n) store_mf<N>(x, 0, ls_x, n - 1 - i, 0, xr);
+            }
+        }
+        i = in;
+        j = jn;
     }
 }
 
 // Adjoint of x = S^{-1} b for loss gradients: given the factor L (in place),
-// x and xbar, writes bbar = S^{-1} xbar (over xbar) and
-// Sbar = -(bbar x^T + x bbar^T) / 2 into the packed Sbar buffer.  Phase 0
-// runs the forward substitution of xbar, the backward kernel follows, and
-// phase 1 forms Sbar.
-template <int N, int NT>
-__global__ void __launch_bounds__(NT)
-    spd_batched_adjoint_kernel(int64_t nblocks, const int64_t *sizes, const int64_t *offsets,
-                               const int64_t *boffsets, const int64_t *order, const double *L,
-                               int64_t ls_s, const double *X, double *XB, int64_t ls_x,
-                               double *SB, const int *info, int *counter, int64_t maxn,
-                               int phase) {
-    __shared__ double bc[2][4];
-    extern __shared__ double prod_raw[];  // [max block size][4]
-    double(*prod)[4] = reinterpret_cast<double(*)[4]>(prod_raw);
-    __shared__ int64_t job;
-    const int t = threadIdx.x;
-    for (;;) {
-        if (t == 0) job = atomicAdd(counter, 1);
-        __syncthreads();
-        const int64_t idx = job;
-        if (idx >= nblocks) return;
-        const int64_t b = order[idx];
-        const int64_t n = sizes[b];
-        if (info[b] == 0 && n <= maxn && phase == 0) {
-            BlockView<N> F{Mat{(double *)L + offsets[b], n > 0 ? n : 1, ls_s}, n};
-            cta_forward<N, NT>(F, XB + boffsets[b], ls_x, bc, prod);
-        } else if (info[b] == 0 && n <= maxn) {
-            const double *x = X + boffsets[b];
-            const double *xb = XB + boffsets[b];
-            double *sb = SB + offsets[b];
-            for (int64_t e = t; e < n * n; e += NT) {
-                const int64_t r = e % n, c = e / n;
-                mf<N> xr, xc, br, bcv;
+// x and xbar, bbar = S^{-1} xbar (the two kernels above, over xbar) and then
+// Sbar = -(bbar x^T + x bbar^T) / 2 into the packed Sbar buffer: one CTA per
+// block, both vectors in shared memory, one column per warp.  Bound by writing
+// Sbar.  10 000 blocks in x2: 770 us (1.1 ms with the vectors read per
+// entry and a 64-bit division for its column).
+constexpr int SPD_ADJ_NT = 256;
+
+template <int N>
+__global__ void __launch_bounds__(SPD_ADJ_NT)
+    spd_adjoint_kernel(const int64_t *sizes, const int64_t *offsets, const int64_t *boffsets,
+                       const int64_t *order, const double *X, const double *XB, int64_t ls_x,
+                       double *SB, int64_t ls_s, const int *info, int64_t maxn) {
+    extern __shared__ double adj_vec[];  // [2][N][max block size]
+    const int64_t b = order[blockIdx.x];
+    const int n = (int)sizes[b];
+    if (n == 0 || sizes[b] > maxn || info[b] != 0) return;
+    double *xs = adj_vec, *bs = adj_vec + N * maxn;
+    for (int r = threadIdx.x; r < n; r += SPD_ADJ_NT)
 #pragma unroll
-                for (int l = 0; l < N; ++l) {
-                    xr.v[l] = x[l * ls_x + r];
-                    xc.v[l] = x[l * ls_x + c];
-                    br.v[l] = xb[l * ls_x + r];
-                    bcv.v[l] = xb[l * ls_x + c];
-                }
-                mf<N> g = add(mul(br, xc), mul(xr, bcv));
-#pragma unroll
-                for (int l = 0; l < N; ++l) sb[l * ls_s + c * n + r] = -0.5 * g.v[l];
-            }
+        for (int l = 0; l < N; ++l) {
+            xs[l * maxn + r] = X[l * ls_x + boffsets[b] + r];
+            bs[l * maxn + r] = XB[l * ls_x + boffsets[b] + r];
         }
-        __syncthreads();
+    __syncthreads();
+    const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+    for (int c = warp; c < n; c += SPD_ADJ_NT / 32) {
+        const mf<N> xc = load_mf<N>(xs, 0, maxn, c, 0), bcv = load_mf<N>(bs, 0, maxn, c, 0);
+        double *sb = SB + offsets[b] + (int64_t)c * n;
+        for (int r = lane; r < n; r += 32) {
+            const mf<N> xr = load_mf<N>(xs, 0, maxn, r, 0), br = load_mf<N>(bs, 0, maxn, r, 0);
+            const mf<N> g = add(mul(br, xc), mul(xr, bcv));
+#pragma unroll
+            for (int l = 0; l < N; ++l) sb[l * ls_s + r] = -0.5 * g.v[l];
+        }
     }
 }
 
@@ -349,63 +476,111 @@ static int batched_check(int limbs, int64_t nblocks, int64_t maxn) {
     return MFLAB_OK;
 }
 
+// Shared memory of a staged panel for blocks of at most maxn rows, or 0 where
+// the unstaged loops are taken: a panel wider than SPD_W, or fewer than two
+// staged CTAs per SM (x2 above 448 rows, x3 above 296, x4 above 224).
+static size_t staged_bytes(int limbs, int64_t maxn, int64_t block) {
+    if (block > mfl::SPD_W) return 0;
+    const size_t bytes = (size_t)limbs * mfl::SPD_W * (size_t)(maxn > 0 ? maxn : 1) * sizeof(double);
+    return bytes <= 112 * 1024 ? bytes : 0;
+}
+
+template <int N, int NT>
+static int launch_factor_n(int grid, int64_t maxn, cudaStream_t s, int64_t nblocks,
+                           const int64_t *sizes, const int64_t *offsets, const int64_t *order,
+                           double *S, int64_t ls_s, int64_t block, int *info, int *counter) {
+    auto kern = mfl::spd_factor_kernel<N, NT>;
+    const size_t smem = staged_bytes(N, maxn, block);
+    if (smem > 48 * 1024) {
+        static std::atomic<unsigned long long> done{0};
+        int rc = mfl::set_smem_once((const void *)kern, 112 * 1024, done, "spd factor smem");
+        if (rc) return rc;
+    }
+    if (grid <= 0) {  // as many CTAs as the SMs hold
+        int per = 0;
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, NT, smem);
+        if (e != cudaSuccess) return mfl::record_cuda_error(e, "spd factor occupancy");
+        grid = 148 * (per > 0 ? per : 1);
+    }
+    if (grid > nblocks) grid = (int)nblocks;
+    kern<<<grid, NT, smem, s>>>(nblocks, sizes, offsets, order, S, ls_s, block, info, counter, maxn,
+                                smem ? (int)(maxn > 0 ? maxn : 1) : 0);
+    return mfl::record_cuda_error(cudaGetLastError(), "spd factor");
+}
+
 template <int NT>
-static void launch_batched(int limbs, int grid, int64_t maxn, cudaStream_t s, int64_t nblocks,
-                           const int64_t *sizes, const int64_t *offsets, const int64_t *boffsets,
-                           const int64_t *order, double *S, int64_t ls_s, double *X, int64_t ls_x,
-                           int64_t block, int *info, int *counter, int solve) {
-    const size_t smem = (size_t)(maxn > 0 ? maxn : 1) * 4 * sizeof(double);
+static int launch_factor(int limbs, int grid, int64_t maxn, cudaStream_t s, int64_t nblocks,
+                         const int64_t *sizes, const int64_t *offsets, const int64_t *order,
+                         double *S, int64_t ls_s, int64_t block, int *info, int *counter) {
     switch (limbs) {
-    case 2: mfl::spd_batched_kernel<2, NT><<<grid, NT, smem, s>>>(nblocks, sizes, offsets, boffsets, order, S, ls_s, X, ls_x, block, info, counter, solve, maxn); break;
-    case 3: mfl::spd_batched_kernel<3, NT><<<grid, NT, smem, s>>>(nblocks, sizes, offsets, boffsets, order, S, ls_s, X, ls_x, block, info, counter, solve, maxn); break;
-    default: mfl::spd_batched_kernel<4, NT><<<grid, NT, smem, s>>>(nblocks, sizes, offsets, boffsets, order, S, ls_s, X, ls_x, block, info, counter, solve, maxn); break;
+    case 2: return launch_factor_n<2, NT>(grid, maxn, s, nblocks, sizes, offsets, order, S, ls_s, block, info, counter);
+    case 3: return launch_factor_n<3, NT>(grid, maxn, s, nblocks, sizes, offsets, order, S, ls_s, block, info, counter);
+    default: return launch_factor_n<4, NT>(grid, maxn, s, nblocks, sizes, offsets, order, S, ls_s, block, info, counter);
+    }
+}
+
+template <int N, int G>
+static int launch_forward(cudaStream_t s, int64_t nblocks, int64_t maxn, const int64_t *sizes,
+                          const int64_t *offsets, const int64_t *boffsets, const int64_t *order,
+                          const double *L, int64_t ls_s, double *X, int64_t ls_x, const int *info) {
+    auto kern = mfl::spd_forward_kernel<N, G>;
+    constexpr int per = 32 / G;  // blocks per CTA
+    const size_t smem = (size_t)per * N * (size_t)maxn * sizeof(double);
+    if (smem > 48 * 1024) {
+        static std::atomic<unsigned long long> done{0};
+        int rc = mfl::set_smem_once((const void *)kern,
+                                    per * N * mfl::BATCH_MAXN * (int)sizeof(double), done,
+                                    "spd forward smem");
+        if (rc) return rc;
+    }
+    kern<<<(unsigned)((nblocks + per - 1) / per), 32, smem, s>>>(
+        nblocks, sizes, offsets, boffsets, order, L, ls_s, X, ls_x, info, maxn);
+    return mfl::record_cuda_error(cudaGetLastError(), "spd forward");
+}
+
+// x <- S^{-1} x of every factored block: forward, then backward substitution
+template <int N>
+static int launch_solve_n(cudaStream_t s, int64_t nblocks, int64_t maxn, const int64_t *sizes,
+                          const int64_t *offsets, const int64_t *boffsets, const int64_t *order,
+                          const double *L, int64_t ls_s, double *X, int64_t ls_x, const int *info) {
+    if (nblocks > 2147483647LL) return MFLAB_ERR_UNSUPPORTED;
+    int rc;
+    if (nblocks >= 148 * 16)
+        rc = launch_forward<N, 16>(s, nblocks, maxn, sizes, offsets, boffsets, order, L, ls_s, X, ls_x, info);
+    else
+        rc = launch_forward<N, 32>(s, nblocks, maxn, sizes, offsets, boffsets, order, L, ls_s, X, ls_x, info);
+    if (rc) return rc;
+    auto kern = mfl::spd_backward_kernel<N>;
+    constexpr size_t smem = sizeof(double) * 2 * mfl::BW_TERMS * mfl::BwStride<N>::value;
+    if (smem > 48 * 1024) {
+        static std::atomic<unsigned long long> done{0};
+        rc = mfl::set_smem_once((const void *)kern, (int)smem, done, "spd backward smem");
+        if (rc) return rc;
+    }
+    kern<<<(unsigned)((nblocks + mfl::BW_BLOCKS - 1) / mfl::BW_BLOCKS), mfl::BW_NT, smem, s>>>(
+        nblocks, sizes, offsets, boffsets, order, L, ls_s, X, ls_x, info, maxn);
+    return mfl::record_cuda_error(cudaGetLastError(), "spd backward");
+}
+
+static int launch_solve(int limbs, cudaStream_t s, int64_t nblocks, int64_t maxn,
+                        const int64_t *sizes, const int64_t *offsets, const int64_t *boffsets,
+                        const int64_t *order, const double *L, int64_t ls_s, double *X,
+                        int64_t ls_x, const int *info) {
+    switch (limbs) {
+    case 2: return launch_solve_n<2>(s, nblocks, maxn, sizes, offsets, boffsets, order, L, ls_s, X, ls_x, info);
+    case 3: return launch_solve_n<3>(s, nblocks, maxn, sizes, offsets, boffsets, order, L, ls_s, X, ls_x, info);
+    default: return launch_solve_n<4>(s, nblocks, maxn, sizes, offsets, boffsets, order, L, ls_s, X, ls_x, info);
     }
 }
 
 template <int N>
-static int launch_backward_n(cudaStream_t s, int64_t nblocks, int64_t maxn, const int64_t *sizes,
-                             const int64_t *offsets, const int64_t *boffsets,
-                             const int64_t *order, const double *L, int64_t ls_s, double *X,
-                             int64_t ls_x, const int *info) {
-    const size_t smem = (size_t)mfl::BW_PER_WARP * (size_t)((maxn > 0 ? maxn : 1) * N + 1) *
-                        sizeof(double);
-    if (smem > 48 * 1024) {  // large blocks only: the opt-in above the default limit
-        static std::atomic<unsigned long long> done{0};
-        constexpr int max_smem =
-            mfl::BW_PER_WARP * (mfl::BATCH_MAXN * N + 1) * (int)sizeof(double);
-        int rc = mfl::set_smem_once((const void *)mfl::spd_batched_backward_kernel<N>, max_smem,
-                                    done, "spd batched backward smem");
-        if (rc) return rc;
-    }
-    const int64_t grid = (nblocks + mfl::BW_PER_WARP - 1) / mfl::BW_PER_WARP;
-    mfl::spd_batched_backward_kernel<N><<<(unsigned)grid, 32, smem, s>>>(
-        nblocks, sizes, offsets, boffsets, order, L, ls_s, X, ls_x, info, maxn);
-    return 0;
-}
-
-static int launch_backward(int limbs, cudaStream_t s, int64_t nblocks, int64_t maxn,
-                           const int64_t *sizes, const int64_t *offsets, const int64_t *boffsets,
-                           const int64_t *order, const double *L, int64_t ls_s, double *X,
-                           int64_t ls_x, const int *info) {
-    switch (limbs) {
-    case 2: return launch_backward_n<2>(s, nblocks, maxn, sizes, offsets, boffsets, order, L, ls_s, X, ls_x, info);
-    case 3: return launch_backward_n<3>(s, nblocks, maxn, sizes, offsets, boffsets, order, L, ls_s, X, ls_x, info);
-    default: return launch_backward_n<4>(s, nblocks, maxn, sizes, offsets, boffsets, order, L, ls_s, X, ls_x, info);
-    }
-}
-
-template <int NT>
-static void launch_adjoint(int limbs, int grid, int64_t maxn, cudaStream_t s, int64_t nblocks,
-                           const int64_t *sizes, const int64_t *offsets, const int64_t *boffsets,
-                           const int64_t *order, const double *L, int64_t ls_s, const double *X,
-                           double *XB, int64_t ls_x, double *SB, const int *info, int *counter,
-                           int phase) {
-    const size_t smem = (size_t)(maxn > 0 ? maxn : 1) * 4 * sizeof(double);
-    switch (limbs) {
-    case 2: mfl::spd_batched_adjoint_kernel<2, NT><<<grid, NT, smem, s>>>(nblocks, sizes, offsets, boffsets, order, L, ls_s, X, XB, ls_x, SB, info, counter, maxn, phase); break;
-    case 3: mfl::spd_batched_adjoint_kernel<3, NT><<<grid, NT, smem, s>>>(nblocks, sizes, offsets, boffsets, order, L, ls_s, X, XB, ls_x, SB, info, counter, maxn, phase); break;
-    default: mfl::spd_batched_adjoint_kernel<4, NT><<<grid, NT, smem, s>>>(nblocks, sizes, offsets, boffsets, order, L, ls_s, X, XB, ls_x, SB, info, counter, maxn, phase); break;
-    }
+static void launch_sbar(cudaStream_t s, int64_t nblocks, int64_t maxn, const int64_t *sizes,
+                        const int64_t *offsets, const int64_t *boffsets, const int64_t *order,
+                        const double *X, const double *XB, int64_t ls_x, double *SB, int64_t ls_s,
+                        const int *info) {
+    mfl::spd_adjoint_kernel<N><<<(unsigned)nblocks, mfl::SPD_ADJ_NT,
+                                 (size_t)maxn * 2 * N * sizeof(double), s>>>(
+        sizes, offsets, boffsets, order, X, XB, ls_x, SB, ls_s, info, maxn);
 }
 
 extern "C" int mflab_spd_batched_ex(mflab_handle *h, void *stream, int limbs, int64_t nblocks,
@@ -424,25 +599,17 @@ extern "C" int mflab_spd_batched_ex(mflab_handle *h, void *stream, int limbs, in
     cudaStream_t s = (cudaStream_t)stream;
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(int), s);
     if (e != cudaSuccess) return mfl::record_cuda_error(e, "spd batched counter");
-    if (grid <= 0) grid = 148 * 4;
     if (threads == 64)
-        launch_batched<64>(limbs, grid, max_size, s, nblocks, sizes, offsets, boffsets, order, S, ls_s, X, ls_x, block, info, counter, solve);
+        rc = launch_factor<64>(limbs, grid, max_size, s, nblocks, sizes, offsets, order, S, ls_s, block, info, counter);
     else if (threads == 128)
-        launch_batched<128>(limbs, grid, max_size, s, nblocks, sizes, offsets, boffsets, order, S, ls_s, X, ls_x, block, info, counter, solve);
+        rc = launch_factor<128>(limbs, grid, max_size, s, nblocks, sizes, offsets, order, S, ls_s, block, info, counter);
     else if (threads == 256)
-        launch_batched<256>(limbs, grid, max_size, s, nblocks, sizes, offsets, boffsets, order, S, ls_s, X, ls_x, block, info, counter, solve);
+        rc = launch_factor<256>(limbs, grid, max_size, s, nblocks, sizes, offsets, order, S, ls_s, block, info, counter);
     else
-        launch_batched<512>(limbs, grid, max_size, s, nblocks, sizes, offsets, boffsets, order, S, ls_s, X, ls_x, block, info, counter, solve);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return mfl::record_cuda_error(e, "spd batched");
-    if (solve) {
-        // the factor kernel ran the forward half; the backward chains follow
-        int rc2 = launch_backward(limbs, s, nblocks, max_size, sizes, offsets, boffsets, order,
-                                  S, ls_s, X, ls_x, info);
-        if (rc2) return rc2;
-        return mfl::record_cuda_error(cudaGetLastError(), "spd batched backward");
-    }
-    return MFLAB_OK;
+        rc = launch_factor<512>(limbs, grid, max_size, s, nblocks, sizes, offsets, order, S, ls_s, block, info, counter);
+    if (rc || !solve) return rc;
+    return launch_solve(limbs, s, nblocks, max_size, sizes, offsets, boffsets, order, S, ls_s, X,
+                        ls_x, info);
 }
 
 extern "C" int mflab_spd_batched(mflab_handle *h, void *stream, int limbs, int64_t nblocks,
@@ -470,30 +637,19 @@ extern "C" int mflab_spd_batched_adjoint_ex(mflab_handle *h, void *stream, int l
     if (threads != 64 && threads != 128 && threads != 256 && threads != 512) return MFLAB_ERR_ARG;
     if (nblocks == 0) return MFLAB_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(int), s);
-    if (e != cudaSuccess) return mfl::record_cuda_error(e, "spd adjoint counter");
-    if (grid <= 0) grid = 148 * 4;
-    for (int phase = 0; phase < 2; ++phase) {
-        if (phase == 1) {
-            // bbar's backward chains, then the counter again for phase 1
-            rc = launch_backward(limbs, s, nblocks, max_size, sizes, offsets, boffsets, order, L,
-                                 ls_s, XB, ls_x, info);
-            if (rc) return rc;
-            e = cudaMemsetAsync(counter, 0, sizeof(int), s);
-            if (e != cudaSuccess) return mfl::record_cuda_error(e, "spd adjoint counter");
-        }
-        if (threads == 64)
-            launch_adjoint<64>(limbs, grid, max_size, s, nblocks, sizes, offsets, boffsets, order, L, ls_s, X, XB, ls_x, SB, info, counter, phase);
-        else if (threads == 128)
-            launch_adjoint<128>(limbs, grid, max_size, s, nblocks, sizes, offsets, boffsets, order, L, ls_s, X, XB, ls_x, SB, info, counter, phase);
-        else if (threads == 256)
-            launch_adjoint<256>(limbs, grid, max_size, s, nblocks, sizes, offsets, boffsets, order, L, ls_s, X, XB, ls_x, SB, info, counter, phase);
-        else
-            launch_adjoint<512>(limbs, grid, max_size, s, nblocks, sizes, offsets, boffsets, order, L, ls_s, X, XB, ls_x, SB, info, counter, phase);
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return mfl::record_cuda_error(e, "spd adjoint");
+    // these kernels take their own shape; grid, threads and counter are the
+    // factor's and stay in the signature
+    (void)grid;
+    (void)counter;
+    rc = launch_solve(limbs, s, nblocks, max_size, sizes, offsets, boffsets, order, L, ls_s, XB,
+                      ls_x, info);
+    if (rc || max_size == 0) return rc;
+    switch (limbs) {
+    case 2: launch_sbar<2>(s, nblocks, max_size, sizes, offsets, boffsets, order, X, XB, ls_x, SB, ls_s, info); break;
+    case 3: launch_sbar<3>(s, nblocks, max_size, sizes, offsets, boffsets, order, X, XB, ls_x, SB, ls_s, info); break;
+    default: launch_sbar<4>(s, nblocks, max_size, sizes, offsets, boffsets, order, X, XB, ls_x, SB, ls_s, info); break;
     }
-    return MFLAB_OK;
+    return mfl::record_cuda_error(cudaGetLastError(), "spd adjoint");
 }
 
 extern "C" int mflab_spd_batched_adjoint(mflab_handle *h, void *stream, int limbs,
