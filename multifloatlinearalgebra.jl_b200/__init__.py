@@ -20,6 +20,7 @@ from __future__ import annotations
 
 import ctypes as C
 import dataclasses
+import math
 import threading
 from typing import Optional, Sequence, Union
 
@@ -151,7 +152,8 @@ def destroy_handle(h: C.c_void_p) -> None:
 
 
 def _stream(device: int) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    # the current stream's handle without a Stream object (about 1.3 us)
+    return torch._C._cuda_getCurrentRawStream(device)
 
 
 def limb_type_name(N: int) -> str:
@@ -257,6 +259,16 @@ class MFMatrix:
     def ptr(self) -> int:
         return self.storage.data_ptr() + 8 * (self.c0 * self.ld + self.r0)
 
+    def _args(self) -> tuple:
+        """(ptr, ld, ls) as every C entry takes them, read from the storage
+        once (a small call spends most of its time in such reads)"""
+        st = self.storage
+        limbs, cols, rows = st.shape
+        plane, column, _ = st.stride()
+        ld = column if cols > 1 else max(rows, 1)
+        ls = plane if limbs > 1 else cols * max(rows, 1)
+        return st.data_ptr() + 8 * (self.c0 * ld + self.r0), ld, ls
+
     def __len__(self):
         return self.m
 
@@ -332,8 +344,8 @@ class MFMatrix:
         lib = _native.load()
         h = handle or _handle(self.device)
         s = _stream(self.device) if stream is None else stream.cuda_stream
-        _check(lib.mflab_h2d_interleaved(h, s, self.N, self.m, self.n, ptr, shape[1], self.ptr(),
-                                         self.ld, self.ls), "h2d_interleaved")
+        _check(lib.mflab_h2d_interleaved(h, s, self.N, self.m, self.n, ptr, shape[1],
+                                         *self._args()), "h2d_interleaved")
         return self
 
     def copy_to_interleaved_(self, X, stream=None, handle=None):
@@ -346,8 +358,8 @@ class MFMatrix:
         lib = _native.load()
         h = handle or _handle(self.device)
         s = _stream(self.device) if stream is None else stream.cuda_stream
-        _check(lib.mflab_d2h_interleaved(h, s, self.N, self.m, self.n, self.ptr(), self.ld,
-                                         self.ls, ptr, shape[1]), "d2h_interleaved")
+        _check(lib.mflab_d2h_interleaved(h, s, self.N, self.m, self.n, *self._args(), ptr,
+                                         shape[1]), "d2h_interleaved")
         return X
 
     @classmethod
@@ -400,7 +412,14 @@ class MFMatrix:
 
 
 # ------------------------------------------------------------ helpers ----
+# the scalars of nearly every call, read only by the library
+_UNITS = {v: (C.c_double * 4)(v, 0.0, 0.0, 0.0) for v in (1.0, -1.0)}
+_UNITS[0.0] = (C.c_double * 4)()
+
+
 def _scalar(N: int, v) -> "C.Array":
+    if type(v) is float and v in _UNITS and not (v == 0.0 and math.copysign(1.0, v) < 0):
+        return _UNITS[v]
     arr = (C.c_double * 4)()
     if isinstance(v, (int, float)):
         arr[0] = float(v)
@@ -414,13 +433,15 @@ def _scalar(N: int, v) -> "C.Array":
 
 
 def _same_type(*mats: MFMatrix) -> int:
-    N = mats[0].N
+    first = mats[0].storage
+    N, device = first.shape[0], first.get_device()
     for x in mats:
         if not isinstance(x, MFMatrix):
             raise ArgumentError("expected MFMatrix operands")
-        if x.N != N:
+        st = x.storage
+        if st.shape[0] != N:
             raise ArgumentError("operands have different limb counts")
-        if x.device != mats[0].device:
+        if st.get_device() != device:
             raise ArgumentError("operands live on different devices")
     if not 1 <= N <= 4:
         raise ArgumentError("only 1-4 limb MultiFloats are supported")
@@ -431,10 +452,10 @@ def _same_type(*mats: MFMatrix) -> int:
 
 def _mightalias(a: MFMatrix, b: MFMatrix) -> bool:
     """2-D index-range overlap of two views (Base.mightalias on views)."""
-    if a.storage.data_ptr() != b.storage.data_ptr():
-        sa, ea = a.storage.data_ptr(), a.storage.data_ptr() + 8 * a.storage.numel()
-        sb, eb = b.storage.data_ptr(), b.storage.data_ptr() + 8 * b.storage.numel()
-        return sa < eb and sb < ea
+    sa, sb = a.storage, b.storage
+    pa, pb = sa.data_ptr(), sb.data_ptr()
+    if pa != pb:
+        return pa < pb + 8 * sb.numel() and pb < pa + 8 * sa.numel()
     rows = a.r0 < b.r0 + b.m and b.r0 < a.r0 + a.m
     cols = a.c0 < b.c0 + b.n and b.c0 < a.c0 + a.n
     return rows and cols and a.m > 0 and b.m > 0 and a.n > 0 and b.n > 0
@@ -446,7 +467,8 @@ def _no_alias(op: str, dest: MFMatrix, src: MFMatrix) -> None:
 
 
 def _lib_h(x: MFMatrix):
-    return _native.load(), _handle(x.device), _stream(x.device)
+    device = x.storage.get_device()
+    return _native.load(), _handle(device), _stream(device)
 
 
 _ORDERS = {"matched": 0, "fast": 1}
@@ -487,8 +509,8 @@ def gemm_(C_: MFMatrix, A: MFMatrix, B: MFMatrix, alpha=1.0, beta=0.0,
     if route == 2:
         rc = _gemm_ozaki(lib, h, s, N, C_, A, B, alpha, beta, config)
     else:
-        rc = lib.mflab_gemm(h, s, N, route, m, n, k, A.ptr(), A.ld, A.ls, B.ptr(), B.ld, B.ls,
-                            C_.ptr(), C_.ld, C_.ls, _scalar(N, alpha), _scalar(N, beta))
+        rc = lib.mflab_gemm(h, s, N, route, m, n, k, *A._args(), *B._args(),
+                            *C_._args(), _scalar(N, alpha), _scalar(N, beta))
     _check(rc, "gemm!")
     return C_
 
@@ -527,7 +549,7 @@ def _int8_engine(config: KernelConfig) -> int:
 def _gemm_ozaki(lib, h, s, N, C_, A, B, alpha, beta, config):
     _check(lib.mflab_set_int8_engine(h, _int8_engine(config)), "gemm!")
     m, k, n = A.m, A.n, B.n
-    args = (m, n, k, A.ptr(), A.ld, A.ls, B.ptr(), B.ld, B.ls, C_.ptr(), C_.ld, C_.ls,
+    args = (m, n, k, *A._args(), *B._args(), *C_._args(),
             _scalar(N, alpha), _scalar(N, beta))
     scheme = ozaki_scheme(config)
     if scheme == "modular":
@@ -566,8 +588,8 @@ def ozaki_crt_tune_moduli(A: MFMatrix, B: MFMatrix) -> int:
         raise DimensionMismatch("gemm! inner dimensions differ")
     lib, h, s = _lib_h(A)
     T = C.c_int()
-    _check(lib.mflab_ozaki_crt_tune(h, s, N, A.m, B.n, A.n, A.ptr(), A.ld, A.ls, B.ptr(), B.ld,
-                                    B.ls, C.byref(T)), "ozaki tune")
+    _check(lib.mflab_ozaki_crt_tune(h, s, N, A.m, B.n, A.n, *A._args(), *B._args(), C.byref(T)),
+           "ozaki tune")
     return int(T.value)
 
 
@@ -596,7 +618,7 @@ class PreparedInt8Operand:
         self.device = A.device
         self.buffer = torch.empty(max(nbytes.value, 1), dtype=torch.uint8,
                                   device=A.storage.device)
-        _check(lib.mflab_ozaki_crt_prepare(h, s, N, self.moduli, A.m, A.n, A.ptr(), A.ld, A.ls,
+        _check(lib.mflab_ozaki_crt_prepare(h, s, N, self.moduli, A.m, A.n, *A._args(),
                                            self.buffer.data_ptr()), "ozaki prepare")
 
 
@@ -615,8 +637,8 @@ def gemm_prepared_(C_: MFMatrix, P: PreparedInt8Operand, B: MFMatrix, alpha=1.0,
     lib, h, s = _lib_h(C_)
     _check(lib.mflab_set_int8_engine(h, _int8_engine(config)), "gemm!")
     _check(lib.mflab_gemm_ozaki_crt_prepared(h, s, N, P.moduli, P.m, B.n, P.k,
-                                             P.buffer.data_ptr(), B.ptr(), B.ld, B.ls, C_.ptr(),
-                                             C_.ld, C_.ls, _scalar(N, alpha), _scalar(N, beta)),
+                                             P.buffer.data_ptr(), *B._args(), *C_._args(),
+                                             _scalar(N, alpha), _scalar(N, beta)),
            "gemm!")
     return C_
 
@@ -667,7 +689,7 @@ def gemv_(y: MFMatrix, A: MFMatrix, x: MFMatrix, alpha=1.0, beta=0.0, trans: str
     _no_alias("gemv!", y, A)
     _no_alias("gemv!", y, x)
     lib, h, s = _lib_h(y)
-    _check(lib.mflab_gemv(h, s, N, 0 if trans == "N" else 1, m, n, A.ptr(), A.ld, A.ls, x.ptr(),
+    _check(lib.mflab_gemv(h, s, N, 0 if trans == "N" else 1, m, n, *A._args(), x.ptr(),
                           x.ls, y.ptr(), y.ls, _scalar(N, alpha), _scalar(N, beta)), "gemv!")
     return y
 
@@ -689,7 +711,7 @@ def symv_(y: MFMatrix, A: MFMatrix, x: MFMatrix, alpha=1.0, beta=0.0, uplo: str 
     _no_alias("symv!", y, A)
     _no_alias("symv!", y, x)
     lib, h, s = _lib_h(y)
-    _check(lib.mflab_symv(h, s, N, 0 if uplo == "lower" else 1, n, A.ptr(), A.ld, A.ls, x.ptr(),
+    _check(lib.mflab_symv(h, s, N, 0 if uplo == "lower" else 1, n, *A._args(), x.ptr(),
                           x.ls, y.ptr(), y.ls, _scalar(N, alpha), _scalar(N, beta)), "symv!")
     return y
 
@@ -702,7 +724,7 @@ def mfdot(x: MFMatrix, y: MFMatrix) -> np.ndarray:
         raise DimensionMismatch("dot product shapes differ")
     out = torch.zeros(N, dtype=torch.float64, device=x.storage.device)
     lib, h, s = _lib_h(x)
-    _check(lib.mflab_dot(h, s, N, x.m, x.n, x.ptr(), x.ld, x.ls, y.ptr(), y.ld, y.ls,
+    _check(lib.mflab_dot(h, s, N, x.m, x.n, *x._args(), *y._args(),
                          out.data_ptr()), "mfdot")
     return out.cpu().numpy()
 
@@ -723,8 +745,8 @@ def syrk_packed_(packed: MFMatrix, panel: MFMatrix, alpha=1.0, beta=0.0, reducti
         raise BoundsError(f"reduction range {reduction_first}:{reduction_last} outside 1:{kp}")
     _no_alias("syrk_packed!", packed, panel)
     lib, h, s = _lib_h(packed)
-    _check(lib.mflab_syrk_packed(h, s, N, n, kp, reduction_first - 1, reduction_last, panel.ptr(),
-                                 panel.ld, panel.ls, packed.ptr(), packed.ls, _scalar(N, alpha),
+    _check(lib.mflab_syrk_packed(h, s, N, n, kp, reduction_first - 1, reduction_last,
+                                 *panel._args(), packed.ptr(), packed.ls, _scalar(N, alpha),
                                  _scalar(N, beta)), "syrk_packed!")
     return packed
 
@@ -744,11 +766,11 @@ def syrk_(C_: MFMatrix, P: MFMatrix, alpha=1.0, beta=0.0, uplo: str = "lower",
         _check(lib.mflab_set_int8_engine(h, _int8_engine(config)), "syrk!")
         if ozaki_scheme(config) != "modular":
             raise ArgumentError("the INT8 syrk! route uses the modular scheme (ozaki_moduli)")
-        rc = lib.mflab_syrk_lower_ozaki(h, s, N, int(config.ozaki_moduli), 1, n, k, P.ptr(), P.ld,
-                                        P.ls, C_.ptr(), C_.ld, C_.ls, _scalar(N, alpha),
+        rc = lib.mflab_syrk_lower_ozaki(h, s, N, int(config.ozaki_moduli), 1, n, k, *P._args(),
+                                        *C_._args(), _scalar(N, alpha),
                                         _scalar(N, beta))
     else:
-        rc = lib.mflab_syrk_lower(h, s, N, n, k, P.ptr(), P.ld, P.ls, C_.ptr(), C_.ld, C_.ls,
+        rc = lib.mflab_syrk_lower(h, s, N, n, k, *P._args(), *C_._args(),
                                   _scalar(N, alpha), _scalar(N, beta))
     _check(rc, "syrk!")
     return C_
@@ -766,8 +788,8 @@ def gemmt_(C_: MFMatrix, A: MFMatrix, B: MFMatrix, alpha=1.0, beta=0.0,
     _no_alias("gemmt!", C_, A)
     _no_alias("gemmt!", C_, B)
     lib, h, s = _lib_h(C_)
-    rc = lib.mflab_gemmt_lower(h, s, N, rows, k, A.ptr(), A.ld, A.ls, B.ptr(), B.ld, B.ls,
-                               C_.ptr(), C_.ld, C_.ls, _scalar(N, alpha), _scalar(N, beta))
+    rc = lib.mflab_gemmt_lower(h, s, N, rows, k, *A._args(), *B._args(),
+                               *C_._args(), _scalar(N, alpha), _scalar(N, beta))
     _check(rc, "gemmt!")
     return C_
 
@@ -800,7 +822,7 @@ def trsm_(B: MFMatrix, A: MFMatrix, alpha=1.0, side: str = "left", uplo: str = "
     lib, h, s = _lib_h(B)
     with _solve_order(B, config):
         rc = lib.mflab_trsm(h, s, N, _SIDE[side], _UPLO[uplo], _TRANS[trans], _DIAG[diag], B.m,
-                            B.n, A.ptr(), A.ld, A.ls, B.ptr(), B.ld, B.ls, _scalar(N, alpha))
+                            B.n, *A._args(), *B._args(), _scalar(N, alpha))
     _check(rc, "trsm!")
     return B
 
@@ -827,7 +849,7 @@ def trmm_(B: MFMatrix, A: MFMatrix, alpha=1.0, side: str = "left", uplo: str = "
     _no_alias("trmm!", B, A)
     lib, h, s = _lib_h(B)
     _check(lib.mflab_trmm(h, s, N, _SIDE[side], _UPLO[uplo], _TRANS[trans], _DIAG[diag], B.m, B.n,
-                          A.ptr(), A.ld, A.ls, B.ptr(), B.ld, B.ls, _scalar(N, alpha)), "trmm!")
+                          *A._args(), *B._args(), _scalar(N, alpha)), "trmm!")
     return B
 
 
@@ -916,7 +938,7 @@ def _read_info(dev_info: torch.Tensor) -> int:
 def _finite_region(A: MFMatrix, region: int) -> bool:
     out = torch.empty(A.N + 1, dtype=torch.float64, device=A.storage.device)
     lib, h, s = _lib_h(A)
-    _check(lib.mflab_max_abs(h, s, A.N, A.m, A.n, A.ptr(), A.ld, A.ls, region, out.data_ptr()),
+    _check(lib.mflab_max_abs(h, s, A.N, A.m, A.n, *A._args(), region, out.data_ptr()),
            "max_abs")
     return bool(out[A.N].item() == 1.0)
 
@@ -934,11 +956,11 @@ def cholesky_(A: MFMatrix, check: bool = True, config: KernelConfig = _DEFAULT) 
         if ozaki_scheme(config) != "modular":
             raise ArgumentError("the INT8 trailing update uses the modular scheme (ozaki_moduli)")
         _check(lib.mflab_set_int8_engine(h, _int8_engine(config)), "cholesky!")
-        _check(lib.mflab_potrf_ozaki(h, s, N, int(config.ozaki_moduli), A.m, A.ptr(), A.ld, A.ls,
+        _check(lib.mflab_potrf_ozaki(h, s, N, int(config.ozaki_moduli), A.m, *A._args(),
                                      max(int(config.ozaki_block), block), block,
                                      info.data_ptr()), "cholesky!")
     else:
-        _check(lib.mflab_potrf(h, s, N, A.m, A.ptr(), A.ld, A.ls, block, info.data_ptr()),
+        _check(lib.mflab_potrf(h, s, N, A.m, *A._args(), block, info.data_ptr()),
                "cholesky!")
     st = _read_info(info)
     if st == -1 and check:
@@ -968,7 +990,7 @@ def cholesky_pivoted_(A: MFMatrix, tol=0.0, check: bool = True,
     perm = torch.empty(max(n, 1), dtype=torch.int64, device=dev)
     rank_info = torch.zeros(2, dtype=torch.int64, device=dev)
     lib, h, s = _lib_h(A)
-    _check(lib.mflab_pstrf(h, s, N, n, A.ptr(), A.ld, A.ls, _scalar(N, t), perm.data_ptr(),
+    _check(lib.mflab_pstrf(h, s, N, n, *A._args(), _scalar(N, t), perm.data_ptr(),
                            rank_info.data_ptr()), "cholesky_pivoted!")
     rank, info = (int(v) for v in rank_info.cpu().tolist())
     if info == -1 and check:
@@ -987,7 +1009,7 @@ def _qr_run(A: MFMatrix, pivoted: int, check: bool, what: str) -> MFQR:
     perm = torch.empty(max(n, 1), dtype=torch.int64, device=dev)
     info = torch.zeros(1, dtype=torch.int32, device=dev)
     lib, h, s = _lib_h(A)
-    _check(lib.mflab_qr(h, s, N, pivoted, m, n, A.ptr(), A.ld, A.ls, tau.data_ptr(), tau.stride(0),
+    _check(lib.mflab_qr(h, s, N, pivoted, m, n, *A._args(), tau.data_ptr(), tau.stride(0),
                         perm.data_ptr(), info.data_ptr()), what)
     st = _read_info(info)
     if st == -1 and check:
@@ -1046,8 +1068,8 @@ def apply_q_(B: MFMatrix, F: MFQR, trans: str = "N") -> MFMatrix:
     Fm = F.factors
     r = min(Fm.m, Fm.n)
     lib, h, s = _lib_h(B)
-    _check(lib.mflab_apply_q(h, s, N, 1 if trans == "T" else 0, Fm.m, r, Fm.ptr(), Fm.ld, Fm.ls,
-                             F.tau.data_ptr(), F.tau.stride(0), B.ptr(), B.ld, B.ls, B.n),
+    _check(lib.mflab_apply_q(h, s, N, 1 if trans == "T" else 0, Fm.m, r, *Fm._args(),
+                             F.tau.data_ptr(), F.tau.stride(0), *B._args(), B.n),
            "apply_q!")
     return B
 
@@ -1097,7 +1119,7 @@ def numerical_rank(F: MFQR, atol=0.0, rtol=0.0) -> int:
     out = torch.zeros(1, dtype=torch.int64, device=F.factors.storage.device)
     Fm = F.factors
     lib, h, s = _lib_h(Fm)
-    _check(lib.mflab_qr_numerical_rank(h, s, N, Fm.m, Fm.n, Fm.ptr(), Fm.ld, Fm.ls,
+    _check(lib.mflab_qr_numerical_rank(h, s, N, Fm.m, Fm.n, *Fm._args(),
                                        _scalar(N, a), _scalar(N, r), out.data_ptr()),
            "numerical_rank")
     return int(out.item())
@@ -1154,19 +1176,19 @@ def lu_(A: MFMatrix, check: bool = True, config: KernelConfig = _DEFAULT,
     omax = torch.zeros(N + 1, dtype=torch.float64, device=dev)
     lib, h, s = _lib_h(A)
     if m > 0 and n > 0:
-        _check(lib.mflab_max_abs(h, s, N, m, n, A.ptr(), A.ld, A.ls, 0, omax.data_ptr()), "lu!")
+        _check(lib.mflab_max_abs(h, s, N, m, n, *A._args(), 0, omax.data_ptr()), "lu!")
     block = max(config.lu_block, 1)
     if config.gemm_strategy == "ozaki":
         # INT8 trailing updates between panels of ozaki_block columns
         if ozaki_scheme(config) != "modular":
             raise ArgumentError("the INT8 trailing update uses the modular scheme (ozaki_moduli)")
         _check(lib.mflab_set_int8_engine(h, _int8_engine(config)), "lu!")
-        _check(lib.mflab_getrf_ozaki(h, s, N, int(config.ozaki_moduli), m, n, A.ptr(), A.ld,
-                                     A.ls, ipiv.data_ptr() if kmax > 0 else None,
+        _check(lib.mflab_getrf_ozaki(h, s, N, int(config.ozaki_moduli), m, n, *A._args(),
+                                     ipiv.data_ptr() if kmax > 0 else None,
                                      max(int(config.ozaki_block), block), block,
                                      info.data_ptr()), "lu!")
     else:
-        _check(lib.mflab_getrf(h, s, N, m, n, A.ptr(), A.ld, A.ls,
+        _check(lib.mflab_getrf(h, s, N, m, n, *A._args(),
                                ipiv.data_ptr() if kmax > 0 else None, block, info.data_ptr()),
                "lu!")
     st = _read_info(info)
@@ -1221,9 +1243,9 @@ def ldlt_(A: MFMatrix, check: bool = True, config: KernelConfig = _DEFAULT,
     omax = torch.zeros(N + 1, dtype=torch.float64, device=dev)
     lib, h, s = _lib_h(A)
     if n > 0:
-        _check(lib.mflab_max_abs(h, s, N, n, n, A.ptr(), A.ld, A.ls, 1, omax.data_ptr()), "ldlt!")
+        _check(lib.mflab_max_abs(h, s, N, n, n, *A._args(), 1, omax.data_ptr()), "ldlt!")
     blocked = 1 if plan["strategy"] == "blocked" else 0
-    _check(lib.mflab_sytrf(h, s, N, n, A.ptr(), A.ld, A.ls, dsub.data_ptr(), dsub.shape[1],
+    _check(lib.mflab_sytrf(h, s, N, n, *A._args(), dsub.data_ptr(), dsub.shape[1],
                            pivots.data_ptr() if n else None, blocks.data_ptr(), blocked,
                            plan["block_size"], info.data_ptr()), "ldlt!")
     st = _read_info(info)
@@ -1274,7 +1296,7 @@ def _ldlt_diag_record(F: MFLDLT) -> np.ndarray:
     out = torch.zeros(6 + 4 * N, dtype=torch.float64, device=A.storage.device)
     lib, h, s = _lib_h(A)
     ds = F.dsub
-    _check(lib.mflab_ldlt_diagnostics(h, s, N, A.m, A.ptr(), A.ld, A.ls, ds.data_ptr(),
+    _check(lib.mflab_ldlt_diagnostics(h, s, N, A.m, *A._args(), ds.data_ptr(),
                                       ds.stride(0) if ds.shape[0] > 1 else max(ds.shape[1], 1),
                                       F.blocks.data_ptr(), F.original_maximum.data_ptr(),
                                       out.data_ptr()), "factor_diagnostics")
@@ -1366,11 +1388,10 @@ def ldiv_(dest: MFMatrix, F: _Factor, source: Optional[MFMatrix] = None,
     L = F.factors
     with _solve_order(dest, config):
         if F.kind == "cholesky":
-            rc = lib.mflab_potrs(h, s, N, n, dest.n, L.ptr(), L.ld, L.ls, dest.ptr(), dest.ld,
-                                 dest.ls)
+            rc = lib.mflab_potrs(h, s, N, n, dest.n, *L._args(), *dest._args())
         elif F.kind == "lu":
-            rc = lib.mflab_getrs(h, s, N, n, dest.n, L.ptr(), L.ld, L.ls, F.ipiv.data_ptr(),
-                                 dest.ptr(), dest.ld, dest.ls)
+            rc = lib.mflab_getrs(h, s, N, n, dest.n, *L._args(), F.ipiv.data_ptr(),
+                                 *dest._args())
         else:
             return _ldiv_extra(dest, F, lib, h, s)
     _check(rc, "ldiv!")
@@ -1384,8 +1405,8 @@ def _ldiv_extra(dest, F, lib, h, s):
     fail = torch.zeros(1, dtype=torch.int32, device=dest.storage.device)
     ds = F.dsub
     lsd = ds.stride(0) if ds.shape[0] > 1 else max(ds.shape[1], 1)
-    _check(lib.mflab_sytrs(h, s, N, L.m, dest.n, L.ptr(), L.ld, L.ls, ds.data_ptr(), lsd,
-                           F.pivots.data_ptr(), F.blocks.data_ptr(), dest.ptr(), dest.ld, dest.ls,
+    _check(lib.mflab_sytrs(h, s, N, L.m, dest.n, *L._args(), ds.data_ptr(), lsd,
+                           F.pivots.data_ptr(), F.blocks.data_ptr(), *dest._args(),
                            fail.data_ptr()), "ldiv!")
     f = int(fail.item())
     if 0 < f < 0x7F7F7F7F:
@@ -1419,7 +1440,7 @@ def factor_diagnostics(F: _Factor, atol=0.0, rtol=0.0) -> dict:
     if F.kind == "cholesky":
         n = A.m
         accepted = n if F.info == 0 else (F.info - 1 if F.info > 0 else 0)
-        _check(lib.mflab_diag_summary(h, s, N, A.ptr(), A.ld, A.ls, accepted, None, None,
+        _check(lib.mflab_diag_summary(h, s, N, *A._args(), accepted, None, None,
                                       out.data_ptr()), "factor_diagnostics")
         mn, mx, spread, _ = _mf_values(out, N, 4)
         has = accepted > 0
@@ -1434,7 +1455,7 @@ def factor_diagnostics(F: _Factor, atol=0.0, rtol=0.0) -> dict:
     if F.kind == "qr":
         # diagnostics.jl:248-275; atol / rtol are forwarded to numerical_rank
         r = min(A.m, A.n)
-        _check(lib.mflab_diag_summary(h, s, N, A.ptr(), A.ld, A.ls, r, None, None,
+        _check(lib.mflab_diag_summary(h, s, N, *A._args(), r, None, None,
                                       out.data_ptr()), "factor_diagnostics")
         mn, mx, spread, _ = _mf_values(out, N, 4)
         has = r > 0
@@ -1454,7 +1475,7 @@ def factor_diagnostics(F: _Factor, atol=0.0, rtol=0.0) -> dict:
     if F.kind == "cholesky_pivoted":
         # diagnostics.jl:53-70: the retained rank is the accepted pivot count
         accepted = F.rank
-        _check(lib.mflab_diag_summary(h, s, N, A.ptr(), A.ld, A.ls, accepted, None, None,
+        _check(lib.mflab_diag_summary(h, s, N, *A._args(), accepted, None, None,
                                       out.data_ptr()), "factor_diagnostics")
         mn, mx, spread, _ = _mf_values(out, N, 4)
         has = accepted > 0
@@ -1471,9 +1492,9 @@ def factor_diagnostics(F: _Factor, atol=0.0, rtol=0.0) -> dict:
         kmax = min(A.m, A.n)
         accepted = F.info - 1 if F.info > 0 else (kmax if F.info == 0 else 0)
         umax = torch.zeros(N + 1, dtype=torch.float64, device=dev)
-        _check(lib.mflab_max_abs(h, s, N, A.m, A.n, A.ptr(), A.ld, A.ls, 2, umax.data_ptr()),
+        _check(lib.mflab_max_abs(h, s, N, A.m, A.n, *A._args(), 2, umax.data_ptr()),
                "factor_diagnostics")
-        _check(lib.mflab_diag_summary(h, s, N, A.ptr(), A.ld, A.ls, accepted, umax.data_ptr(),
+        _check(lib.mflab_diag_summary(h, s, N, *A._args(), accepted, umax.data_ptr(),
                                       F.original_maximum.data_ptr(), out.data_ptr()),
                "factor_diagnostics")
         mn, mx, _, growth = _mf_values(out, N, 4)
@@ -1553,9 +1574,8 @@ def residual_(R: MFMatrix, A: MFMatrix, X: MFMatrix, B: MFMatrix, uplo: str = "g
                                                   and (R.r0, R.c0) == (B.r0, B.c0)):
         raise ArgumentError("residual output may equal b but must not partially alias it")
     lib, h, s = _lib_h(R)
-    _check(lib.mflab_residual(h, s, N, _UPLO_R[uplo], int(R.is_vector), A.m, A.n, R.n, A.ptr(),
-                              A.ld, A.ls, X.ptr(), X.ld, X.ls, B.ptr(), B.ld, B.ls, R.ptr(), R.ld,
-                              R.ls), "residual!")
+    _check(lib.mflab_residual(h, s, N, _UPLO_R[uplo], int(R.is_vector), A.m, A.n, R.n, *A._args(),
+                              *X._args(), *B._args(), *R._args()), "residual!")
     return R
 
 
@@ -1572,9 +1592,8 @@ def residual_mixed_(R: MFMatrix, A: MFMatrix, X: MFMatrix, B: MFMatrix, uplo: st
         raise ArgumentError("residual_mixed! supports only widening to a higher limb count")
     _check_residual_dims(R, A, X, B, uplo)
     lib, h, s = _lib_h(R)
-    _check(lib.mflab_residual_mixed(h, s, src, res, _UPLO_R[uplo], A.m, A.n, R.n, A.ptr(), A.ld,
-                                    A.ls, X.ptr(), X.ld, X.ls, B.ptr(), B.ld, B.ls, R.ptr(), R.ld,
-                                    R.ls), "residual_mixed!")
+    _check(lib.mflab_residual_mixed(h, s, src, res, _UPLO_R[uplo], A.m, A.n, R.n, *A._args(),
+                                    *X._args(), *B._args(), *R._args()), "residual_mixed!")
     return R
 
 
@@ -1592,7 +1611,7 @@ class OpNormInf:
         lib, h, s = _lib_h(A)
         if handle is not None:
             h = handle
-        _check(lib.mflab_opnorm_inf(h, s, N, _UPLO_R[uplo], A.m, A.n, A.ptr(), A.ld, A.ls,
+        _check(lib.mflab_opnorm_inf(h, s, N, _UPLO_R[uplo], A.m, A.n, *A._args(),
                                     self.value.data_ptr(), self.nonfinite.data_ptr()),
                "opnorm")
 
@@ -1610,13 +1629,13 @@ def normwise_backward_error(A: MFMatrix, X: MFMatrix, B: MFMatrix, R: MFMatrix,
         if (anorm.N, anorm.m, anorm.k) != (N, A.m, A.n):
             raise DimensionMismatch("normwise_backward_error: anorm belongs to another matrix")
         _check(lib.mflab_backward_error_norm(h, s, N, A.m, A.n, R.n, anorm.value.data_ptr(),
-                                             anorm.nonfinite.data_ptr(), X.ptr(), X.ld, X.ls,
-                                             B.ptr(), B.ld, B.ls, R.ptr(), R.ld, R.ls,
+                                             anorm.nonfinite.data_ptr(), *X._args(),
+                                             *B._args(), *R._args(),
                                              out.data_ptr()), "normwise_backward_error")
     else:
-        _check(lib.mflab_backward_error(h, s, N, _UPLO_R[uplo], A.m, A.n, R.n, A.ptr(), A.ld,
-                                        A.ls, X.ptr(), X.ld, X.ls, B.ptr(), B.ld, B.ls, R.ptr(),
-                                        R.ld, R.ls, out.data_ptr()), "normwise_backward_error")
+        _check(lib.mflab_backward_error(h, s, N, _UPLO_R[uplo], A.m, A.n, R.n, *A._args(),
+                                        *X._args(), *B._args(), *R._args(), out.data_ptr()),
+                                        "normwise_backward_error")
     vals = out.cpu().numpy().reshape(-1, N)[:R.n]
     return vals[0].copy() if R.is_vector else [v.copy() for v in vals]
 
@@ -1695,7 +1714,7 @@ def solve_mixed_lu(A: MFMatrix, B: MFMatrix, tol: float = 0.0, maxiter: int = 40
     LU = _leading_limb(A)
     ipiv = torch.arange(1, n + 1, dtype=torch.int64, device=dev)
     info = torch.zeros(1, dtype=torch.int32, device=dev)
-    _check(lib.mflab_getrf(h, s, 1, n, n, LU.ptr(), LU.ld, LU.ls, ipiv.data_ptr() if n else None,
+    _check(lib.mflab_getrf(h, s, 1, n, n, *LU._args(), ipiv.data_ptr() if n else None,
                            _LU64_PANEL, info.data_ptr()), "lu! (binary64)")
     if timing:
         ev[1].record()
@@ -1724,8 +1743,8 @@ def solve_mixed_lu(A: MFMatrix, B: MFMatrix, tol: float = 0.0, maxiter: int = 40
         D.planes().copy_(R.planes()[0:1])  # round(R): the leading limbs
         _check(lib.mflab_lu64_solve(h, s, n, D.n, LU.ptr(), LU.ld, work.data_ptr(), D.ptr(),
                                     D.ld), "ldiv! (binary64)")
-        _check(lib.mflab_add_widened(h, s, 1, N, n, X.n, D.ptr(), D.ld, D.ls, X.ptr(), X.ld,
-                                     X.ls), "refinement update")
+        _check(lib.mflab_add_widened(h, s, 1, N, n, X.n, *D._args(), *X._args()),
+               "refinement update")
         if residual == "int8":
             R.copy_(B)
             if prepared is None:

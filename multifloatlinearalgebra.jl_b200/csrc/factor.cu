@@ -1643,7 +1643,9 @@ __global__ void __launch_bounds__(NT) maxabs_partial_kernel(int64_t m, int64_t n
     }
 }
 
-// one warp over the partial maxima
+// One warp over the partial maxima.  With a non-finite entry the maximum depends
+// on the order (a NaN yields to what follows it): then one lane folds the parts
+// in ascending order.
 template <int N>
 __global__ void maxabs_final_kernel(int nparts, const double *part, double *out) {
     mf<N> best = from_double<N>(0.0);
@@ -1663,6 +1665,15 @@ __global__ void maxabs_final_kernel(int nparts, const double *part, double *out)
     }
     fin = __all_sync(0xffffffffu, fin);
     if (threadIdx.x) return;
+    if (!fin) {
+        best = from_double<N>(0.0);
+        for (int i = 0; i < nparts; ++i) {
+            mf<N> v;
+#pragma unroll
+            for (int l = 0; l < N; ++l) v.v[l] = part[i * (N + 1) + l];
+            best = max_mf(best, v);
+        }
+    }
 #pragma unroll
     for (int l = 0; l < N; ++l) out[l] = best.v[l];
     out[N] = fin ? 1.0 : 0.0;
