@@ -254,7 +254,8 @@ int mflab_set_int8_engine(mflab_handle *h, int engine);
 
 /* Device-side status word of the tcgen05 kernels issued through this handle:
    0, or the code of a bounded wait that ran out (MFLAB_ERR_TIMEOUT is then
-   the caller's conclusion: 1 producer, 2 MMA issuer, 3 epilogue, 4 drain).
+   the caller's conclusion: 1 producer, 2 MMA issuer, 3 epilogue, 4 drain; 5 the
+   binary64 LU panel's exchange, 6 the one-launch binary64 solve).
    Reading it resets it to 0.  Synchronises.  No reference counterpart. */
 int mflab_device_status(mflab_handle *h, int *status);
 

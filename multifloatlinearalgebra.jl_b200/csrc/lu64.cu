@@ -35,7 +35,7 @@ namespace mfl {
 namespace {
 
 constexpr int IB = 128;        // diagonal block size
-constexpr int64_t PIVOT_PERM_MAXN_LU64 = 24576;  // indices in shared memory (96 KB)
+constexpr int64_t PIVOT_PERM_MAXN_LU64 = 24576;  // indices and pivots in shared memory (192 KB)
 
 size_t perm_bytes(int64_t n) { return ((size_t)n * 4 + 255) / 256 * 256; }
 int64_t nblocks(int64_t n) { return (n + IB - 1) / IB; }
@@ -102,14 +102,18 @@ __global__ void __launch_bounds__(IB)
 
 // perm[i] = the original row that ends up in row i after the interchanges
 // ipiv[0..n) (1-based, applied in ascending order): replayed by one thread on
-// an index array in shared memory
+// index and pivot arrays in shared memory
 __global__ void lu64_perm_kernel(int64_t n, const int64_t *ipiv, int *perm) {
-    extern __shared__ int sidx[];
-    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) sidx[i] = (int)i;
+    extern __shared__ int sidx[];  // [n] indices, [n] pivots
+    int *spiv = sidx + n;
+    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
+        sidx[i] = (int)i;
+        spiv[i] = (int)(ipiv[i] - 1);
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
         for (int64_t k = 0; k < n; ++k) {
-            const int64_t p = ipiv[k] - 1;
+            const int p = spiv[k];
             if (p != k) {
                 const int x = sidx[k];
                 sidx[k] = sidx[p];
@@ -239,6 +243,223 @@ int mstep_launch(cudaStream_t s, int64_t nrhs, int64_t j0, int jb, const double 
                              "lu64 solve step");
 }
 
+// The same solve in one cooperative launch, every CTA 32 rows of the right-hand
+// side in registers.  A step of the block kernel above is bound by launch and
+// load latency (7.2 us a step at n = 4096, 64 steps); here the owners of block
+// i publish its rows and every CTA that still needs them reads them, applies its
+// 32 x 128 slice of M (or inv(D_i), an owner) and goes on to the next block.
+// The rows are their own flags: the buffer starts as all ones (a NaN no value
+// is written as), and a reader polls its own words until none of them is, so a
+// step costs one store and one load through L2 instead of a fence, a flag and
+// then the load.  The rows are written LS_COPIES times: copy 0 is for the
+// owners of the block itself and of the next one, the only CTAs the chain of
+// steps waits for, and the others' polls are spread over the rest.  The slices do not depend on the solve: two are prefetched
+// into shared memory ahead of the rows.  Arithmetic and results are the block
+// kernel's.  All CTAs are co-resident (cooperative launch); a wait that runs
+// out (LS_SPIN polls) records error 6 and the CTA leaves at its next barrier,
+// the others as their waits run out or see the abort word.  n = 4096, 16
+// right-hand sides: 220 us (460 us as 64 launches, 348 us with flags, 286 us
+// before the 2 x 2 tiles below).
+constexpr int LS_STAGES = 3, LS_ERR_TIMEOUT = 6;
+constexpr long long LS_SPIN = 1LL << 21;
+constexpr int64_t LS_MAX_RHS = 32;  // more right-hand sides: the block kernel
+constexpr unsigned long long LS_UNSET = ~0ULL;
+constexpr int LS_COPIES = 4;
+
+__device__ __forceinline__ void ls_cp_async(void *dst, const void *src, int bytes, bool pred) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    if (bytes == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src),
+                     "r"(pred ? 16 : 0)
+                     : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src),
+                     "r"(pred ? 8 : 0)
+                     : "memory");
+}
+__device__ __forceinline__ unsigned long long ls_word(double v) {
+    const unsigned long long w = (unsigned long long)__double_as_longlong(v);
+    return w == LS_UNSET ? 0x7ff8000000000000ULL : w;
+}
+
+struct LsShared {
+    double tile[LS_STAGES][IB][MS_ROWS];  // slices of M or inv(D), [k][row]
+    double b[IB][MS_RHS];                 // the block's rows
+};
+
+// pub: [chunk][2][nblk][LS_COPIES][IB][MS_RHS] words, all LS_UNSET at the start
+__global__ void __launch_bounds__(MS_NT)
+    lu64_solve_kernel(int64_t n, int64_t nrhs, const int *perm, const double *__restrict__ invL,
+                      const double *__restrict__ invU, const double *__restrict__ ML,
+                      const double *__restrict__ MU, double *B, int64_t ldb,
+                      unsigned long long *pub, int *abort_word, int *err) {
+    extern __shared__ __align__(16) uint8_t ls_raw[];
+    LsShared &sh = *reinterpret_cast<LsShared *>(ls_raw);
+    __shared__ int s_stop;
+    const int t = threadIdx.x, lane = t % 32, warp = t / 32;
+    const int nb = (int)((n + IB - 1) / IB);
+    const int64_t rb = (int64_t)blockIdx.x * MS_ROWS;
+    const int nrows = (int)(n - rb < MS_ROWS ? n - rb : MS_ROWS);
+    const int own = (int)(rb / IB), inner = (int)(rb % IB);
+    // blocks 0 .. own forward, then nb-1 .. own backward
+    const int fwd = own + 1, steps = fwd + nb - own;
+    auto block_of = [&](int s) { return s < fwd ? s : nb - 1 - (s - fwd); };
+    auto rows_of = [&](int i) { return (int)(n - (int64_t)i * IB < IB ? n - (int64_t)i * IB : IB); };
+    // 16-byte copies where every column of the slice starts on 16 bytes
+    const bool wide = nrows == MS_ROWS && (n & 1) == 0 &&
+                      (((uintptr_t)invL | (uintptr_t)invU | (uintptr_t)ML | (uintptr_t)MU) & 15) == 0;
+    auto prefetch = [&](int s) {
+        if (s < steps) {
+            const int i = block_of(s), jb = rows_of(i);
+            const bool forward = s < fwd;
+            const double *src = i == own ? (forward ? invL : invU) + (int64_t)i * IB * IB + inner
+                                         : (forward ? ML : MU) + (int64_t)i * IB * n + rb;
+            const int64_t ld = i == own ? IB : n;
+            double(*tile)[MS_ROWS] = sh.tile[s % LS_STAGES];
+            if (wide) {
+                const int r = 2 * (t % 16), k0 = t / 16;
+                const double *p = src + k0 * ld + r;
+#pragma unroll
+                for (int u = 0; u < IB / 16; ++u, p += 16 * ld)
+                    ls_cp_async(&tile[k0 + 16 * u][r], k0 + 16 * u < jb ? p : src, 16,
+                                k0 + 16 * u < jb);
+            } else {
+                const double *p = src + warp * ld + lane;
+#pragma unroll
+                for (int u = 0; u < IB / 8; ++u, p += 8 * ld) {
+                    const bool ok = lane < nrows && warp + 8 * u < jb;
+                    ls_cp_async(&tile[warp + 8 * u][lane], ok ? p : src, 8, ok);
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (t == 0) s_stop = 0;
+    __syncthreads();
+    // Warps 0-3 hold the right-hand sides, 2 rows x 2 columns per thread (16 x 8
+    // per warp): a k step is then one 16-byte read of the slice and one of the
+    // rows, a wavefront each, for four products; one row per lane and two
+    // columns per warp over eight warps made three wavefronts for two.
+    const bool holds = warp < 4;
+    const int r0 = 16 * (warp & 1) + 2 * (lane % 8), q0 = 8 * (warp >> 1 & 1) + 2 * (lane / 8);
+    bool stop = false;
+    for (int64_t c0 = 0; c0 < nrhs && !stop; c0 += MS_RHS, pub += 2 * (int64_t)nb * LS_COPIES * IB * MS_RHS) {
+        double w[2][2];
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const bool in = holds && r0 + a < nrows && c0 + q0 + c < nrhs;
+                w[a][c] = in ? B[(c0 + q0 + c) * ldb + perm[rb + r0 + a]] : 0.0;
+            }
+        for (int s = 0; s < LS_STAGES - 1; ++s) prefetch(s);
+        for (int s = 0; s < steps; ++s) {
+            const int i = block_of(s), dir = s < fwd ? 0 : 1, jb = rows_of(i);
+            unsigned long long *rows = pub + ((int64_t)dir * nb + i) * LS_COPIES * IB * MS_RHS;
+            if (i == own && holds) {  // this CTA's rows of the block are final
+#pragma unroll
+                for (int c = 0; c < LS_COPIES; ++c)
+#pragma unroll
+                    for (int a = 0; a < 2; ++a)
+                        if (r0 + a < nrows)
+                            asm volatile("st.volatile.global.v2.u64 [%0], {%1, %2};" ::"l"(
+                                             rows + (int64_t)(c * IB + inner + r0 + a) * MS_RHS + q0),
+                                         "l"(ls_word(w[a][0])), "l"(ls_word(w[a][1]))
+                                         : "memory");
+            }
+            const int far = dir == 0 ? own - i : i - own;  // blocks until this CTA's own
+            if (far > 1) rows += (int64_t)(1 + blockIdx.x % (LS_COPIES - 1)) * IB * MS_RHS;
+            prefetch(s + LS_STAGES - 1);
+            // the block's rows: every thread polls its own words
+            constexpr int PER = IB * MS_RHS / (2 * MS_NT);
+            unsigned long long y[PER][2];
+            bool open = true;
+            for (long long polls = 0; open; ++polls) {
+                open = false;
+#pragma unroll
+                for (int u = 0; u < PER; ++u) {
+                    const int e = 2 * (t + u * MS_NT);
+                    y[u][0] = y[u][1] = 0;
+                    if (e / MS_RHS < jb)
+                        asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];"
+                                     : "=l"(y[u][0]), "=l"(y[u][1])
+                                     : "l"(rows + e)
+                                     : "memory");
+                }
+#pragma unroll
+                for (int u = 0; u < PER; ++u)
+                    open = open || y[u][0] == LS_UNSET || y[u][1] == LS_UNSET;
+                if (open && (polls >= LS_SPIN ||
+                             ((polls & 255) == 255 && *(volatile int *)abort_word))) {
+                    if (atomicExch(abort_word, 1) == 0) atomicExch(err, LS_ERR_TIMEOUT);
+                    s_stop = 1;
+                    break;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < PER; ++u) {
+                double2 v;
+                v.x = __longlong_as_double((long long)y[u][0]);
+                v.y = __longlong_as_double((long long)y[u][1]);
+                *(double2 *)(&sh.b[0][0] + 2 * (t + u * MS_NT)) = v;
+            }
+            // the slice of step s has landed (the two newer groups may be open)
+            asm volatile("cp.async.wait_group %0;" ::"n"(LS_STAGES - 1) : "memory");
+            __syncthreads();
+            stop = s_stop != 0;
+            if (stop) break;
+            const double(*tile)[MS_ROWS] = sh.tile[s % LS_STAGES];
+            if (holds) {
+                double x[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll 16
+                for (int k = 0; k < IB; ++k) {
+                    const double2 m = *(const double2 *)&tile[k][r0];
+                    const double2 bb = *(const double2 *)&sh.b[k][q0];
+                    x[0][0] = fma(m.x, bb.x, x[0][0]);
+                    x[0][1] = fma(m.x, bb.y, x[0][1]);
+                    x[1][0] = fma(m.y, bb.x, x[1][0]);
+                    x[1][1] = fma(m.y, bb.y, x[1][1]);
+                }
+#pragma unroll
+                for (int a = 0; a < 2; ++a)
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) w[a][c] = i == own ? x[a][c] : w[a][c] - x[a][c];
+            }
+            __syncthreads();  // tile and b before they are written again
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        if (stop) break;
+        // every CTA has read its right-hand side: this one's last block waited
+        // for rows that depend on all of them
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+                if (holds && r0 + a < nrows && c0 + q0 + c < nrhs)
+                    B[(c0 + q0 + c) * ldb + rb + r0 + a] = w[a][c];
+        __syncthreads();
+    }
+}
+
+// Scratch of the one-launch solve, or 0 where the block kernel is taken: more
+// right-hand sides than two rounds are worth, or more CTAs than fit at once.
+size_t solve_bytes(int64_t n, int64_t nrhs) {
+    if (nrhs > LS_MAX_RHS) return 0;
+    static std::atomic<unsigned long long> configured{0};
+    if (set_smem_once((const void *)lu64_solve_kernel, (int)sizeof(LsShared), configured,
+                      "lu64 solve attribute"))
+        return 0;
+    int dev = 0, sms = 0, per = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, lu64_solve_kernel, MS_NT,
+                                                      sizeof(LsShared)) != cudaSuccess)
+        return 0;
+    if ((n + MS_ROWS - 1) / MS_ROWS > (int64_t)sms * per) return 0;
+    const size_t chunks = (size_t)((nrhs + MS_RHS - 1) / MS_RHS), nb = (size_t)nblocks(n);
+    return sizeof(double) * chunks * 2 * nb * LS_COPIES * IB * MS_RHS + 256;
+}
+
 std::atomic<unsigned long long> g_inv_configured{0};
 
 }  // namespace
@@ -268,10 +489,10 @@ extern "C" int mflab_lu64_prepare(mflab_handle *h, void *stream, int64_t n, cons
     if (rc) return rc;
     static std::atomic<unsigned long long> perm_configured{0};
     rc = mfl::set_smem_once((const void *)mfl::lu64_perm_kernel,
-                            (int)(mfl::PIVOT_PERM_MAXN_LU64 * sizeof(int)), perm_configured,
+                            (int)(2 * mfl::PIVOT_PERM_MAXN_LU64 * sizeof(int)), perm_configured,
                             "lu64 perm attribute");
     if (rc) return rc;
-    mfl::lu64_perm_kernel<<<1, 256, (size_t)n * sizeof(int), s>>>(n, ipiv, perm);
+    mfl::lu64_perm_kernel<<<1, 256, 2 * (size_t)n * sizeof(int), s>>>(n, ipiv, perm);
     mfl::lu64_inv_diag_kernel<<<dim3((unsigned)mfl::nblocks(n), 2), mfl::IB, smem, s>>>(
         n, LU, ldl, invL, invU);
     rc = mfl::record_cuda_error(cudaGetLastError(), "lu64 prepare");
@@ -307,6 +528,21 @@ extern "C" int mflab_lu64_solve(mflab_handle *h, void *stream, int64_t n, int64_
     const int *perm = (const int *)work;
     const double *invL = (const double *)((const char *)work + mfl::perm_bytes(n));
     const double *invU = invL + (size_t)mfl::nblocks(n) * mfl::IB * mfl::IB;
+    const double *ML = invU + (size_t)mfl::nblocks(n) * mfl::IB * mfl::IB, *MU = ML + (size_t)n * n;
+    if (const size_t bytes = mfl::solve_bytes(n, nrhs)) {
+        int rc = mflab_reserve_scratch(h, bytes);
+        if (rc) return rc;
+        unsigned long long *pub = (unsigned long long *)h->scratch;
+        int *abort_word = (int *)((char *)h->scratch + bytes - 256), *err = h->dev_flags + 1;
+        cudaError_t e = cudaMemsetAsync(pub, 0xff, bytes - 256, s);
+        if (e == cudaSuccess) e = cudaMemsetAsync(abort_word, 0, sizeof(int), s);
+        if (e != cudaSuccess) return mfl::record_cuda_error(e, "lu64 solve rows");
+        void *args[] = {&n, &nrhs, &perm, &invL, &invU, &ML, &MU, &B, &ldb, &pub, &abort_word, &err};
+        e = cudaLaunchCooperativeKernel((const void *)mfl::lu64_solve_kernel,
+                                        dim3((unsigned)((n + mfl::MS_ROWS - 1) / mfl::MS_ROWS)),
+                                        dim3(mfl::MS_NT), args, sizeof(mfl::LsShared), s);
+        return mfl::record_cuda_error(e, "lu64 solve");
+    }
     // W: the permuted right-hand sides, then the forward solution
     int rc = mflab_reserve_scratch(h, (size_t)n * nrhs * sizeof(double));
     if (rc) return rc;
@@ -316,7 +552,6 @@ extern "C" int mflab_lu64_solve(mflab_handle *h, void *stream, int64_t n, int64_
                                                                          n);
     rc = mfl::record_cuda_error(cudaGetLastError(), "lu64 gather");
     if (rc) return rc;
-    const double *ML = invU + (size_t)mfl::nblocks(n) * mfl::IB * mfl::IB, *MU = ML + (size_t)n * n;
     const int64_t nb = mfl::nblocks(n);
     // forward: L y = P b, y written into B, W updated below each block
     for (int64_t i = 0; i < nb && rc == MFLAB_OK; ++i) {

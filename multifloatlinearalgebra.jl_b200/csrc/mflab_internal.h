@@ -136,6 +136,10 @@ int int8_gemm_tc_mod(int64_t mp, int64_t np, int64_t K, const int8_t *A, int64_t
                      int64_t a_cols, const int8_t *B, int64_t ldb, int64_t b_cols, int64_t b_xoff,
                      uint8_t *R, int64_t ldr, int *err, cudaStream_t s, const TcOpts &o, int nz,
                      int64_t r_zstride, int tri = 0);
+// all levels of a residue product with at most 32 columns (int8_narrow.cu)
+int int8_gemm_narrow(int Q, int nc, int64_t mp, int64_t kp, const int8_t *A8, const int8_t *B8,
+                     uint8_t *R, int64_t ldr, size_t plane, int nz, int *err, cudaStream_t s,
+                     const TcOpts &o);
 void record_error_message(const char *msg);
 // modular INT8 route (ozaki_crt.cu); T = 0 lets the tuner choose.  The SYRK
 // form writes lower(C) = alpha op(A) op(A)^T + beta lower(C), op(A) = A

@@ -999,6 +999,7 @@ static int ceil_log2(int64_t v) {
 
 struct CrtPlan {
     int Q, h, T, WD, WP;
+    int narrow;  // columns padded to 16 or 32 only (crt_narrow)
     int64_t kp, mp, np, ldi;
     size_t plane, plane8a, plane8b, a8, b8, lev, ws, total;
 };
@@ -1024,6 +1025,7 @@ static void crt_layout(CrtPlan &p);
 // allow; T_req == 0: the tuner's requirement from the sampled scale gap.
 // Returns MFLAB_ERR_UNSUPPORTED when no table entry reaches the requirement.
 static int crt_plan(int N, int64_t m, int64_t n, int64_t k, int T_req, int gap8, CrtPlan &p) {
+    p.narrow = 0;
     p.kp = (k + 127) / 128 * 128;
     if (p.kp == 0) p.kp = 128;
     if (T_req > 0) {
@@ -1071,6 +1073,15 @@ static void crt_layout(CrtPlan &p) {
     p.lev = al((size_t)p.Q * p.T * p.plane);                 // byte residues
     p.ws = ((size_t)64 << 20) + al(p.plane * sizeof(int32_t));  // library path only
     p.total = p.a8 + p.b8 + p.lev + p.ws;
+}
+
+// At most 32 columns on the one-SM tcgen05 engine: columns padded to 16 or 32
+// and all levels in one launch (int8_narrow.cu)
+static void crt_narrow(const mflab_handle *hd, int64_t n, CrtPlan &p) {
+    if (n > 32 || hd->int8_engine != MFLAB_INT8_TCGEN05) return;
+    p.narrow = 1;
+    p.np = n <= 16 ? 16 : 32;
+    crt_layout(p);
 }
 
 template <int N, int WD>
@@ -1219,7 +1230,10 @@ static int crt_gemm_n(mflab_handle *hd, const CrtPlan &p, int64_t m, int64_t n, 
     if (rc) return rc;
     ozaki_phase(1, s);
     const int64_t ld8 = (int64_t)p.Q * p.kp;
-    for (int L = 0; L < p.Q && rc == MFLAB_OK; ++L) {
+    if (p.narrow)
+        rc = int8_gemm_narrow(p.Q, (int)p.np, p.mp, p.kp, A8, B8, Rs, p.ldi, p.plane, p.T,
+                              hd->dev_flags + 1, s, tc_opts(hd));
+    for (int L = 0; L < p.Q && rc == MFLAB_OK && !p.narrow; ++L) {
         const int64_t K = (int64_t)(L + 1) * p.kp, bx = (int64_t)(p.Q - 1 - L) * p.kp;
         uint8_t *RL = Rs + (size_t)L * p.T * p.plane;
         if (tc_engine(hd)) {
@@ -1275,6 +1289,7 @@ int ozaki_crt_gemm(mflab_handle *hd, int N, int T, int64_t m, int64_t n, int64_t
     }
     if ((int64_t)p.T * p.mp > 0x7fffffffLL || (int64_t)p.T * p.np > 0x7fffffffLL)
         return MFLAB_ERR_UNSUPPORTED;
+    crt_narrow(hd, n, p);
     rc = mflab_reserve_scratch(hd, p.total);
     if (rc) return rc;
     if (T_used) *T_used = p.T;
@@ -1635,6 +1650,7 @@ extern "C" int mflab_gemm_ozaki_crt_prepared(mflab_handle *h, void *stream, int 
     if (m == 0 || n == 0) return MFLAB_OK;
     if (mfl::views_overlap(C, ldc, lsc, m, n, limbs, B, ldb, lsb, k, n)) return MFLAB_ERR_ALIAS;
     cudaStream_t s = (cudaStream_t)stream;
+    mfl::crt_narrow(h, n, p);
     rc = mflab_reserve_scratch(h, p.total - p.a8);
     if (rc) return rc;
     rc = mflab_reserve_aux(h, sizeof(int) * (size_t)(n + 64));
