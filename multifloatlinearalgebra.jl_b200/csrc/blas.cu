@@ -283,6 +283,10 @@ static int run_mm_n(int64_t m, int64_t n, int64_t k, Mat A, Mat B, Mat C, const 
             return run_mm<N, 16, 8, 16, 1, 1, (N == 2 ? 8 : N == 3 ? 4 : 2), TA, TB, TRI, FUSED, TRMM>(
                 m, n, k, A, B, C, alpha, beta, s, info, mode);
         if constexpr (N == 2) {
+            // one 32 x 16 tile per SM: sixteen warps of one output each hide the
+            // chains better than eight of two (256 cubed: 43.5 us, 47.8)
+            if (tile == MM_MID && !TRI && (m + 31) / 32 * ((n + 15) / 16) <= MM_SMS)
+                return run_mm<2, 32, 16, 32, 1, 1, 8, TA, TB, TRI, FUSED, TRMM>(m, n, k, A, B, C, alpha, beta, s, info, mode);
             if (tile == MM_MID)
                 return run_mm<2, 32, 16, 16, 2, 1, 4, TA, TB, TRI, FUSED, TRMM>(m, n, k, A, B, C, alpha, beta, s, info, mode);
             return run_mm<2, 64, 64, 16, 4, 4, 2, TA, TB, TRI, FUSED, TRMM>(m, n, k, A, B, C, alpha, beta, s, info, mode);
@@ -300,16 +304,21 @@ static int run_mm_n(int64_t m, int64_t n, int64_t k, Mat A, Mat B, Mat C, const 
 // chain acc = acc + a(i,k) x(k), so a launch cannot end before K dependent
 // additions have (about 90 cycles each in x2, 220 in x3, 350 in x4).  A CTA
 // owns 32 rows: one warp runs their chains and does nothing else, six warps on
-// the other three schedulers load A and form the products of the next 32
+// the other three schedulers load A and form the products of the next slab of
 // columns into shared memory (two slabs, one CTA barrier per slab).  The
 // second warp on the chain's own scheduler stays idle, and the chain warp's
 // place rotates over the schedulers with the CTA so that CTAs that share an
-// SM do not share a scheduler.  TA as in mm_kernel; a 32 x 32 block of a
-// symmetric matrix lies on one side of the diagonal or on it.  2500 x 3100 in
-// x2: 168 us, 103 cycles a term (590 us on mm_kernel's 32 x 16 tile, of whose
+// SM do not share a scheduler.  TA as in mm_kernel.  2500 x 3100 in
+// x2: 154 us, 96 cycles a term (590 us on mm_kernel's 32 x 16 tile, of whose
 // sixteen columns one was used; 298 us on 32 x 1 tiles that load and multiply
-// in the chain's own warp).
-constexpr int MV_ROWS = 32, MV_KB = 32, MV_NT = 256, MV_HELPERS = 6;
+// in the chain's own warp; 167 us with slabs of 32 columns).
+constexpr int MV_ROWS = 32, MV_NT = 256, MV_HELPERS = 6;
+
+// columns per slab: a slab costs the chain a barrier and a loop end
+template <int N>
+struct MVSlab {
+    static constexpr int value = N == 2 ? 64 : 32;
+};
 
 template <int N>
 struct MVStride {  // odd: the columns of one row fall on all banks
@@ -328,7 +337,7 @@ __global__ void __launch_bounds__(MV_NT)
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (info && *info != 0 && *info <= last) return;
     extern __shared__ double prod[];  // [2][MV_KB][ST]
-    constexpr int ST = MVStride<N>::value;
+    constexpr int ST = MVStride<N>::value, MV_KB = MVSlab<N>::value;
     const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
     const int chain = (int)((blockIdx.x + blockIdx.x / MM_SMS) % 4);
     const int side = (warp - chain) & 3;                        // scheduler beside the chain's
@@ -340,9 +349,10 @@ __global__ void __launch_bounds__(MV_NT)
     auto produce = [&](int64_t s) {
         double *out = prod + (s & 1) * MV_KB * ST;
         const int64_t k0 = s * MV_KB;
-        // is the block read down its rows (A[i,k]) or across (A[k,i])?  On the
-        // diagonal block of a symmetric matrix every entry decides for itself.
-        const bool across = TA == 1 || (TA == 2 && k0 > row0) || (TA == 3 && k0 < row0);
+        // is the slab read down its rows (A[i,k]) or across (A[k,i])?  A slab on
+        // the diagonal of a symmetric matrix decides entry by entry.
+        const bool across = TA == 1 || (TA == 2 && k0 > row0 + MV_ROWS - 1) ||
+                            (TA == 3 && k0 + MV_KB - 1 < row0);
         mf<N> a[PER];
         if (!across) {
             const int64_t row = row0 + lane;
@@ -365,22 +375,26 @@ __global__ void __launch_bounds__(MV_NT)
                 for (int l = 0; l < N; ++l) out[kk * ST + l * MV_ROWS + lane] = p.v[l];
             }
         } else {
-            const int64_t k = k0 + lane;
-            const bool kin = k < K;
 #pragma unroll
-            for (int q = 0; q < PER; ++q) {
-                const int64_t row = row0 + helper + MV_HELPERS * q;
-                const bool ok = kin && helper + MV_HELPERS * q < MV_ROWS && row < m;
-                a[q] = ok ? load_mf<N>(A.p, A.ld, A.ls, k, row) : from_double<N>(0.0);
-            }
-            const mf<N> x = kin ? load_mf<N>(X.p, 0, X.ls, k, 0) : from_double<N>(0.0);
+            for (int half = 0; half < MV_KB; half += 32) {
+                const int64_t k = k0 + half + lane;
+                const bool kin = k < K;
+                constexpr int RPER = (MV_ROWS + MV_HELPERS - 1) / MV_HELPERS;
 #pragma unroll
-            for (int q = 0; q < PER; ++q) {
-                const int i = helper + MV_HELPERS * q;
-                if (i >= MV_ROWS) break;
-                const mf<N> p = mul(a[q], x);
+                for (int q = 0; q < RPER; ++q) {
+                    const int64_t row = row0 + helper + MV_HELPERS * q;
+                    const bool ok = kin && helper + MV_HELPERS * q < MV_ROWS && row < m;
+                    a[q] = ok ? load_mf<N>(A.p, A.ld, A.ls, k, row) : from_double<N>(0.0);
+                }
+                const mf<N> x = kin ? load_mf<N>(X.p, 0, X.ls, k, 0) : from_double<N>(0.0);
 #pragma unroll
-                for (int l = 0; l < N; ++l) out[lane * ST + l * MV_ROWS + i] = p.v[l];
+                for (int q = 0; q < RPER; ++q) {
+                    const int i = helper + MV_HELPERS * q;
+                    if (i >= MV_ROWS) break;
+                    const mf<N> p = mul(a[q], x);
+#pragma unroll
+                    for (int l = 0; l < N; ++l) out[(half + lane) * ST + l * MV_ROWS + i] = p.v[l];
+                }
             }
         }
     };
@@ -399,7 +413,7 @@ __global__ void __launch_bounds__(MV_NT)
             };
             const int64_t left = K - s * MV_KB;
             if (left >= MV_KB) {
-#pragma unroll 8
+#pragma unroll (N == 2 ? 32 : 8)
                 for (int kk = 0; kk < MV_KB; ++kk) term(kk);
             } else {
                 for (int kk = 0; kk < (int)left; ++kk) term(kk);
@@ -422,7 +436,7 @@ __global__ void __launch_bounds__(MV_NT)
 template <int N, int TA>
 static int run_mv(int64_t m, int64_t k, Mat A, Mat X, Mat Y, const double *alpha,
                   const double *beta, cudaStream_t s, const int *info) {
-    constexpr size_t smem = sizeof(double) * 2 * MV_KB * MVStride<N>::value;
+    constexpr size_t smem = sizeof(double) * 2 * MVSlab<N>::value * MVStride<N>::value;
     auto kern = mv_kernel<N, TA, false>;
     static std::atomic<unsigned long long> configured{0};
     if (int rc = set_smem_once((const void *)kern, (int)smem, configured, "mv_kernel attribute"))
@@ -443,7 +457,7 @@ static int run_mv(int64_t m, int64_t k, Mat A, Mat X, Mat Y, const double *alpha
 template <int N>
 static int run_column_chains(int64_t cols, int64_t k, Mat A, Mat X, Mat Y, cudaStream_t s,
                              const int *stop, int last) {
-    constexpr size_t smem = sizeof(double) * 2 * MV_KB * MVStride<N>::value;
+    constexpr size_t smem = sizeof(double) * 2 * MVSlab<N>::value * MVStride<N>::value;
     auto kern = mv_kernel<N, 1, true>;
     static std::atomic<unsigned long long> configured{0};
     if (int rc = set_smem_once((const void *)kern, (int)smem, configured, "column chains attribute"))

@@ -253,9 +253,9 @@ int mstep_launch(cudaStream_t s, int64_t nrhs, int64_t j0, int jb, const double 
 // step costs one store and one load through L2 instead of a fence, a flag and
 // then the load.  The rows are written LS_COPIES times: copy 0 is for the
 // owners of the block itself and of the next one, the only CTAs the chain of
-// steps waits for, and the others' polls are spread over the rest.  The slices do not depend on the solve: two are prefetched
-// into shared memory ahead of the rows.  Arithmetic and results are the block
-// kernel's.  All CTAs are co-resident (cooperative launch); a wait that runs
+// steps waits for, and the others' polls are spread over the rest.  The slices
+// do not depend on the solve: two are prefetched into shared memory ahead of
+// the rows.  Arithmetic and results are the block kernel's.  All CTAs are co-resident (cooperative launch); a wait that runs
 // out (LS_SPIN polls) records error 6 and the CTA leaves at its next barrier,
 // the others as their waits run out or see the abort word.  n = 4096, 16
 // right-hand sides: 220 us (460 us as 64 launches, 348 us with flags, 286 us
