@@ -345,16 +345,29 @@ __global__ void __launch_bounds__(128)
     const int e = j < n ? colexp[j] : OZ_EXP_EMPTY;
     const int sh = oz_scale_exp(e);
     mf<N> z[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-        const int64_t kk = kg + u;
-        const bool ok = kk < k && j < n && e != OZ_EXP_BAD;
+    const bool used = j < n && e != OZ_EXP_BAD;
+    const double *src = B.p + j * B.ld + kg;
+    if (used && kg + U <= k && ((uintptr_t)src & 15) == 0 && (B.ls & 1) == 0) {
+        // a thread's U values of a limb are consecutive: 16-byte loads
 #pragma unroll
         for (int l = 0; l < N; ++l)
-            z[u].v[l] = ok ? scale2(B.p[l * B.ls + j * B.ld + kk], -sh) : 0.0;
+#pragma unroll
+            for (int u = 0; u < U; u += 2) {
+                const double2 v = *(const double2 *)(src + l * B.ls + u);
+                z[u].v[l] = scale2(v.x, -sh);
+                z[u + 1].v[l] = scale2(v.y, -sh);
+            }
+    } else {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int l = 0; l < N; ++l)
+                z[u].v[l] = used && kg + u < k ? scale2(src[l * B.ls + u], -sh) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
 #pragma unroll
         for (int l = N - 1; l > 0; --l) two_sum(z[u].v[l - 1], z[u].v[l], z[u].v[l - 1], z[u].v[l]);
-    }
     int8_t *dst = B8 + (size_t)j * Q * kp + kg;
     if (!MFLAB_IDX_OK(kg + U <= kp && j < np, 3, j, kg)) return;
     for (int q = 0; q < Q; ++q) {
