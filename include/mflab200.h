@@ -525,7 +525,9 @@ int mflab_spd_batched_adjoint(mflab_handle *h, void *stream, int limbs, int64_t 
    threads = 64, 128, 256 or 512 (the plain entries use 256).  Neither the CTA
    size nor the number of persistent CTAs (grid) changes any result: every
    block's arithmetic is per element in the reference order; they are the
-   knobs of the batched autotuner.  No reference counterpart. */
+   knobs of the batched autotuner.  They shape the factor's launch; the
+   substitutions and the adjoint size their launches by the number of blocks and
+   only check these arguments.  No reference counterpart. */
 int mflab_spd_batched_ex(mflab_handle *h, void *stream, int limbs, int64_t nblocks,
                          int64_t max_size, const int64_t *sizes, const int64_t *offsets,
                          const int64_t *boffsets, const int64_t *order, double *S, int64_t ls_s,

@@ -2,9 +2,8 @@
 
 No reference counterpart: MultiFloatLinearAlgebra.jl factors one matrix per
 call.  Every block here follows cholesky!(S_i) / ldiv!(x_i, F_i) of the
-reference exactly (one persistent CTA per block for the factor, a small CTA
-per block for the forward and a lane per block for the backward substitution),
-so per block the results equal the single-matrix routines.
+reference exactly (one persistent CTA per block for the factor, 16 or 32 lanes
+per block for the forward and one for the backward substitution), so per block the results equal the single-matrix routines.
 
     batch = SPDBatch(N, sizes)              # packed device storage
     batch.set_block(i, S_i); batch.set_rhs(i, b_i)
@@ -12,8 +11,9 @@ so per block the results equal the single-matrix routines.
     Sbar, bbar = pullback(xbar)             # ChainRulesCore-style pullback
 
 `BatchedSPDGraph` captures the whole solve (counter reset, the persistent
-factor kernel, the two substitution kernels) in a CUDA graph and replays it.  `autotune` picks the launch shape (CTA size, number of
-persistent CTAs) by timing the batch itself.
+factor kernel, the two substitution kernels) in a CUDA graph and replays it.
+`autotune` picks the factor's launch shape (CTA size, number of persistent
+CTAs) by timing the batch itself.
 """
 from __future__ import annotations
 
