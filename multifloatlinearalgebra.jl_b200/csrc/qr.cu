@@ -222,31 +222,26 @@ __global__ void qr_finite_kernel(int64_t m, int64_t n, Mat A, int *flag) {
 constexpr int QRR_TILE = 256, QRR_NT = QRR_TILE + 32;
 enum : unsigned char { QRR_SKIP = 0, QRR_ADD = 1, QRR_RAISE = 2, QRR_FIRST = 3 };
 
+// scale and sum of squares of rows r0..m-1 of column c by a CTA of QRR_NT
+// threads; the first thread of the last warp has the result
 template <int N>
-__global__ void __launch_bounds__(QRR_NT)
-    qr_reflector_kernel(int64_t m, int64_t s, Mat A, double *tau, int64_t lt, int blocked,
-                        double *diag, const int *stop) {
-    // every step's kernels are programmatic dependents of one another: wait
-    // for the previous grid, let the next one be placed
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    if (stop && *stop != 0 && *stop <= (int)s) return;
+__device__ __forceinline__ void cta_norm(const Mat &A, int64_t m, int64_t r0, int64_t c,
+                                         mf<N> &scale, mf<N> &sum) {
     __shared__ double val[2][N][QRR_TILE];  // squares (QRR_ADD) or ratios (QRR_RAISE)
     __shared__ unsigned char flag[2][QRR_TILE];
     __shared__ unsigned plain[2][QRR_TILE / 32];  // rows of a group that only add
-    __shared__ double wmax[QRR_TILE / 32][N], carry[2][N], slead[N];
-    __shared__ int go;
+    __shared__ double wmax[QRR_TILE / 32][N], carry[2][N];
     const unsigned FULL = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const mf<N> one = from_double<N>(1.0), zero = from_double<N>(0.0);
-    const int64_t tiles = (m - s + QRR_TILE - 1) / QRR_TILE;
+    const int64_t tiles = (m - r0 + QRR_TILE - 1) / QRR_TILE;
     if (tid < N) carry[0][tid] = 0.0;
     __syncthreads();
 
     auto produce = [&](int64_t t) {  // warps 0 .. 7
         const int b = (int)(t & 1);
-        const int64_t r = s + t * QRR_TILE + tid;
-        const mf<N> mag = r < m ? abs_mf(load_mf<N>(A.p, A.ld, A.ls, r, s)) : zero;
+        const int64_t r = r0 + t * QRR_TILE + tid;
+        const mf<N> mag = r < m ? abs_mf(load_mf<N>(A.p, A.ld, A.ls, r, c)) : zero;
         const bool nz = !iszero(mag);
         mf<N> pm = mag;  // running maximum within the warp
 #pragma unroll
@@ -299,7 +294,7 @@ __global__ void __launch_bounds__(QRR_NT)
         }
     };
 
-    mf<N> sum = one;
+    sum = one;
     if (warp < QRR_TILE / 32) produce(0);
     for (int64_t t = 0; t < tiles; ++t) {
         __syncthreads();
@@ -333,10 +328,26 @@ __global__ void __launch_bounds__(QRR_NT)
         }
     }
     __syncthreads();
-    if (tid == QRR_TILE) {
-        mf<N> scale;
 #pragma unroll
-        for (int l = 0; l < N; ++l) scale.v[l] = carry[tiles & 1][l];
+    for (int l = 0; l < N; ++l) scale.v[l] = carry[tiles & 1][l];
+}
+
+template <int N>
+__global__ void __launch_bounds__(QRR_NT)
+    qr_reflector_kernel(int64_t m, int64_t s, Mat A, double *tau, int64_t lt, int blocked,
+                        double *diag, const int *stop) {
+    // every step's kernels are programmatic dependents of one another: wait
+    // for the previous grid, let the next one be placed
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (stop && *stop != 0 && *stop <= (int)s) return;
+    __shared__ double slead[N];
+    __shared__ int go;
+    const mf<N> one = from_double<N>(1.0), zero = from_double<N>(0.0);
+    const int tid = threadIdx.x;
+    mf<N> scale, sum;
+    cta_norm<N>(A, m, s, s, scale, sum);
+    if (tid == QRR_TILE) {
         const mf<N> nrm = norm_value(scale, sum);
         mf<N> t = zero;
         go = 0;
@@ -548,13 +559,32 @@ __global__ void __launch_bounds__(QRR_NT)
     }
 }
 
-// norm state of columns c0..n-1 from rows r0 (qr.jl:143-155, 417-448), one
-// warp per column
-constexpr int QR_NORM_WARPS = 4;
+// norm state of columns c0..n-1 from rows r0 (qr.jl:143-155, 417-448): a CTA per
+// column from QR_NORM_ROWS rows on, where the column's own chain bounds it, else
+// a warp per column.  Many columns fill the FP64 pipe with either, and the
+// warp's divisions, 32 at a time, then cost less: the line lies at two columns
+// per SM in x2, one in x3 and x4.  us, CTA / warp:
+//   x2  32 x 40 15 / 7, 128 x 40 18 / 21, 500 x 40 34 / 79, 500 x 296 43 / 80,
+//       500 x 592 79 / 81, 500 x 1200 124 / 94;
+//   x4  128 x 40 40 / 51, 500 x 148 109 / 189, 500 x 296 217 / 194.
+// rrqr 500 x 40 in x2 3.42 -> 3.30 ms, 2000 x 40 10.35 -> 9.82 ms.
+constexpr int QR_NORM_WARPS = 4, QR_NORM_ROWS = 128;
+
+template <int N>
+__global__ void __launch_bounds__(QRR_NT)
+    qr_norm_init_kernel(int64_t m, int64_t r0, int64_t c0, Mat A, QRNorms<N> S) {
+    const int64_t c = c0 + blockIdx.x;
+    mf<N> scale, sum;
+    cta_norm<N>(A, m, r0, c, scale, sum);
+    if (threadIdx.x == QRR_TILE) {
+        S.set(c, scale, sum);
+        S.dirty[c] = 0;
+    }
+}
 
 template <int N>
 __global__ void __launch_bounds__(32 * QR_NORM_WARPS)
-    qr_norm_init_kernel(int64_t m, int64_t r0, int64_t c0, Mat A, QRNorms<N> S) {
+    qr_norm_init_warp_kernel(int64_t m, int64_t r0, int64_t c0, Mat A, QRNorms<N> S) {
     __shared__ double nbuf[QR_NORM_WARPS][QR_NORM_BUF(N)];
     const int w = threadIdx.x >> 5;
     const int64_t c = c0 + (int64_t)blockIdx.x * QR_NORM_WARPS + w;
@@ -567,8 +597,15 @@ __global__ void __launch_bounds__(32 * QR_NORM_WARPS)
     }
 }
 
-static inline unsigned norm_grid(int64_t cols) {
-    return (unsigned)((cols + QR_NORM_WARPS - 1) / QR_NORM_WARPS);
+template <int N>
+static void launch_norm_init(int64_t m, int64_t r0, int64_t c0, const Mat &A, const QRNorms<N> &S,
+                             cudaStream_t s) {
+    const int64_t cols = S.n - c0;
+    if (m - r0 >= QR_NORM_ROWS && cols <= (N == 2 ? 2 * 148 : 148))
+        qr_norm_init_kernel<N><<<(unsigned)cols, QRR_NT, 0, s>>>(m, r0, c0, A, S);
+    else
+        qr_norm_init_warp_kernel<N><<<(unsigned)((cols + QR_NORM_WARPS - 1) / QR_NORM_WARPS),
+                                      32 * QR_NORM_WARPS, 0, s>>>(m, r0, c0, A, S);
 }
 
 // _qr_update_norm_state! for one column (qr.jl:264-304)
@@ -934,7 +971,7 @@ static int qr_n(mflab_handle *h, cudaStream_t s, int pivoted, int64_t m, int64_t
         }
         fl.v[0] = ldexp(1.0, 4 - 52 * N);
         if (n > 0)
-            qr_norm_init_kernel<N><<<norm_grid(n), 32 * QR_NORM_WARPS, 0, s>>>(m, 0, 0, A, S);
+            launch_norm_init<N>(m, 0, 0, A, S, s);
         const bool blocked = r >= QR_BLOCK && m * n >= 16384;
         if (!blocked) {
             for (int64_t st = 0; st < r; ++st) {
@@ -1008,7 +1045,7 @@ static int qr_n(mflab_handle *h, cudaStream_t s, int pivoted, int64_t m, int64_t
                     if (rc) break;
                 }
                 if (be < n)
-                    qr_norm_init_kernel<N><<<norm_grid(n - be), 32 * QR_NORM_WARPS, 0, s>>>(m, be, be, A, S);
+                    launch_norm_init<N>(m, be, be, A, S, s);
                 bs = be;
             }
             if (rc) return rc;

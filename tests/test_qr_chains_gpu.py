@@ -42,3 +42,15 @@ def test_apply_q_column_counts(mf, ref, rng, N, nd):
     Dd = mf.MFMatrix.from_numpy(D)
     mf.apply_q_(Dd, F, trans="T")
     assert_bitwise(Dd.to_numpy(), ref.apply_q(F.factors.to_numpy(), F.tau.cpu().numpy(), D, "T"))
+
+
+@pytest.mark.parametrize("N,m,n", [(2, 128, 296), (2, 129, 297), (2, 127, 20), (3, 130, 148),
+                                   (4, 128, 148), (4, 130, 149)])
+def test_initial_norms_at_the_rule(mf, ref, rng, N, m, n):
+    """a CTA or a warp per column for the first norms of a pivoted QR"""
+    A = _panel(rng, N, m, n)
+    F = mf.rrqr_(mf.MFMatrix.from_numpy(A))
+    want, wtau, wperm, _ = ref.rrqr(A)
+    assert np.array_equal(mf.factor_permutation(F), wperm)
+    assert_bitwise(F.tau.cpu().numpy(), wtau, "tau")
+    assert_bitwise(F.factors.to_numpy(), want, "factors")
