@@ -31,6 +31,9 @@ __device__ __forceinline__ void ld_remote_f64(uint32_t a, double v) {
 __device__ __forceinline__ void ld_remote_s32(uint32_t a, int v) {
     asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
+__device__ __forceinline__ void ld_remote_max(uint32_t a, int v) {
+    asm volatile("red.relaxed.cluster.shared::cluster.max.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
 
 template <int N>
 __device__ __forceinline__ mf<N> ld_get(const double *p) {
@@ -46,7 +49,9 @@ __device__ __forceinline__ void ld_put(double *p, const mf<N> &v) {
 }
 
 // larger of two candidates: the first strictly larger value in ascending index
-// order; index -1 holds no candidate
+// order; index -1 holds no candidate.  The indices of a reduction's candidates
+// are distinct: only then do both sides of an exchange pick the same one where
+// neither value is the larger.
 template <int N>
 __device__ __forceinline__ void ld_better(mf<N> &v, int &i, const mf<N> &o, int oi) {
     bool take = oi >= 0;

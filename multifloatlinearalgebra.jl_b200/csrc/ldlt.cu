@@ -107,6 +107,7 @@ struct LdShared {
     int regular;                  // 0 singular, 1 |a| >= |b|, 2 |a| < |b|
     unsigned char type[LD_PANEL];
     int flag;
+    int nan_at;                   // last NaN of the row scan, -1 without one
 };
 
 // coefficients D * A[col, pf + i], i < cnt, of one column's lazy entries
@@ -341,6 +342,7 @@ __global__ void __launch_bounds__(LD_NT)
     };
     while (k <= pl) {
         const int cnt = LAZY ? (int)(k - pf) : 0;
+        if (t == 0) sh.nan_at = -1;
         if (LAZY) {
             ld_stage_coef<N>(F, sh, sh.coef[0], k, pf, cnt);
             __syncthreads();
@@ -361,7 +363,9 @@ __global__ void __launch_bounds__(LD_NT)
                         held = e;
                         held_row = r;
                     }
-                    ld_better(best, bi, abs_mf(e), (int)r);
+                    // a NaN is never strictly larger; in the first row nothing
+                    // is strictly larger than it
+                    if (r == k + 1 || !isnan(e.v[0])) ld_better(best, bi, abs_mf(e), (int)r);
                 }
             }
             if (t == LD_NT - 1) ld_put<N>(sh.val[0], entry(0, k, k));
@@ -379,20 +383,37 @@ __global__ void __launch_bounds__(LD_NT)
                     for (int i = t; i < cnt; i += LD_NT) ld_put<N>(sh.rowi[i], F.at(imax, pf + i));
                     __syncthreads();
                 }
-                // max |entry| along row imax of the active matrix
-                mf<N> rowmax = zero;
-                for (int64_t c = mine; c < n; c += total) {
-                    if (c < k || c == imax) continue;
-                    mf<N> e;
-                    if (c > imax) e = entry(1, c, imax);
-                    else if constexpr (LAZY) e = ld_row_entry<N>(F, sh, imax, c, pf, cnt);
-                    else e = F.at(imax, c);
-                    rowmax = max_mf(rowmax, abs_mf(e));
+                // max |entry| along row imax of the active matrix.  max(x, y)
+                // is y where x is NaN (an elimination that overflowed), so the
+                // fold of ldlt.jl:203-209 is the maximum of what follows the
+                // last NaN: a second scan takes that.  The candidates carry
+                // their positions: every pair then has one winner, whatever
+                // the values, and all threads of the cluster agree on the
+                // branches below.
+                mf<N> rowmax;
+                for (int from = -1;;) {
+                    rowmax = zero;
+                    int ri = -1, nan_at = -1;
+                    for (int64_t c = mine; c < n; c += total) {
+                        if (c < k || c == imax || c <= from) continue;
+                        mf<N> e;
+                        if (c > imax) e = entry(1, c, imax);
+                        else if constexpr (LAZY) e = ld_row_entry<N>(F, sh, imax, c, pf, cnt);
+                        else e = F.at(imax, c);
+                        if (isnan(e.v[0])) nan_at = (int)c;
+                        else ld_better(rowmax, ri, abs_mf(e), (int)c);
+                    }
+                    if (t == LD_NT - 1) ld_put<N>(sh.val[1], entry(1, imax, imax));
+                    if (nan_at >= 0)
+                        for (int q = 0; q < nc; ++q)
+                            ld_remote_max(ld_remote(&sh.nan_at, (uint32_t)q), nan_at);
+                    __syncwarp();
+                    ld_reduce<N>(sh, 1, rank, nc, rowmax, ri);
+                    if (ri < 0) rowmax = from_double<N>(nan(""));  // nothing follows the NaN
+                    if (sh.nan_at == from) break;
+                    from = sh.nan_at;
+                    ld_cluster_sync();  // the readers of the candidates and of nan_at are done
                 }
-                if (t == LD_NT - 1) ld_put<N>(sh.val[1], entry(1, imax, imax));
-                __syncwarp();
-                int ri = 0;
-                ld_reduce<N>(sh, 1, rank, nc, rowmax, ri);
                 if (!ge(absakk, mul(mul(alpha, best), div_call(best, rowmax)))) {
                     piv = imax;
                     bs = ge(abs_mf(ld_get<N>(sh.val[1])), mul(alpha, rowmax)) ? 1 : 2;
