@@ -38,6 +38,14 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(n) : "memory");
 }
 
+// column tiles in a grid's y dimension; wider products take layers in z, up to
+// as many columns as a grid of the widest tiles (64 columns, 32 in x4) holds
+constexpr int64_t MM_GRID_Y = 65535;
+template <int N>
+struct MMColumns {
+    static constexpr int64_t most = MM_GRID_Y * (N == 4 ? 32 : 64);
+};
+
 template <int N, int BM, int BN, int BK, int TM, int TN>
 struct MMShape {
     static constexpr int TX = BM / TM;
@@ -71,7 +79,9 @@ __global__ void __launch_bounds__(MMShape<N, BM, BN, BK, TM, TN>::NT)
     double *Bs = smem + 2 * N * BK * BM;  // [2][N][BK][BN]
     const int tid = threadIdx.x;
     const int tx = tid % TX, ty = tid / TX;
-    const int64_t row0 = (int64_t)blockIdx.x * BM, col0 = (int64_t)blockIdx.y * BN;
+    const int64_t row0 = (int64_t)blockIdx.x * BM;
+    const int64_t col0 = ((int64_t)blockIdx.z * MM_GRID_Y + blockIdx.y) * BN;
+    if (col0 >= n) return;  // the last of several layers of column tiles
     if (TRI && row0 + BM - 1 < col0) return;  // tile strictly above the diagonal
     // debug builds: C's column stride holds its rows
     if (!(mode & MM_PACKED) && !MFLAB_IDX_OK(C.ld >= m, 6, C.ld, m)) return;
@@ -226,8 +236,10 @@ static int run_mm(int64_t m, int64_t n, int64_t k, Mat A, Mat B, Mat C, const do
         if (beta[l] != 0.0) overwrite = 0;
     }
     if (m <= 0 || n <= 0) return MFLAB_OK;
-    dim3 grid((unsigned)((m + BM - 1) / BM), (unsigned)((n + BN - 1) / BN));
-    if (grid.y > 65535) return MFLAB_ERR_UNSUPPORTED;
+    if (n > MMColumns<N>::most) return MFLAB_ERR_UNSUPPORTED;
+    const int64_t tiles = (n + BN - 1) / BN;
+    const dim3 grid((unsigned)((m + BM - 1) / BM), (unsigned)std::min(tiles, MM_GRID_Y),
+                    (unsigned)((tiles + MM_GRID_Y - 1) / MM_GRID_Y));
     kern<<<grid, S::NT, S::smem_bytes, s>>>(m, n, k, A, B, C, al, be, overwrite, info, mode);
     return record_cuda_error(cudaGetLastError(), "mm_kernel launch");
 }
