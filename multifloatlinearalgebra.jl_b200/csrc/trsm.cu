@@ -12,10 +12,10 @@
 //     applies its term k.  Each row thus receives its terms in the reference's
 //     ascending order while the rows progress in parallel.
 //   * trsm_left_warp: the same with the rows over the lanes of a warp, for
-//     triangles of at most 64 rows (LU's U12 block).
+//     triangles of at most 64 rows and up to some thousand columns.
 //   * trsm_left_backward_cta: backward substitution, one CTA per column.
 //   * trsm_left_thread: one thread per right-hand-side column, the plain
-//     serial loop (many columns of a backward substitution).
+//     serial loop (many columns).
 //   * trsm_right_thread: one thread per row of B, the plain serial loop (the
 //     Cholesky panel solve A21 <- A21 / L11^T).
 #include "mf_device.cuh"
@@ -106,6 +106,20 @@ __global__ void __launch_bounds__(NT) trsm_left_cta(int64_t m, int64_t n, Mat A,
 // x4, 16 unit rows, 685 columns: about 7 us (77 us with a thread per column
 // whose 120 terms wait for their loads one by one).
 constexpr int TRSW_NT = 128;
+
+// Its line against the thread kernel: a column costs the warp kernel m steps of
+// issue, an unknown's division for 16 or 32 lanes alone, so its time grows with
+// the columns, while the thread kernel's, bound by its chains, is the same up to
+// some 20 000 columns.  They meet in proportion to m, by the lanes and rows per
+// lane.  us, warp / thread: x2, 16 rows 10000 44 / 52, 100000 261 / 170; x2, 64
+// rows 10000 322 / 510, 20000 630 / 717, 100000 2988 / 1889; x3, 32 rows 4000
+// 183 / 255, 8000 334 / 255; x4, 8 rows 2000 45 / 49, 4000 71 / 48; x4, 64 rows
+// 4000 1336 / 1347, 100000 31900 / 4225.
+template <int N>
+static int64_t trsw_columns(int64_t m) {
+    constexpr int per_row[3][3] = {{640, 270, 200}, {300, 145, 125}, {200, 90, 60}};
+    return m * per_row[N - 2][m <= 16 ? 0 : m <= 32 ? 1 : 2];
+}
 
 template <int N, int W, int RPL>
 __global__ void __launch_bounds__(TRSW_NT)
@@ -410,7 +424,8 @@ static int run_trsm(int side, int uplo, int trans, int diag, int64_t m, int64_t 
     if (N == 1 && !transposed && m > 2 * TRSM64_NB && n <= 65535 && !info)
         return trsm64_blocked(m, n, A, B, eff_lower, unit, s, info);
     if constexpr (N >= 2) {
-        if (eff_lower && m <= 64) return run_trsm_left_warp<N>(m, n, A, B, transposed, unit, s, info);
+        if (eff_lower && m <= 64 && n <= trsw_columns<N>(m))
+            return run_trsm_left_warp<N>(m, n, A, B, transposed, unit, s, info);
         // one CTA per column; short triangles of many columns go to the
         // thread kernel, whose 32 chains share a warp
         if (!wavefront_ok && n < (m <= 64 ? (N == 4 ? 2 : 4) * TRSB_SMS : 4096)) {

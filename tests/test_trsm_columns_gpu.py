@@ -1,0 +1,25 @@
+"""Left triangular solves of many columns, on both sides of the lines between
+their kernels, bit for bit against the oracle."""
+import pytest
+
+from conftest import assert_bitwise
+from test_blas_gpu import _tri
+from test_oracle import syn
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(mf, ref, rng, N, m, n, uplo, trans):
+    T = _tri(rng, N, m, uplo == "lower")
+    B = syn.randn_mf(rng, N, m, n)
+    Bd = mf.MFMatrix.from_numpy(B)
+    mf.trsm_(Bd, mf.MFMatrix.from_numpy(T), 1.0, "left", uplo, trans)
+    assert_bitwise(Bd.to_numpy(), ref.trsm(B, T, 1.0, "left", uplo, trans), "trsm")
+
+
+@pytest.mark.parametrize("uplo,trans", [("lower", "N"), ("upper", "T")])
+@pytest.mark.parametrize("N,m,line", [(2, 4, 2560), (3, 17, 2465), (4, 16, 3200), (4, 33, 1980)],
+                         ids=str)
+@pytest.mark.parametrize("past", [0, 1])
+def test_forward_short_triangle(mf, ref, rng, N, m, line, uplo, trans, past):
+    _check(mf, ref, rng, N, m, line + past, uplo, trans)
