@@ -23,6 +23,8 @@
 
 namespace mfl {
 
+constexpr int TRSM_SMS = 148;
+
 template <int N>
 __device__ __forceinline__ mf<N> tri_coef(const Mat &A, int64_t r, int64_t c, bool transposed) {
     return transposed ? load_mf<N>(A.p, A.ld, A.ls, c, r) : load_mf<N>(A.p, A.ld, A.ls, r, c);
@@ -38,11 +40,12 @@ __global__ void scale_kernel(int64_t m, int64_t n, Mat B, scal<N> alpha) {
 }
 
 // one CTA per column; NT threads; each thread owns up to MAXR rows.  A step is
-// a division, a CTA barrier and the rows' multiply-subtracts; the coefficients
-// of the next step (the diagonal among them, for the row it finalises) are
-// loaded behind the ones just used.  x2, n = 2048, 64 columns: 4200 us
-// (4711 us with the loads inside the step).
-template <int N, int NT, int MAXR>
+// a division, a CTA barrier and the rows' multiply-subtracts.  AHEAD loads the
+// coefficients of the next step (the diagonal among them, for the row it
+// finalises) behind the ones just used, which shortens the step and costs the
+// registers of a CTA per SM.  x2, n = 2048, 64 columns: 4200 us (4711 us with
+// the loads inside the step).
+template <int N, int NT, int MAXR, bool AHEAD>
 __global__ void __launch_bounds__(NT) trsm_left_cta(int64_t m, int64_t n, Mat A, Mat B,
                                                     bool eff_lower, bool transposed, bool unit,
                                                     const int *info) {
@@ -51,18 +54,20 @@ __global__ void __launch_bounds__(NT) trsm_left_cta(int64_t m, int64_t n, Mat A,
     const int64_t col = blockIdx.x;
     if (col >= n) return;
     const int t = threadIdx.x;
-    mf<N> v[MAXR], coef[MAXR];
+    mf<N> v[MAXR], coef[AHEAD ? MAXR : 1];
     auto fetch = [&](int q, int64_t k) {
-        const int64_t r = t + (int64_t)q * NT;
-        if (r < m && (eff_lower ? r >= k && k < m : r <= k && k >= 0) && !(unit && r == k))
-            coef[q] = tri_coef<N>(A, r, k, transposed);
+        if constexpr (AHEAD) {
+            const int64_t r = t + (int64_t)q * NT;
+            if (r < m && (eff_lower ? r >= k && k < m : r <= k && k >= 0) && !(unit && r == k))
+                coef[q] = tri_coef<N>(A, r, k, transposed);
+        }
     };
     const int64_t k0 = eff_lower ? 0 : m - 1;
 #pragma unroll
     for (int q = 0; q < MAXR; ++q) {
         int64_t r = t + (int64_t)q * NT;
         v[q] = r < m ? load_mf<N>(B.p, B.ld, B.ls, r, col) : from_double<N>(0.0);
-        coef[q] = from_double<N>(1.0);
+        if constexpr (AHEAD) coef[q] = from_double<N>(1.0);
         fetch(q, k0);
     }
     for (int64_t s = 0; s < m; ++s) {
@@ -76,8 +81,10 @@ __global__ void __launch_bounds__(NT) trsm_left_cta(int64_t m, int64_t n, Mat A,
             for (int q = 0; q < MAXR; ++q)
                 if (q == qk) {
                     x = v[q];
-                    d = coef[q];
+                    if constexpr (AHEAD) d = coef[q];
                 }
+            if constexpr (!AHEAD)
+                if (!unit) d = load_mf<N>(A.p, A.ld, A.ls, k, k);
             if (!unit) x = div(x, d);
             store_mf<N>(B.p, B.ld, B.ls, k, col, x);
 #pragma unroll
@@ -92,11 +99,28 @@ __global__ void __launch_bounds__(NT) trsm_left_cta(int64_t m, int64_t n, Mat A,
             const int64_t r = t + (int64_t)q * NT;
             const bool later = eff_lower ? (r > k) : (r < k);
             if (r < m && later) {
-                v[q] = submul(v[q], coef[q], xk);
+                if constexpr (AHEAD) v[q] = submul(v[q], coef[q], xk);
+                else v[q] = submul(v[q], tri_coef<N>(A, r, k, transposed), xk);
                 fetch(q, kn);
             }
         }
     }
+}
+
+// AHEAD is the faster form for as long as it takes no more rounds of CTAs over
+// the chip.  CTAs per SM (AHEAD / not): up to 2048 rows x2 2 / 3, x3 and x4
+// 1 / 2; beyond x2 1 / 2, x3 1 / 1; x4 spills there (35.5 / 28.0 ms at 3000
+// rows).  us, 300 rows: x2 296 columns 371 / 413, 444 columns 685 / 440, 3000
+// columns 3798 / 2962; x4 148 columns 1113 / 1210, 222 columns 1975 / 1217, 3000
+// columns 20554 / 12481.
+template <int N>
+static bool trsm_ahead(int64_t m, int64_t n) {
+    if (N == 1) return true;  // no registers to win
+    const bool tall = m > 256 * 8;
+    if (N == 4 && tall) return false;
+    const int64_t with = TRSM_SMS * (N == 2 && !tall ? 2 : 1);
+    const int64_t without = TRSM_SMS * (N == 2 && !tall ? 3 : N == 3 && tall ? 1 : 2);
+    return (n + with - 1) / with <= (n + without - 1) / without;
 }
 
 // Forward substitution of a triangle of at most 64 rows: W lanes per column, RPL
@@ -204,7 +228,7 @@ static int run_trsm_left_warp(int64_t m, int64_t n, Mat A, Mat B, bool transpose
 // chain warp's place rotates over the schedulers with the CTA.  x2, n = 2048,
 // 64 columns: 101 ms (105.2 ms with the products of a row formed between
 // two barriers before its chain).
-constexpr int TRSB_TILE = 256, TRSB_NT = TRSB_TILE + 32, TRSB_SMS = 148;
+constexpr int TRSB_TILE = 256, TRSB_NT = TRSB_TILE + 32;
 
 template <int N>
 __global__ void __launch_bounds__(TRSB_NT)
@@ -216,7 +240,7 @@ __global__ void __launch_bounds__(TRSB_NT)
     const int64_t col = blockIdx.x;
     if (col >= n) return;
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    const int chain = (int)((blockIdx.x + blockIdx.x / TRSB_SMS) % 4);
+    const int chain = (int)((blockIdx.x + blockIdx.x / TRSM_SMS) % 4);
     const int slot = (warp - (warp > chain ? 1 : 0)) * 32 + lane;  // of a producing thread
     auto slabs = [&](int64_t r) { return (m - 1 - r + TRSB_TILE - 1) / TRSB_TILE; };
     auto produce = [&](int64_t r, int64_t j, int b) {
@@ -428,7 +452,7 @@ static int run_trsm(int side, int uplo, int trans, int diag, int64_t m, int64_t 
             return run_trsm_left_warp<N>(m, n, A, B, transposed, unit, s, info);
         // one CTA per column; short triangles of many columns go to the
         // thread kernel, whose 32 chains share a warp
-        if (!wavefront_ok && n < (m <= 64 ? (N == 4 ? 2 : 4) * TRSB_SMS : 4096)) {
+        if (!wavefront_ok && n < (m <= 64 ? (N == 4 ? 2 : 4) * TRSM_SMS : 4096)) {
             trsm_left_backward_cta<N><<<(unsigned)n, TRSB_NT, 0, s>>>(m, n, A, B, transposed, unit,
                                                                      info);
             return record_cuda_error(cudaGetLastError(), "trsm left backward");
@@ -440,16 +464,15 @@ static int run_trsm(int side, int uplo, int trans, int diag, int64_t m, int64_t 
         return record_cuda_error(cudaGetLastError(), "trsm left thread");
     }
     if (n > 2147483647LL) return MFLAB_ERR_UNSUPPORTED;
-    if (m <= 256 * 8) {
-        trsm_left_cta<N, 256, 8><<<(unsigned)n, 256, 0, s>>>(m, n, A, B, eff_lower, transposed,
-                                                             unit, info);
-    } else if (m <= 256 * 16) {
-        trsm_left_cta<N, 256, 16><<<(unsigned)n, 256, 0, s>>>(m, n, A, B, eff_lower, transposed,
-                                                              unit, info);
-    } else {
+    if (m > 256 * 16) {
         trsm_left_thread<N><<<(unsigned)((n + 127) / 128), 128, 0, s>>>(m, n, A, B, eff_lower,
                                                                         transposed, unit, info);
+        return record_cuda_error(cudaGetLastError(), "trsm left thread");
     }
+    const bool ahead = trsm_ahead<N>(m, n);
+    auto kern = m <= 256 * 8 ? (ahead ? trsm_left_cta<N, 256, 8, true> : trsm_left_cta<N, 256, 8, false>)
+                             : (ahead ? trsm_left_cta<N, 256, 16, true> : trsm_left_cta<N, 256, 16, false>);
+    kern<<<(unsigned)n, 256, 0, s>>>(m, n, A, B, eff_lower, transposed, unit, info);
     return record_cuda_error(cudaGetLastError(), "trsm left cta");
 }
 

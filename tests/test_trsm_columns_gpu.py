@@ -9,12 +9,14 @@ from test_oracle import syn
 pytestmark = pytest.mark.gpu
 
 
-def _check(mf, ref, rng, N, m, n, uplo, trans):
+def _check(mf, ref, rng, N, m, n, uplo, trans, diag="nonunit"):
     T = _tri(rng, N, m, uplo == "lower")
+    if diag == "unit":
+        T *= 2.0 ** -8  # bounded growth
     B = syn.randn_mf(rng, N, m, n)
     Bd = mf.MFMatrix.from_numpy(B)
-    mf.trsm_(Bd, mf.MFMatrix.from_numpy(T), 1.0, "left", uplo, trans)
-    assert_bitwise(Bd.to_numpy(), ref.trsm(B, T, 1.0, "left", uplo, trans), "trsm")
+    mf.trsm_(Bd, mf.MFMatrix.from_numpy(T), 1.0, "left", uplo, trans, diag)
+    assert_bitwise(Bd.to_numpy(), ref.trsm(B, T, 1.0, "left", uplo, trans, diag), "trsm")
 
 
 @pytest.mark.parametrize("uplo,trans", [("lower", "N"), ("upper", "T")])
@@ -23,3 +25,11 @@ def _check(mf, ref, rng, N, m, n, uplo, trans):
 @pytest.mark.parametrize("past", [0, 1])
 def test_forward_short_triangle(mf, ref, rng, N, m, line, uplo, trans, past):
     _check(mf, ref, rng, N, m, line + past, uplo, trans)
+
+
+@pytest.mark.parametrize("uplo,trans,diag", [("lower", "N", "nonunit"), ("upper", "T", "unit")])
+@pytest.mark.parametrize("N,m,n", [(2, 65, 296), (2, 65, 297), (2, 300, 445), (2, 65, 593),
+                                   (3, 70, 148), (3, 70, 149), (4, 66, 148), (4, 257, 149),
+                                   (2, 2049, 149), (4, 2049, 2)], ids=str)
+def test_forward_wavefront(mf, ref, rng, N, m, n, uplo, trans, diag):
+    _check(mf, ref, rng, N, m, n, uplo, trans, diag)
