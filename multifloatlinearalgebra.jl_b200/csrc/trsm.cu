@@ -13,7 +13,8 @@
 //     ascending order while the rows progress in parallel.
 //   * trsm_left_warp: the same with the rows over the lanes of a warp, for
 //     triangles of at most 64 rows and up to some thousand columns.
-//   * trsm_left_backward_cta: backward substitution, one CTA per column.
+//   * trsm_left_backward_cta, trsm_left_backward_rows: backward substitution, one
+//     CTA per column.
 //   * trsm_left_thread: one thread per right-hand-side column, the plain
 //     serial loop (many columns).
 //   * trsm_right_thread: one thread per row of B, the plain serial loop (the
@@ -228,7 +229,7 @@ static int run_trsm_left_warp(int64_t m, int64_t n, Mat A, Mat B, bool transpose
 // chain warp's place rotates over the schedulers with the CTA.  x2, n = 2048,
 // 64 columns: 101 ms (105.2 ms with the products of a row formed between
 // two barriers before its chain).
-constexpr int TRSB_TILE = 256, TRSB_NT = TRSB_TILE + 32;
+constexpr int TRSB_TILE = 256, TRSB_NT = TRSB_TILE + 32, TRSR_NT = 256;
 
 template <int N>
 __global__ void __launch_bounds__(TRSB_NT)
@@ -307,6 +308,48 @@ __global__ void __launch_bounds__(TRSB_NT)
     }
 }
 
+// The same, less of it at once: the products of row r are formed by all threads
+// into shared memory between two barriers, thread 0 runs the chain.  An SM
+// holds more of these CTAs, and their chains then hide one another's barriers.
+template <int N>
+__global__ void __launch_bounds__(TRSR_NT)
+    trsm_left_backward_rows(int64_t m, int64_t n, Mat A, Mat B, bool transposed, bool unit,
+                            const int *info) {
+    if (info && *info) return;
+    extern __shared__ double row_prod[];  // [m][N]
+    const int64_t col = blockIdx.x;
+    if (col >= n) return;
+    const int t = threadIdx.x;
+    auto get = [&](int64_t k) {
+        mf<N> p;
+#pragma unroll
+        for (int l = 0; l < N; ++l) p.v[l] = row_prod[k * N + l];
+        return p;
+    };
+    for (int64_t r = m - 1; r >= 0; --r) {
+        for (int64_t k = r + 1 + t; k < m; k += TRSR_NT) {
+            const mf<N> p = mul(tri_coef<N>(A, r, k, transposed), load_mf<N>(B.p, B.ld, B.ls, k, col));
+#pragma unroll
+            for (int l = 0; l < N; ++l) row_prod[k * N + l] = p.v[l];
+        }
+        __syncthreads();
+        if (t == 0) {
+            // the next term is read from shared memory while the current one
+            // is subtracted
+            mf<N> v = load_mf<N>(B.p, B.ld, B.ls, r, col), next = v;
+            if (r + 1 < m) next = get(r + 1);
+            for (int64_t k = r + 1; k < m; ++k) {
+                const mf<N> p = next;
+                if (k + 1 < m) next = get(k + 1);
+                v = sub(v, p);
+            }
+            if (!unit) v = div(v, load_mf<N>(A.p, A.ld, A.ls, r, r));
+            store_mf<N>(B.p, B.ld, B.ls, r, col, v);
+        }
+        __syncthreads();
+    }
+}
+
 template <int N>
 __global__ void trsm_left_thread(int64_t m, int64_t n, Mat A, Mat B, bool eff_lower,
                                  bool transposed, bool unit, const int *info) {
@@ -330,6 +373,40 @@ __global__ void trsm_left_thread(int64_t m, int64_t n, Mat A, Mat B, bool eff_lo
             store_mf<N>(B.p, B.ld, B.ls, row, c, v);
         }
     }
+}
+
+// Which of the three kernels solves n columns backward.  The slab kernel wins
+// while its CTAs have an SM to themselves (in x2 up to 256 rows two share one),
+// the row kernel after that, and a thread per column where either takes too
+// many rounds: beyond four (x4 three) CTAs per SM for short triangles and for
+// those whose row exceeds the row kernel's buffer, else from 4096 columns on.
+// us, slab / row / thread kernel: x2, 64 rows 148 columns 160 / 182 / 518, 296
+// 172 / 185 / 518, 444 217 / 185 / 518, 800 337 / 342 / 517, 2400 780 / 668 /
+// 519; x2, 300 rows 148 columns 2357 / 2548, 444 3589 / 2580, 4095 20501 / 15911;
+// x4, 300 rows 148 columns 8201 / 8354, 222 13261 / 8398, 4095 106437 / 83817;
+// x4, 8 rows 444 columns 68 / 47 / 46, 592 77 / 71 / 48.
+constexpr size_t TRSR_SMEM = 200 * 1024;
+
+template <int N>
+static int run_trsm_left_backward(int64_t m, int64_t n, Mat A, Mat B, bool transposed, bool unit,
+                                  cudaStream_t s, const int *info) {
+    const size_t smem = (size_t)m * N * sizeof(double);
+    const bool fits = smem <= TRSR_SMEM;
+    const int64_t most = m > 64 && fits ? 4095 : (N == 4 ? 3 : 4) * TRSM_SMS;
+    if (n > most) {
+        trsm_left_thread<N><<<(unsigned)((n + 127) / 128), 128, 0, s>>>(m, n, A, B, false, transposed,
+                                                                        unit, info);
+    } else if (!fits || n <= (N == 2 && m <= 256 ? 2 : 1) * TRSM_SMS) {
+        trsm_left_backward_cta<N><<<(unsigned)n, TRSB_NT, 0, s>>>(m, n, A, B, transposed, unit, info);
+    } else {
+        static std::atomic<unsigned long long> configured{0};
+        if (int rc = set_smem_once((const void *)trsm_left_backward_rows<N>, (int)TRSR_SMEM, configured,
+                                   "trsm backward attribute"))
+            return rc;
+        trsm_left_backward_rows<N><<<(unsigned)n, TRSR_NT, smem, s>>>(m, n, A, B, transposed, unit,
+                                                                    info);
+    }
+    return record_cuda_error(cudaGetLastError(), "trsm left backward");
 }
 
 template <int N>
@@ -450,15 +527,9 @@ static int run_trsm(int side, int uplo, int trans, int diag, int64_t m, int64_t 
     if constexpr (N >= 2) {
         if (eff_lower && m <= 64 && n <= trsw_columns<N>(m))
             return run_trsm_left_warp<N>(m, n, A, B, transposed, unit, s, info);
-        // one CTA per column; short triangles of many columns go to the
-        // thread kernel, whose 32 chains share a warp
-        if (!wavefront_ok && n < (m <= 64 ? (N == 4 ? 2 : 4) * TRSM_SMS : 4096)) {
-            trsm_left_backward_cta<N><<<(unsigned)n, TRSB_NT, 0, s>>>(m, n, A, B, transposed, unit,
-                                                                     info);
-            return record_cuda_error(cudaGetLastError(), "trsm left backward");
-        }
+        if (!wavefront_ok) return run_trsm_left_backward<N>(m, n, A, B, transposed, unit, s, info);
     }
-    if (m <= 64 || n >= 4096 || !wavefront_ok) {
+    if (m <= 64 || n >= 4096) {
         trsm_left_thread<N><<<(unsigned)((n + 127) / 128), 128, 0, s>>>(m, n, A, B, eff_lower,
                                                                         transposed, unit, info);
         return record_cuda_error(cudaGetLastError(), "trsm left thread");

@@ -33,3 +33,11 @@ def test_forward_short_triangle(mf, ref, rng, N, m, line, uplo, trans, past):
                                    (2, 2049, 149), (4, 2049, 2)], ids=str)
 def test_forward_wavefront(mf, ref, rng, N, m, n, uplo, trans, diag):
     _check(mf, ref, rng, N, m, n, uplo, trans, diag)
+
+
+@pytest.mark.parametrize("uplo,trans,diag", [("upper", "N", "nonunit"), ("lower", "T", "unit")])
+@pytest.mark.parametrize("N,m,n", [(2, 65, 296), (2, 65, 297), (2, 257, 149), (2, 5, 592),
+                                   (2, 5, 593), (3, 64, 149), (3, 1, 400), (4, 2, 444), (4, 2, 445),
+                                   (4, 67, 149), (4, 65, 4096)], ids=str)
+def test_backward(mf, ref, rng, N, m, n, uplo, trans, diag):
+    _check(mf, ref, rng, N, m, n, uplo, trans, diag)
