@@ -772,6 +772,16 @@ __global__ void ldlt_pivots_kernel(int64_t n, int64_t nrhs, Mat B, const int64_t
 // (286 us with the swaps in the column itself).
 constexpr int64_t LDLT_GATHER_MAXN = 12000;  // 16 bytes a row of shared memory
 
+// Many short columns pay for a CTA each and take the kernel above, a thread per
+// column.  us of a whole solve, gather / thread: x2, 8 rows 1000 columns 81 / 80,
+// 10000 156 / 118; x2, 30 rows 3000 columns 184 / 183, 10000 306 / 272; x2, 150
+// rows 10000 columns 4885 / 4920, 30000 5701 / 5535; x4, 100 rows 10000 columns
+// 6666 / 6776, 30000 10369 / 10293.  Longer columns: within 1 % at any count.
+static bool ldlt_gathers(int64_t n, int64_t nrhs) {
+    if (n <= 8 || n > LDLT_GATHER_MAXN) return false;
+    return n > 200 || nrhs <= (n <= 32 ? 3000 : 20000);
+}
+
 template <int N>
 __global__ void __launch_bounds__(256)
     ldlt_gather_kernel(int64_t n, Mat B, const int64_t *pivots, const uint8_t *blocks, int reverse) {
@@ -808,7 +818,7 @@ __global__ void __launch_bounds__(256)
 template <int N>
 static int ldlt_interchange(int64_t n, int64_t nrhs, Mat B, const int64_t *pivots,
                             const uint8_t *blocks, int reverse, cudaStream_t s) {
-    if (n <= LDLT_GATHER_MAXN) {
+    if (ldlt_gathers(n, nrhs)) {
         static std::atomic<unsigned long long> configured{0};
         if (int rc = set_smem_once((const void *)ldlt_gather_kernel<N>, (int)(16 * LDLT_GATHER_MAXN),
                                    configured, "sytrs interchange attribute"))
