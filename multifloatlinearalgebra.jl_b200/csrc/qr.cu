@@ -332,7 +332,14 @@ __device__ __forceinline__ void cta_norm(const Mat &A, int64_t m, int64_t r0, in
     for (int l = 0; l < N; ++l) scale.v[l] = carry[tiles & 1][l];
 }
 
-template <int N>
+// Columns of fewer than QRR_ROWS rows (TALL false) leave the norm to the last
+// warp: the nine warps' scan and barriers cost more than the chain.  us a step,
+// whole factorization, TALL / not: 40 rows and fewer 21 / 13, 80 rows 29 / 27,
+// 90 rows 31 / 31, 120 rows 32 / 36 (x2); x4 5 rows 58 / 48, 80 rows 76 / 76, 120
+// rows 90 / 100.
+constexpr int64_t QRR_ROWS = 88;
+
+template <int N, bool TALL>
 __global__ void __launch_bounds__(QRR_NT)
     qr_reflector_kernel(int64_t m, int64_t s, Mat A, double *tau, int64_t lt, int blocked,
                         double *diag, const int *stop) {
@@ -346,7 +353,12 @@ __global__ void __launch_bounds__(QRR_NT)
     const mf<N> one = from_double<N>(1.0), zero = from_double<N>(0.0);
     const int tid = threadIdx.x;
     mf<N> scale, sum;
-    cta_norm<N>(A, m, s, s, scale, sum);
+    if constexpr (TALL) {
+        cta_norm<N>(A, m, s, s, scale, sum);
+    } else {
+        __shared__ double nbuf[QR_NORM_BUF(N)];
+        if (tid >= QRR_TILE) norm_state_warp<N>(A, m, s, s, nbuf, scale, sum);
+    }
     if (tid == QRR_TILE) {
         const mf<N> nrm = norm_value(scale, sum);
         mf<N> t = zero;
@@ -946,10 +958,13 @@ static int qr_n(mflab_handle *h, cudaStream_t s, int pivoted, int64_t m, int64_t
             return record_cuda_error(e, "qr info");
         }
     }
+    auto reflector = [&](int64_t st) {
+        return m - st >= QRR_ROWS ? qr_reflector_kernel<N, true> : qr_reflector_kernel<N, false>;
+    };
     if (!pivoted) {
         // each step's kernels are programmatic dependent launches
         for (int64_t st = 0; st < r; ++st) {
-            int rc = launch_programmatic(qr_reflector_kernel<N>, dim3(1), dim3(QRR_NT), 0, s,
+            int rc = launch_programmatic(reflector(st), dim3(1), dim3(QRR_NT), 0, s,
                                          "qr reflector", m, st, A, tau, lt, 0, nullptr, nullptr);
             if (rc) return rc;
             if (st + 1 < n) {
@@ -978,7 +993,7 @@ static int qr_n(mflab_handle *h, cudaStream_t s, int pivoted, int64_t m, int64_t
                 int rc = launch_programmatic(qr_hybrid_pivot_kernel<N>, dim3(1), dim3(QR_CTA), 0,
                                              s, "qr pivot", m, st, A, perm, S, om);
                 if (rc == MFLAB_OK)
-                    rc = launch_programmatic(qr_reflector_kernel<N>, dim3(1), dim3(QRR_NT), 0, s,
+                    rc = launch_programmatic(reflector(st), dim3(1), dim3(QRR_NT), 0, s,
                                              "qr reflector", m, st, A, tau, lt, 0, nullptr,
                                              nullptr);
                 if (rc == MFLAB_OK && st + 1 < n) {
@@ -1013,7 +1028,7 @@ static int qr_n(mflab_handle *h, cudaStream_t s, int pivoted, int64_t m, int64_t
                                              0, s, "qr panel pivot", m, st, bs, ls, A, perm, S, F,
                                              (const int *)flag);
                     if (rc == MFLAB_OK)
-                        rc = launch_programmatic(qr_reflector_kernel<N>, dim3(1), dim3(QRR_NT), 0,
+                        rc = launch_programmatic(reflector(st), dim3(1), dim3(QRR_NT), 0,
                                                  s, "qr panel reflector", m, st, A, tau, lt, 1,
                                                  diag + ls * N, (const int *)flag);
                     if (rc == MFLAB_OK && st + 1 < n) {
