@@ -397,8 +397,9 @@ __global__ void __launch_bounds__(QRR_NT)
 // them in row order (the reference's chain; only the additions are
 // sequential) while the next 32 rows' operands are on their way.  All 32
 // lanes call it; buf holds 32 N doubles of this warp; the result is returned
-// in every lane.
-template <int N>
+// in every lane.  U additions are unrolled: a kernel that runs one reflector of
+// a short column spends more on fetching the longer x4 loop than it saves.
+template <int N, int U>
 __device__ mf<N> chain_warp(mf<N> acc, int64_t r0, int64_t m, const Mat &X, int64_t cx,
                             const Mat &Y, int64_t cy, double *buf) {
     const unsigned FULL = 0xffffffffu;
@@ -426,7 +427,7 @@ __device__ mf<N> chain_warp(mf<N> acc, int64_t r0, int64_t m, const Mat &X, int6
             };
             const int cnt = m - base < 32 ? (int)(m - base) : 32;
             if (cnt == 32) {
-#pragma unroll 8
+#pragma unroll U
                 for (int i = 0; i < 32; ++i) term(i);
             } else {
                 for (int i = 0; i < cnt; ++i) term(i);
@@ -442,12 +443,12 @@ __device__ mf<N> chain_warp(mf<N> acc, int64_t r0, int64_t m, const Mat &X, int6
 // reflector s of V (implicit one at row s) applied to column c of D by one
 // warp (qr.jl:624-642): the projection chain, then the rank-one update with
 // the rows spread over the lanes
-template <int N>
+template <int N, int U = 8>
 __device__ __forceinline__ void apply_reflector_col_warp(int64_t m, int64_t s, const Mat &V,
                                                          const mf<N> &t, const Mat &D, int64_t c,
                                                          double *buf) {
     const int lane = threadIdx.x & 31;
-    mf<N> proj = chain_warp<N>(load_mf<N>(D.p, D.ld, D.ls, s, c), s + 1, m, V, s, D, c, buf);
+    mf<N> proj = chain_warp<N, U>(load_mf<N>(D.p, D.ld, D.ls, s, c), s + 1, m, V, s, D, c, buf);
     proj = mul(proj, t);
     if (lane == 0) store_mf<N>(D.p, D.ld, D.ls, s, c, sub(load_mf<N>(D.p, D.ld, D.ls, s, c), proj));
     for (int64_t r = s + 1 + lane; r < m; r += 32)
@@ -462,7 +463,12 @@ static inline unsigned warp_col_grid(int64_t cols) {
     return (unsigned)((cols + QR_COL_WARPS - 1) / QR_COL_WARPS);
 }
 
-template <int N>
+// x4 columns of fewer than QR_SHORT_ROWS rows (SHORT) unroll less: 64 x 20
+// 1367 -> 1318 us, 300 x 300 30.9 -> 30.6 ms; 1000 x 100 would take 42.8 ms, not
+// 42.5.
+constexpr int64_t QR_SHORT_ROWS = 300;
+
+template <int N, bool SHORT>
 __global__ void __launch_bounds__(32 * QR_COL_WARPS)
     qr_apply_kernel(int64_t m, int64_t s, Mat V, const double *tau, int64_t lt, Mat D, int64_t c0,
                     int64_t nd) {
@@ -476,7 +482,7 @@ __global__ void __launch_bounds__(32 * QR_COL_WARPS)
 #pragma unroll
     for (int l = 0; l < N; ++l) t.v[l] = tau[l * lt + s];
     if (iszero(t)) return;
-    apply_reflector_col_warp<N>(m, s, V, t, D, c0 + j, buf[w]);
+    apply_reflector_col_warp<N, SHORT ? 2 : 8>(m, s, V, t, D, c0 + j, buf[w]);
 }
 
 // apply_q! (qr.jl:890-956): every reflector in order on one column of D
@@ -958,6 +964,9 @@ static int qr_n(mflab_handle *h, cudaStream_t s, int pivoted, int64_t m, int64_t
             return record_cuda_error(e, "qr info");
         }
     }
+    auto apply = [&](int64_t st) {
+        return N == 4 && m - st < QR_SHORT_ROWS ? qr_apply_kernel<N, N == 4> : qr_apply_kernel<N, false>;
+    };
     auto reflector = [&](int64_t st) {
         return m - st >= QRR_ROWS ? qr_reflector_kernel<N, true> : qr_reflector_kernel<N, false>;
     };
@@ -968,7 +977,7 @@ static int qr_n(mflab_handle *h, cudaStream_t s, int pivoted, int64_t m, int64_t
                                          "qr reflector", m, st, A, tau, lt, 0, nullptr, nullptr);
             if (rc) return rc;
             if (st + 1 < n) {
-                rc = launch_programmatic(qr_apply_kernel<N>, dim3(warp_col_grid(n - st - 1)),
+                rc = launch_programmatic(apply(st), dim3(warp_col_grid(n - st - 1)),
                                          dim3(32 * QR_COL_WARPS), 0, s, "qr apply", m, st, A,
                                          (const double *)tau, lt, A, st + 1, n - st - 1);
                 if (rc) return rc;
@@ -997,7 +1006,7 @@ static int qr_n(mflab_handle *h, cudaStream_t s, int pivoted, int64_t m, int64_t
                                              "qr reflector", m, st, A, tau, lt, 0, nullptr,
                                              nullptr);
                 if (rc == MFLAB_OK && st + 1 < n) {
-                    rc = launch_programmatic(qr_apply_kernel<N>, dim3(warp_col_grid(n - st - 1)),
+                    rc = launch_programmatic(apply(st), dim3(warp_col_grid(n - st - 1)),
                                              dim3(32 * QR_COL_WARPS), 0, s, "qr apply", m, st, A,
                                              (const double *)tau, lt, A, st + 1, n - st - 1);
                     if (rc == MFLAB_OK)
