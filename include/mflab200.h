@@ -522,7 +522,8 @@ int mflab_spd_batched_adjoint(mflab_handle *h, void *stream, int limbs, int64_t 
                               const int *info, int *counter, int grid);
 
 /* mflab_spd_batched / mflab_spd_batched_adjoint with the CTA size chosen:
-   threads = 64, 128, 256 or 512 (the plain entries use 256).  Neither the CTA
+   threads = 64, 128, 256 or 512 (the plain entries use 256); batches whose
+   largest block has at most 48 rows take at most 128.  Neither the CTA
    size nor the number of persistent CTAs (grid) changes any result: every
    block's arithmetic is per element in the reference order; they are the
    knobs of the batched autotuner.  They shape the factor's launch; the

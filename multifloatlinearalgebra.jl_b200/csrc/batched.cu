@@ -29,6 +29,12 @@ constexpr int BATCH_MAXN = 512;  // largest block size
 // small blocks leave room for many CTAs per SM: each block's factor and solve
 // are chains of dependent steps, and throughput comes from blocks in flight.
 constexpr int SPD_W = 16;  // columns of a staged panel
+// Batches of blocks of at most SPD_SHORT rows take at most 128 threads per CTA:
+// a short panel has no work for more, and their registers hold three CTAs per SM
+// where 128 threads hold six.  Factor, us, 256 / 128 threads: x2 50 000 blocks of
+// 8 rows 2379 / 900, of 16 5712 / 2116, 10 000 of 48 3313 / 1455; x3 50 000 of 8
+// 3522 / 2155, 10 000 of 48 6275 / 5324; x4 50 000 of 8 8225 / 6460.
+constexpr int64_t SPD_SHORT = 48;
 
 template <int N>
 struct BlockView {
@@ -599,6 +605,7 @@ extern "C" int mflab_spd_batched_ex(mflab_handle *h, void *stream, int limbs, in
     cudaStream_t s = (cudaStream_t)stream;
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(int), s);
     if (e != cudaSuccess) return mfl::record_cuda_error(e, "spd batched counter");
+    if (max_size <= mfl::SPD_SHORT && threads > 128) threads = 128;
     if (threads == 64)
         rc = launch_factor<64>(limbs, grid, max_size, s, nblocks, sizes, offsets, order, S, ls_s, block, info, counter);
     else if (threads == 128)
