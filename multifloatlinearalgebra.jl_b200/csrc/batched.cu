@@ -201,8 +201,11 @@ __device__ int cta_potrf_staged(const BlockView<N> &F, int block, double *P, int
     return 0;
 }
 
-// rows > 0: the staged panel of `rows` rows per limb in dynamic shared memory
-template <int N, int NT>
+// STAGED: the panel of `rows` rows per limb in dynamic shared memory.  The
+// unstaged loops are a kernel of their own: in one with the staged ones they
+// would take its registers and a CTA less per SM (x2, 2000 blocks of 40 .. 100
+// rows, panels of 32 columns: 2157 us, 1726 us so).
+template <int N, int NT, bool STAGED>
 __global__ void __launch_bounds__(NT)
     spd_factor_kernel(int64_t nblocks, const int64_t *sizes, const int64_t *offsets,
                       const int64_t *order, double *S, int64_t ls_s, int64_t block, int *info,
@@ -228,8 +231,9 @@ __global__ void __launch_bounds__(NT)
             continue;
         }
         BlockView<N> F{Mat{S + offsets[b], n > 0 ? n : 1, ls_s}, n};
-        const int st = rows > 0 ? cta_potrf_staged<N, NT>(F, (int)block, spd_panel, rows, &flag)
-                                : cta_potrf<N, NT>(F, block, bc, &flag);
+        int st;
+        if constexpr (STAGED) st = cta_potrf_staged<N, NT>(F, (int)block, spd_panel, rows, &flag);
+        else st = cta_potrf<N, NT>(F, block, bc, &flag);
         if (t == 0) info[b] = st;
         __syncthreads();
     }
@@ -495,8 +499,8 @@ template <int N, int NT>
 static int launch_factor_n(int grid, int64_t maxn, cudaStream_t s, int64_t nblocks,
                            const int64_t *sizes, const int64_t *offsets, const int64_t *order,
                            double *S, int64_t ls_s, int64_t block, int *info, int *counter) {
-    auto kern = mfl::spd_factor_kernel<N, NT>;
     const size_t smem = staged_bytes(N, maxn, block);
+    auto kern = smem ? mfl::spd_factor_kernel<N, NT, true> : mfl::spd_factor_kernel<N, NT, false>;
     if (smem > 48 * 1024) {
         static std::atomic<unsigned long long> done{0};
         int rc = mfl::set_smem_once((const void *)kern, 112 * 1024, done, "spd factor smem");
