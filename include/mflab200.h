@@ -449,9 +449,11 @@ int mflab_getrs(mflab_handle *h, void *stream, int limbs, int64_t n, int64_t nrh
    more) the row permutation of ipiv, the inverses of the 128 x 128 diagonal
    blocks of L and U, and each off-diagonal block column of L and U times its
    inverted diagonal block; mflab_lu64_solve then overwrites B (n x nrhs
-   binary64, column-major) with inv(A) B: one gather and one kernel per block
-   row and direction, reading only `work` (LU and ldl are checked, not read).
-   Results differ from mflab_getrs in rounding only.  n <= 24576. */
+   binary64, column-major) with inv(A) B, reading only `work` (LU and ldl are
+   checked, not read).  At most 32 right-hand sides are one cooperative launch
+   where its CTAs fit the device; a wait in it that runs out leaves B unsolved
+   and 6 in mflab_device_status.  More, or larger systems, take one gather and
+   one kernel per block row and direction.  Results differ from mflab_getrs in rounding only.  n <= 24576. */
 int mflab_lu64_work_bytes(int64_t n, size_t *bytes);
 int mflab_lu64_prepare(mflab_handle *h, void *stream, int64_t n, const double *LU, int64_t ldl,
                        const int64_t *ipiv, void *work);

@@ -64,7 +64,7 @@ int mflab_int8_gemm_tn(struct mflab_handle *h, void *stream, int engine, int64_t
 
 /* Test hooks of the tcgen05 kernels issued through this handle: wait_limit
    bounds their waits of one role on another (mbarrier polls; 0 restores the
-   default), inject = 1 makes the MMA issuer of each launch first wait a
+   default) and the polls of the one-launch binary64 solve, inject = 1 makes the MMA issuer of each launch first wait a
    short fixed bound on a barrier nothing arrives on, so that wait runs out
    with copies in flight and the kernel takes its timeout path (error code in the device status word,
    every issued copy and MMA drained, TMEM freed).  Nothing faults or hangs;

@@ -1764,6 +1764,9 @@ def solve_mixed_lu(A: MFMatrix, B: MFMatrix, tol: float = 0.0, maxiter: int = 40
     if timing:
         ev[2].record()
         ev[2].synchronize()
+    code = device_status(A.device)  # the factor's and the solves' bounded waits
+    if code:
+        raise MFLABError(f"solve_mixed_lu: a wait on the device ran out (device status {code})")
     report = {"iterations": it, "backward_error": history[-1] if history else None,
               "history": history, "converged": bool(history) and history[-1] <= tol,
               "factor": "binary64 partial-pivoting LU",

@@ -255,11 +255,13 @@ int mstep_launch(cudaStream_t s, int64_t nrhs, int64_t j0, int jb, const double 
 // owners of the block itself and of the next one, the only CTAs the chain of
 // steps waits for, and the others' polls are spread over the rest.  The slices
 // do not depend on the solve: two are prefetched into shared memory ahead of
-// the rows.  Arithmetic and results are the block kernel's.  All CTAs are co-resident (cooperative launch); a wait that runs
-// out (LS_SPIN polls) records error 6 and the CTA leaves at its next barrier,
-// the others as their waits run out or see the abort word.  n = 4096, 16
-// right-hand sides: 220 us (460 us as 64 launches, 348 us with flags, 286 us
-// before the 2 x 2 tiles below).
+// the rows.  Arithmetic and results are the block kernel's.  All CTAs are
+// co-resident (cooperative launch); a wait that runs out (LS_SPIN polls, or the
+// handle's limit) records error 6 in the handle's status word and the CTA leaves
+// at its next barrier, the others as their waits run out or see the abort word.
+// B is then not solved: a caller reads the status word before it uses the
+// result.  n = 4096, 16 right-hand sides: 220 us (460 us as 64 launches, 348 us
+// with flags, 286 us before the 2 x 2 tiles below).
 constexpr int LS_STAGES = 3, LS_ERR_TIMEOUT = 6;
 constexpr long long LS_SPIN = 1LL << 21;
 constexpr int64_t LS_MAX_RHS = 32;  // more right-hand sides: the block kernel
@@ -292,7 +294,7 @@ __global__ void __launch_bounds__(MS_NT)
     lu64_solve_kernel(int64_t n, int64_t nrhs, const int *perm, const double *__restrict__ invL,
                       const double *__restrict__ invU, const double *__restrict__ ML,
                       const double *__restrict__ MU, double *B, int64_t ldb,
-                      unsigned long long *pub, int *abort_word, int *err) {
+                      unsigned long long *pub, int *abort_word, int *err, long long spin) {
     extern __shared__ __align__(16) uint8_t ls_raw[];
     LsShared &sh = *reinterpret_cast<LsShared *>(ls_raw);
     __shared__ int s_stop;
@@ -389,7 +391,7 @@ __global__ void __launch_bounds__(MS_NT)
 #pragma unroll
                 for (int u = 0; u < PER; ++u)
                     open = open || y[u][0] == LS_UNSET || y[u][1] == LS_UNSET;
-                if (open && (polls >= LS_SPIN ||
+                if (open && (polls >= spin ||
                              ((polls & 255) == 255 && *(volatile int *)abort_word))) {
                     if (atomicExch(abort_word, 1) == 0) atomicExch(err, LS_ERR_TIMEOUT);
                     s_stop = 1;
@@ -537,7 +539,9 @@ extern "C" int mflab_lu64_solve(mflab_handle *h, void *stream, int64_t n, int64_
         cudaError_t e = cudaMemsetAsync(pub, 0xff, bytes - 256, s);
         if (e == cudaSuccess) e = cudaMemsetAsync(abort_word, 0, sizeof(int), s);
         if (e != cudaSuccess) return mfl::record_cuda_error(e, "lu64 solve rows");
-        void *args[] = {&n, &nrhs, &perm, &invL, &invU, &ML, &MU, &B, &ldb, &pub, &abort_word, &err};
+        long long spin = h->tc_limit > 0 ? h->tc_limit : mfl::LS_SPIN;
+        void *args[] = {&n,   &nrhs, &perm, &invL, &invU,       &ML,  &MU,
+                        &B,   &ldb,  &pub,  &abort_word, &err, &spin};
         e = cudaLaunchCooperativeKernel((const void *)mfl::lu64_solve_kernel,
                                         dim3((unsigned)((n + mfl::MS_ROWS - 1) / mfl::MS_ROWS)),
                                         dim3(mfl::MS_NT), args, sizeof(mfl::LsShared), s);
