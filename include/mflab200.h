@@ -505,7 +505,8 @@ int mflab_ldlt_diagnostics(mflab_handle *h, void *stream, int limbs, int64_t n, 
    stream-ordered memset).  Each block follows cholesky!(S_b; block) and
    ldiv!(x_b, F_b) exactly; info[b] receives 0 or the failing column.
    max_size <= 512 bounds every sizes[b] (it sizes the per-CTA shared
-   buffer); a block larger than max_size is left untouched with info[b] = -1.  grid <= 0 picks 4 CTAs per SM.  No allocation, no
+   buffer); a block larger than max_size is left untouched with info[b] = -1.
+   grid <= 0 picks as many CTAs as the SMs hold.  No allocation, no
    synchronisation.  No reference counterpart (the reference factors one
    matrix per call: src/factorizations/cholesky.jl:68-107). */
 int mflab_spd_batched(mflab_handle *h, void *stream, int limbs, int64_t nblocks, int64_t max_size,
@@ -515,8 +516,9 @@ int mflab_spd_batched(mflab_handle *h, void *stream, int limbs, int64_t nblocks,
 
 /* Adjoint of x_b = S_b^{-1} b_b reusing the factors of mflab_spd_batched: XB
    holds xbar on entry and bbar = S^{-1} xbar on exit; SB (packed like S)
-   receives Sbar = -(bbar x^T + x bbar^T) / 2.  Blocks with info != 0 are
-   skipped.  No reference counterpart. */
+   receives Sbar = -(bbar x^T + x bbar^T) / 2.  A block without a factor
+   (info != 0, or larger than max_size) keeps its part of XB and gets Sbar = 0.
+   No reference counterpart. */
 int mflab_spd_batched_adjoint(mflab_handle *h, void *stream, int limbs, int64_t nblocks,
                               int64_t max_size, const int64_t *sizes, const int64_t *offsets,
                               const int64_t *boffsets, const int64_t *order, const double *L,

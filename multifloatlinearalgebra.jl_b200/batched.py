@@ -228,8 +228,7 @@ def solve_spd_batched_rrule(batch: SPDBatch, block: int = 16, tuning=None):
     def pullback(xbar: torch.Tensor):
         lib = _native.load()
         xb = xbar.clone()
-        # every block was factored (a failure raised above), so the kernel
-        # writes every entry
+        # the kernel writes every entry, zeros where a block has no factor now
         sb = torch.empty_like(batch.S) if batch.total_s else torch.zeros_like(batch.S)
         rc = lib.mflab_spd_batched_adjoint_ex(
             _handle(batch.device), torch.cuda.current_stream(batch.device).cuda_stream, batch.N,

@@ -455,7 +455,14 @@ __global__ void __launch_bounds__(SPD_ADJ_NT)
     extern __shared__ double adj_vec[];  // [2][N][max block size]
     const int64_t b = order[blockIdx.x];
     const int n = (int)sizes[b];
-    if (n == 0 || sizes[b] > maxn || info[b] != 0) return;
+    if (sizes[b] > maxn || info[b] != 0) {  // no factor: the gradient is zero
+        const int64_t all = (int64_t)n * n;
+        for (int64_t e = threadIdx.x; e < all; e += SPD_ADJ_NT)
+#pragma unroll
+            for (int l = 0; l < N; ++l) SB[l * ls_s + offsets[b] + e] = 0.0;
+        return;
+    }
+    if (n == 0) return;
     double *xs = adj_vec, *bs = adj_vec + N * maxn;
     for (int r = threadIdx.x; r < n; r += SPD_ADJ_NT)
 #pragma unroll
