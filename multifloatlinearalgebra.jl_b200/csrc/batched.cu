@@ -189,7 +189,7 @@ __device__ int cta_potrf_staged(const BlockView<N> &F, int block, double *P, int
             const mf<N> old = F.at(row, col);
             mf<N> acc = from_double<N>(0.0);
             if (w == SPD_W) {
-#pragma unroll 4
+#pragma unroll (N == 2 ? 8 : 4)
                 for (int k = 0; k < SPD_W; ++k) acc = add(acc, mul(get(k, w + r), get(k, w + c)));
             } else {
                 for (int k = 0; k < w; ++k) acc = add(acc, mul(get(k, w + r), get(k, w + c)));
