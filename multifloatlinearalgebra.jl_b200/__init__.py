@@ -433,6 +433,8 @@ def _scalar(N: int, v) -> "C.Array":
 
 
 def _same_type(*mats: MFMatrix) -> int:
+    if not isinstance(mats[0], MFMatrix):
+        raise ArgumentError("expected MFMatrix operands")
     first = mats[0].storage
     N, device = first.shape[0], first.get_device()
     for x in mats:
