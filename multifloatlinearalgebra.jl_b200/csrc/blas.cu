@@ -38,8 +38,8 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(n) : "memory");
 }
 
-// column tiles in a grid's y dimension; wider products take layers in z, up to
-// as many columns as a grid of the widest tiles (64 columns, 32 in x4) holds
+// column tiles in a grid's y dimension; wider products take several launches, up
+// to as many columns as a grid of the widest tiles (64 columns, 32 in x4) holds
 constexpr int64_t MM_GRID_Y = 65535;
 template <int N>
 struct MMColumns {
@@ -79,9 +79,7 @@ __global__ void __launch_bounds__(MMShape<N, BM, BN, BK, TM, TN>::NT)
     double *Bs = smem + 2 * N * BK * BM;  // [2][N][BK][BN]
     const int tid = threadIdx.x;
     const int tx = tid % TX, ty = tid / TX;
-    const int64_t row0 = (int64_t)blockIdx.x * BM;
-    const int64_t col0 = ((int64_t)blockIdx.z * MM_GRID_Y + blockIdx.y) * BN;
-    if (col0 >= n) return;  // the last of several layers of column tiles
+    const int64_t row0 = (int64_t)blockIdx.x * BM, col0 = (int64_t)blockIdx.y * BN;
     if (TRI && row0 + BM - 1 < col0) return;  // tile strictly above the diagonal
     // debug builds: C's column stride holds its rows
     if (!(mode & MM_PACKED) && !MFLAB_IDX_OK(C.ld >= m, 6, C.ld, m)) return;
@@ -237,11 +235,17 @@ static int run_mm(int64_t m, int64_t n, int64_t k, Mat A, Mat B, Mat C, const do
     }
     if (m <= 0 || n <= 0) return MFLAB_OK;
     if (n > MMColumns<N>::most) return MFLAB_ERR_UNSUPPORTED;
-    const int64_t tiles = (n + BN - 1) / BN;
-    const dim3 grid((unsigned)((m + BM - 1) / BM), (unsigned)std::min(tiles, MM_GRID_Y),
-                    (unsigned)((tiles + MM_GRID_Y - 1) / MM_GRID_Y));
-    kern<<<grid, S::NT, S::smem_bytes, s>>>(m, n, k, A, B, C, al, be, overwrite, info, mode);
-    return record_cuda_error(cudaGetLastError(), "mm_kernel launch");
+    // the columns' own indices matter to a triangular or packed result and to a
+    // triangle on the right, which no memory holds at that many columns
+    if (n > MM_GRID_Y * BN && (TRI || (mode & (MM_PACKED | MM_RIGHT)))) return MFLAB_ERR_UNSUPPORTED;
+    for (int64_t c0 = 0; c0 < n; c0 += MM_GRID_Y * BN) {
+        const int64_t cols = std::min(n - c0, MM_GRID_Y * BN);
+        const dim3 grid((unsigned)((m + BM - 1) / BM), (unsigned)((cols + BN - 1) / BN));
+        kern<<<grid, S::NT, S::smem_bytes, s>>>(m, cols, k, A, TB ? B.at(c0, 0) : B.at(0, c0),
+                                                C.at(0, c0), al, be, overwrite, info, mode);
+        if (int rc = record_cuda_error(cudaGetLastError(), "mm_kernel launch")) return rc;
+    }
+    return MFLAB_OK;
 }
 
 // Tile shapes.  Every output is the same chain in every shape, so the choice
