@@ -437,7 +437,7 @@ def _same_type(*mats: MFMatrix) -> int:
         raise ArgumentError("expected MFMatrix operands")
     first = mats[0].storage
     N, device = first.shape[0], first.get_device()
-    for x in mats:
+    for x in mats[1:]:
         if not isinstance(x, MFMatrix):
             raise ArgumentError("expected MFMatrix operands")
         st = x.storage
