@@ -3,7 +3,8 @@
 No reference counterpart: MultiFloatLinearAlgebra.jl factors one matrix per
 call.  Every block here follows cholesky!(S_i) / ldiv!(x_i, F_i) of the
 reference exactly (one persistent CTA per block for the factor, 16 or 32 lanes
-per block for the forward and one for the backward substitution), so per block the results equal the single-matrix routines.
+per block for the forward and one for the backward substitution), so per block
+the results equal the single-matrix routines.
 
     batch = SPDBatch(N, sizes)              # packed device storage
     batch.set_block(i, S_i); batch.set_rhs(i, b_i)
@@ -114,8 +115,10 @@ def autotune(batch: SPDBatch, block: int = 16, candidates: Optional[Sequence] = 
     """Launch shape of the batched factor + solve for this batch: the CTA size
     (64, 128, 256 or 512 threads) and the number of persistent CTAs (1 to 32
     per SM, at most 2048 threads per SM), picked by timing the real launch on
-    the batch's own blocks (restored afterwards).  Neither knob changes any result (each block's
-    arithmetic is per element in the reference order), so the choice is free.
+    the batch's own blocks (restored afterwards).  Batches of at most 48 rows
+    per block take at most 128 threads.  Neither knob changes any result (each
+    block's arithmetic is per element in the reference order), so the choice is
+    free.
     Cached per (limbs, block, size signature of the batch); a tuning
     profile (tuning.TuneProfile, fingerprint checked) that holds this
     signature supplies the shape without any timing.

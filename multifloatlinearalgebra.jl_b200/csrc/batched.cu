@@ -123,8 +123,8 @@ __device__ int cta_potrf(const BlockView<N> &F, int64_t block, double (*bc)[4], 
 // latency (2.5 k cycles in x2) for all rows at once, and the trailing update
 // reads both factors of a product from shared memory, where it read four values
 // per product through L1.  10 000 blocks of 8 .. 256 rows in x2: 20.7 ms
-// (29.4 ms with the forward substitution on the loops above, which batches with less than two CTAs of this
-// kind per SM still take).
+// (29.4 ms with the forward substitution on the loops above, which batches with
+// less than two CTAs of this kind per SM still take).
 template <int N, int NT>
 __device__ int cta_potrf_staged(const BlockView<N> &F, int block, double *P, int rows, int *flag) {
     const int t = threadIdx.x;
