@@ -163,10 +163,20 @@ __device__ __forceinline__ mf<N> warp_max(mf<N> v) {
     return v;
 }
 
+// Threads per column: 512 while a column has an SM to itself, 256 and then 128
+// as the divisions' registers let several CTAs share one.  us, the former 256
+// threads / now: x3, 5 rows 16 columns 24 / 23, 5000 120 / 89, 60000 1216 / 615;
+// x4, 4096 rows 16 columns 51 / 36, 222 69 / 49, 900 352 / 175 (512 threads
+// throughout: 36, 68, 255, and x3 with 60000 columns 5003).
+template <int N>
+struct BeColumns {
+    static constexpr int64_t few = 148, some = N == 3 ? 4 * 148 : 2 * 148;
+};
+
 template <int N, int NT>
-__global__ void __launch_bounds__(NT) backward_error_kernel(int64_t m, int64_t k, Mat X, Mat B,
-                                                            Mat R, const double *anorm,
-                                                            const int *a_nonfinite, double *out) {
+__global__ void __launch_bounds__(NT, NT == 128 && N <= 3 ? 8 : NT == 256 && N == 3 ? 4 : 1)
+    backward_error_kernel(int64_t m, int64_t k, Mat X, Mat B, Mat R, const double *anorm,
+                          const int *a_nonfinite, double *out) {
     __shared__ double sv[3][NT / 32][N];
     const int t = threadIdx.x, lane = t % 32, warp = t / 32;
     const int64_t j = blockIdx.x;
@@ -175,7 +185,7 @@ __global__ void __launch_bounds__(NT) backward_error_kernel(int64_t m, int64_t k
     for (int q = 0; q < 3; ++q) top[q] = from_double<N>(0.0);
     bool fin = true;
     auto scan = [&](const Mat &M, int64_t rows, mf<N> &best) {
-#pragma unroll 4
+#pragma unroll (N == 3 && NT == 256 ? 2 : 4)
         for (int64_t r = t; r < rows; r += NT) {
             const mf<N> v = load_mf<N>(M.p, M.ld, M.ls, r, j);
             fin = fin && isfinite_mf(v);
@@ -207,6 +217,17 @@ __global__ void __launch_bounds__(NT) backward_error_kernel(int64_t m, int64_t k
     if (lane == 0)
 #pragma unroll
         for (int l = 0; l < N; ++l) out[j * N + l] = v.v[l];
+}
+
+template <int N>
+static void launch_backward_error(int64_t m, int64_t k, int64_t nrhs, const Mat &X, const Mat &B,
+                                  const Mat &R, const double *anorm, const int *a_nonfinite,
+                                  double *out, cudaStream_t s) {
+    const int nt = nrhs <= BeColumns<N>::few ? 512 : nrhs <= BeColumns<N>::some ? 256 : 128;
+    auto kern = nt == 512   ? backward_error_kernel<N, 512>
+                : nt == 256 ? backward_error_kernel<N, 256>
+                            : backward_error_kernel<N, 128>;
+    kern<<<(unsigned)nrhs, (unsigned)nt, 0, s>>>(m, k, X, B, R, anorm, a_nonfinite, out);
 }
 
 template <int N>
@@ -317,21 +338,21 @@ extern "C" int mflab_backward_error(mflab_handle *h, void *stream, int limbs, in
             mfl::abs_row_sum_kernel<2><<<gm, 128, 0, s>>>(m, k, a, uplo, rowsum, anf);
             mfl::max_rowsum_kernel<2, 256><<<1, 256, 0, s>>>(m, rowsum, anorm);
         }
-        mfl::backward_error_kernel<2, 512><<<(unsigned)nrhs, 512, 0, s>>>(m, k, x, b, r, anorm, anf, out);
+        mfl::launch_backward_error<2>(m, k, nrhs, x, b, r, anorm, anf, out, s);
         break;
     case 3:
         if (m > 0) {
             mfl::abs_row_sum_kernel<3><<<gm, 128, 0, s>>>(m, k, a, uplo, rowsum, anf);
             mfl::max_rowsum_kernel<3, 256><<<1, 256, 0, s>>>(m, rowsum, anorm);
         }
-        mfl::backward_error_kernel<3, 512><<<(unsigned)nrhs, 512, 0, s>>>(m, k, x, b, r, anorm, anf, out);
+        mfl::launch_backward_error<3>(m, k, nrhs, x, b, r, anorm, anf, out, s);
         break;
     default:
         if (m > 0) {
             mfl::abs_row_sum_kernel<4><<<gm, 128, 0, s>>>(m, k, a, uplo, rowsum, anf);
             mfl::max_rowsum_kernel<4, 256><<<1, 256, 0, s>>>(m, rowsum, anorm);
         }
-        mfl::backward_error_kernel<4, 512><<<(unsigned)nrhs, 512, 0, s>>>(m, k, x, b, r, anorm, anf, out);
+        mfl::launch_backward_error<4>(m, k, nrhs, x, b, r, anorm, anf, out, s);
         break;
     }
     return mfl::record_cuda_error(cudaGetLastError(), "backward error");
@@ -391,16 +412,13 @@ extern "C" int mflab_backward_error_norm(mflab_handle *h, void *stream, int limb
     cudaStream_t s = (cudaStream_t)stream;
     switch (limbs) {
     case 2:
-        mfl::backward_error_kernel<2, 512><<<(unsigned)nrhs, 512, 0, s>>>(m, k, x, b, r, anorm,
-                                                                         nonfinite, out);
+        mfl::launch_backward_error<2>(m, k, nrhs, x, b, r, anorm, nonfinite, out, s);
         break;
     case 3:
-        mfl::backward_error_kernel<3, 512><<<(unsigned)nrhs, 512, 0, s>>>(m, k, x, b, r, anorm,
-                                                                         nonfinite, out);
+        mfl::launch_backward_error<3>(m, k, nrhs, x, b, r, anorm, nonfinite, out, s);
         break;
     default:
-        mfl::backward_error_kernel<4, 512><<<(unsigned)nrhs, 512, 0, s>>>(m, k, x, b, r, anorm,
-                                                                         nonfinite, out);
+        mfl::launch_backward_error<4>(m, k, nrhs, x, b, r, anorm, nonfinite, out, s);
         break;
     }
     return mfl::record_cuda_error(cudaGetLastError(), "backward error (given norm)");
