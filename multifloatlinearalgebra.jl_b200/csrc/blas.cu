@@ -275,11 +275,16 @@ static double mm_cost(int64_t m, int64_t n, bool tri, int bm, int bn, double rat
 }
 
 // the shape with the smallest estimate; a lone 16 x 8 CTA (one chain per
-// scheduler) leaves the pipe half idle, hence at least two rounds for it
-template <int N>
+// scheduler) leaves the pipe half idle, hence at least two rounds for it.  The
+// small x2 tiles of a triangle run below their rate: every other CTA returns at
+// once, and a transposed left operand (TA 1) is staged across its columns.  k =
+// 256, mid / wide, us: P^T P n = 1600 777 / 843, 2000 1191 / 1111, 3500 3477 /
+// 2980; A B^T 2000 977 / 1032, 3500 2854 / 2773.
+template <int N, int TA>
 static int mm_tile(int64_t m, int64_t n, bool tri) {
-    const double tiny = mm_cost(m, n, tri, 16, 8, N == 2 ? 14.6 : 16.8, 2);
-    const double mid = N == 2 ? mm_cost(m, n, tri, 32, 16, 15.6, 1)
+    const double slow = N == 2 && tri ? (TA == 1 ? 1.18 : 1.035) : 1.0;
+    const double tiny = slow * mm_cost(m, n, tri, 16, 8, N == 2 ? 14.6 : 16.8, 2);
+    const double mid = N == 2 ? slow * mm_cost(m, n, tri, 32, 16, 15.6, 1)
                               : mm_cost(m, n, tri, 16, 16, N == 3 ? 17.0 : 17.7, 1);
     const double wide = N == 2   ? mm_cost(m, n, tri, 64, 64, 16.5, 1)
                         : N == 3 ? mm_cost(m, n, tri, 32, 32, 17.4, 1)
@@ -294,7 +299,7 @@ static int run_mm_n(int64_t m, int64_t n, int64_t k, Mat A, Mat B, Mat C, const 
     if constexpr (N == 1) {
         return run_mm<1, 64, 64, 16, 4, 4, 2, TA, TB, TRI, FUSED, TRMM>(m, n, k, A, B, C, alpha, beta, s, info, mode);
     } else {
-        const int tile = mm_tile<N>(m, n, TRI);
+        const int tile = mm_tile<N, TA>(m, n, TRI);
         if (tile == MM_TINY)
             return run_mm<N, 16, 8, 16, 1, 1, (N == 2 ? 8 : N == 3 ? 4 : 2), TA, TB, TRI, FUSED, TRMM>(
                 m, n, k, A, B, C, alpha, beta, s, info, mode);

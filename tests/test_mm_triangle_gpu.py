@@ -1,0 +1,22 @@
+"""x2 products into a triangle on both sides of the line between their tile
+shapes, bit for bit against the oracle."""
+import pytest
+
+from conftest import assert_bitwise
+from test_oracle import syn
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,k", [(1856, 2), (1920, 3), (2000, 2)], ids=str)
+def test_triangle_tiles(mf, ref, rng, n, k):
+    Q, P, P2 = syn.randn_mf(rng, 2, k, n), syn.randn_mf(rng, 2, n, k), syn.randn_mf(rng, 2, n, k)
+    C0 = syn.randn_mf(rng, 2, n, n)
+    Cd = mf.MFMatrix.from_numpy(C0)
+    mf.gemmt_(Cd, mf.MFMatrix.from_numpy(P), mf.MFMatrix.from_numpy(P2), -1.0, 1.0)
+    assert_bitwise(Cd.to_numpy(), ref.gemmt_lower(P, P2, C0.copy(), -1.0, 1.0), "gemmt")
+    Cd = mf.MFMatrix.from_numpy(C0)
+    mf.syrk_(Cd, mf.MFMatrix.from_numpy(Q), -1.0, 1.0)
+    want = ref.gemmt_lower(Q.transpose(0, 2, 1).copy(), Q.transpose(0, 2, 1).copy(), C0.copy(), -1.0,
+                           1.0)
+    assert_bitwise(Cd.to_numpy(), want, "syrk")
