@@ -204,9 +204,11 @@ __device__ int cta_potrf_staged(const BlockView<N> &F, int block, double *P, int
 // STAGED: the panel of `rows` rows per limb in dynamic shared memory.  The
 // unstaged loops are a kernel of their own: in one with the staged ones they
 // would take its registers and a CTA less per SM (x2, 2000 blocks of 40 .. 100
-// rows, panels of 32 columns: 2157 us, 1726 us so).
+// rows, panels of 32 columns: 2157 us, 1726 us so).  The x2 kernel of 256
+// threads is compiled for the three CTAs that its panels leave room for (10 000
+// blocks 20.81 -> 20.77 ms); 0 leaves the others to the compiler.
 template <int N, int NT, bool STAGED>
-__global__ void __launch_bounds__(NT)
+__global__ void __launch_bounds__(NT, (N == 2 && STAGED && NT == 256) ? 3 : 0)
     spd_factor_kernel(int64_t nblocks, const int64_t *sizes, const int64_t *offsets,
                       const int64_t *order, double *S, int64_t ls_s, int64_t block, int *info,
                       int *counter, int64_t maxn, int rows) {
